@@ -28,7 +28,8 @@ enum Status : uint8_t { DEAD = 0, ALIVE = 1, FOUND = 2, W2CUT = 3, W3CUT = 4, OV
 // exit codes of the drop-in binaries (reference cheese.cu:1023-1026, 1153-1220, 1284, 1848-1891)
 enum Rc : int { RC_CIRCUIT = 0, RC_PROOF = 1, RC_SPEC = 2, RC_USAGE = 3, RC_OVERFLOW = 4, RC_CUDA = 5 };
 
-template <typename T> struct Z4 { T a, b, c, d; };
+// 16-byte aligned: an int32 entry is one 128-bit load, and arrays of entries may be read as int4
+template <typename T> struct alignas(16) Z4 { T a, b, c, d; };
 using Zw = Z4<int64_t>;
 
 CZ_HD Zw zadd(Zw x, Zw y) { return {x.a + y.a, x.b + y.b, x.c + y.c, x.d + y.d}; }
