@@ -70,6 +70,7 @@ struct DevSpec {
   const int *cxtable;
   const int4 *ginv;                    // GMAX x 64 local inverse matrices (a, b, c, d as int32)
   const longlong2 *goal;               // N*N entries as (a, b), (c, d) pairs
+  int unit;                            // target and gates unitary: every residual is sqrt2^k times a unitary matrix
   int states, m;                       // state targets: m rows (images of the inputs) are searched for the goal rows
   const int *ginfo;                    // state targets: per row the goal's sde, nullity and Schmidt rank per cut
 };
@@ -278,6 +279,112 @@ __device__ __forceinline__ int tbound_lanes(const Z4<ST> *S, int k, int lane) {
   const int top = 2 * (NQ + k);
   return top - v > 0 ? top - v : 0;
 }
+// ---- the same T bound for unitary residuals of small exponent, four components to a register ----
+// In a unitary residual (entries sqrt2^k U) sum |entry|^2 per row is 2^k in both embeddings of Z[sqrt2], so an entry's
+// coefficients satisfy a^2 + b^2 + c^2 + d^2 <= 2^k, and a transform output X_f(z) = 2^k N PTM(f, z) has |A| <= 2^(n +
+// k - 1) and |X| <= 2^(n + k - 1/2). While n + k <= 7 the coefficients and their sums and differences fit in 8 bits
+// and so does every output, so the four components of a product are four dp4a of 8-bit words and travel through the
+// transform as the base-256 digits of one 32-bit integer (additions are linear in the digits; intermediate digits may
+// leave the range, the outputs do not). A digit bias of 128 at point 0 reaches every output, so the output bytes are
+// digit + 128: their low 7 bits are the digit's, all that a valuation needs. One lane per pair f as above: 32 x (2
+// shared loads, 4 dp4a, 3 shifts) + 80 butterflies, where 32-bit components took 32 x (2 wide loads, 28 multiply-adds)
+// + 320 butterflies and four times the registers.
+constexpr int PACK_MAX = 7;              // n + k up to which the packed form is exact
+__device__ __forceinline__ int pack4(int a, int b, int c, int d) {
+  return (int)__byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+// an entry y as four words of 8-bit coefficients: dot products with x's first word are the components a, c, b - d and
+// b + d of x conj(y)
+template <typename ST> __device__ __forceinline__ int4 pack_entry(const Z4<ST> &v) {
+  const int a = (int)v.a, b = (int)v.b, c = (int)v.c, d = (int)v.d;
+  return make_int4(pack4(a, b, c, d), pack4(-c, -d, a, b), pack4(b - d, a + c, b + d, c - a),
+                   pack4(-b - d, a - c, b - d, a + c));
+}
+// OR of the output bytes of pair f (0 for f = 0); the point map as in tbound_round
+template <int NQ, bool IDENT>
+__device__ __forceinline__ unsigned packed_round(const int4 *Y, int f) {
+  constexpr int E = 1 << (2 * NQ), HP = E / 2;
+  if (f == 0) return 0;
+  const int lomask = IDENT ? E - 1 : ((f & HP) ? E - 1 : (f & -f) - 1);
+  int v[HP];
+#pragma unroll
+  for (int i = 0; i < HP; i++) {
+    const int e = IDENT ? i : (i & lomask) | ((i & ~lomask) << 1);
+    const int4 y = Y[e];
+    const int x = Y[e ^ f].x;
+    int s = __dp4a(x, y.w, 0);
+    s = __dp4a(x, y.z, s << 8);
+    s = __dp4a(x, y.y, s << 8);
+    v[i] = __dp4a(x, y.x, s << 8);
+  }
+  v[0] += (int)0x80808080u;
+#pragma unroll
+  for (int h = 1; h < HP; h <<= 1)
+#pragma unroll
+    for (int i = 0; i < HP; i++)
+      if (!(i & h)) {
+        const int u = v[i], w = v[i | h];
+        v[i] = u + w;
+        v[i | h] = u - w;
+      }
+  int o = 0;
+#pragma unroll
+  for (int i = 0; i < HP; i++) o |= v[i];
+  return (unsigned)o;
+}
+// the bound from the OR words of the transform outputs: O1 = OR of 2A, X, alpha, beta, O2 = OR of 2A, alpha
+template <int NQ> __device__ __forceinline__ int bound_of(unsigned O1, unsigned O2, int k) {
+  if (!O1) return 0;
+  const int mv = __ffs((int)O1) - 1;
+  return max(0, 2 * (NQ + k) - (2 * mv + (((O2 >> mv) & 1) ? 0 : 1)));
+}
+// bytes (A, C, X, Y) of an OR word to (O1, O2)
+__device__ __forceinline__ void unpack_or(unsigned o, unsigned &O1, unsigned &O2) {
+  O2 = ((o | (o >> 8)) & 0x7fu) << 1;
+  O1 = O2 | (((o >> 16) | (o >> 24)) & 0x7fu);
+}
+// T bound of the residual packed in Y (E words). At 3 qubits the 32 pairs f >= 32 come first: `dead(T)` says whether
+// a bound of T already decides the entry (bounds only grow with further pairs); then the rest is left out and T is a
+// lower bound. On the deep proofs 92 % of the entries are dead and these 32 pairs show it for every one of them.
+template <int NQ, typename Dead>
+__device__ __forceinline__ int packed_tbound(const int4 *Y, int k, int lane, Dead dead) {
+  constexpr int E = 1 << (2 * NQ), PL = E > 32 ? E / 32 : 1;
+  unsigned o = 0, O1, O2;
+  if constexpr (E == 64) {
+    o = __reduce_or_sync(FULL, packed_round<NQ, true>(Y, 32 + lane));
+    unpack_or(o, O1, O2);
+    const int T = bound_of<NQ>(O1, O2, k);
+    if (dead(T)) return T;
+  }
+  o |= packed_round<NQ, false>(Y, lane < E ? lane : 0);
+  // f = 0: alpha + 2^16 beta over all E points across the warp (|alpha| <= 2^7, |beta| < 2^7)
+  int v[PL];
+#pragma unroll
+  for (int t = 0; t < PL; t++) {
+    const int4 y = lane + 32 * t < E ? Y[lane + 32 * t] : make_int4(0, 0, 0, 0);
+    // beta = ab + bc + cd - da: half of (a, b, c, d) . (b - d, a + c, b + d, c - a)
+    v[t] = __dp4a(y.x, y.x, 0) + ((__dp4a(y.x, y.z, 0) >> 1) << 16);
+  }
+#pragma unroll
+  for (int h = 1; h < PL; h <<= 1)
+#pragma unroll
+    for (int t = 0; t < PL; t++)
+      if (!(t & h)) { const int u = v[t], w = v[t | h]; v[t] = u + w; v[t | h] = u - w; }
+  unsigned R = 0;
+#pragma unroll
+  for (int t = 0; t < PL; t++) {
+#pragma unroll
+    for (int h = 1; h < 32 && h < E; h <<= 1) {
+      const int u = __shfl_xor_sync(FULL, v[t], h);
+      v[t] = (lane & h) ? u - v[t] : u + v[t];
+    }
+    R |= (unsigned)(v[t] + 0x8000) ^ 0x8000u;
+  }
+  o = __reduce_or_sync(FULL, o);
+  R = __reduce_or_sync(FULL, R);
+  unpack_or(o, O1, O2);
+  return bound_of<NQ>(O1 | (R & 0xffffu) | (R >> 16), O2 | (R & 0xffffu), k);
+}
 // 32-bit residues in one pass (3 qubits: 128 transform values per lane); 64-bit residues (k > 29, rare) one
 // component per pass
 template <int NQ, typename ST> __device__ __noinline__ int warp_tbound32(const Z4<ST> *S, int k, int lane) {
@@ -285,6 +392,10 @@ template <int NQ, typename ST> __device__ __noinline__ int warp_tbound32(const Z
 }
 template <int NQ, typename ST> __device__ __noinline__ int warp_tbound64(const Z4<ST> *S, int k, int lane) {
   return tbound_lanes<NQ, uint64_t, 4>(S, k, lane);
+}
+// the same values one component per pass: a quarter of the registers, for kernels where this is the rare path
+template <int NQ, typename ST> __device__ __noinline__ int warp_tbound_slim(const Z4<ST> *S, int k, int lane) {
+  return 2 * (NQ + k) > 64 ? tbound_lanes<NQ, uint64_t, 4>(S, k, lane) : tbound_lanes<NQ, uint32_t, 4>(S, k, lane);
 }
 template <int NQ, typename ST> __device__ __forceinline__ int ptm_bound(const Z4<ST> *S, int k, int lane) {
   return 2 * (NQ + k) > 64 ? warp_tbound64<NQ, ST>(S, k, lane) : warp_tbound32<NQ, ST>(S, k, lane);
@@ -1409,37 +1520,40 @@ template <typename ST> struct TBoundArgs {
   uint64_t *sh1, *sh2, *sidx;
   NodeMeta *smeta;
 };
+// One block's warps walk the queue with a fixed stride. Bound by issue: a dead entry (most are) is the child's update,
+// its packing and one packed round, about 800 instructions.
 template <int NQ, typename ST, bool BATCHED = false>
-__global__ void __launch_bounds__(TB_WARPS * 32) k_tbound(const __grid_constant__ DevSpec sp0, const TBoundArgs<ST> a) {
+__global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? 3 : 1)
+    k_tbound(const __grid_constant__ DevSpec sp0, const TBoundArgs<ST> a) {
   constexpr int N = 1 << NQ, E = N * N, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
+  constexpr bool PACKED = sizeof(ST) == 4;               // the packed T bound (int32 limbs)
   constexpr int NB = sizeof(ST) == 4 ? 2 : 1;            // int64 limbs: one buffer (shared memory), no overlap
   __shared__ __align__(16) Z4<ST> sP[TB_WARPS][NB][E];  // the entry's parent, and the next entry's arriving
   __shared__ Z4<ST> sC[TB_WARPS][E];
+  __shared__ int4 sY[PACKED ? TB_WARPS : 1][PACKED ? E : 1];
   __shared__ uint64_t W[E];
-  __shared__ DevSpec sps[TB_WARPS];
+  __shared__ DevSpec s_sp;
+  const unsigned long long n = a.st->n_tq < a.tqcap ? a.st->n_tq : a.tqcap;
+  const unsigned long long stride = (unsigned long long)gridDim.x * TB_WARPS;
+  if ((unsigned long long)blockIdx.x * TB_WARPS >= n) return;
   init_weights(W, E);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Z4<ST> *C = sC[w];
   // the search's spec is copied to shared memory once; a batch's entries read their job's spec where it lies (the
   // entries of a many-job chunk change job often, and the specs stay in cache)
   unsigned conjmask = 0;
   if constexpr (!BATCHED) {
-    for (int i = lane; i < (int)(sizeof(DevSpec) / 4); i += 32) ((int *)&sps[w])[i] = ((const int *)&sp0)[i];
-    __syncwarp();
-    for (int i = 0; i < sps[w].nsym; i++) conjmask |= (unsigned)(sps[w].symconj[i] != 0) << i;
+    for (int i = threadIdx.x; i < (int)(sizeof(DevSpec) / 4); i += blockDim.x) ((int *)&s_sp)[i] = ((const int *)&sp0)[i];
+    for (int i = 0; i < sp0.nsym; i++) conjmask |= (unsigned)(sp0.symconj[i] != 0) << i;
   }
-  const DevSpec *spp = &sps[w];
-  const unsigned long long n = a.st->n_tq < a.tqcap ? a.st->n_tq : a.tqcap;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  Z4<ST> *C = sC[w];
+  const DevSpec *spp = &s_sp;
   WarpTally c;
   int job = -2, rem = a.rem;
   bool keep = a.keep != 0;
-  // entries are taken one ahead: the next entry's parent residual is copied into shared memory asynchronously
+  // entries are read one ahead: the next entry's parent residual is copied into shared memory asynchronously
   // (cp.async) while the current entry's T bound runs
-  auto take = [&](TQEntry &q, int b) {
-    unsigned long long e = 0;
-    if (lane == 0) e = atomicAdd(&a.st->tq_work, 1ULL);
-    e = __shfl_sync(FULL, e, 0);
+  auto take = [&](TQEntry &q, unsigned long long e, int b) {
     if (e >= n) return false;
     q = a.tq[e];
     const char *src = (const char *)(a.R + q.p * (unsigned long long)E);
@@ -1449,13 +1563,15 @@ __global__ void __launch_bounds__(TB_WARPS * 32) k_tbound(const __grid_constant_
   };
   TQEntry q;
   int b = 0;
-  bool have = take(q, 0);
+  unsigned long long e = (unsigned long long)blockIdx.x * TB_WARPS + w;
+  bool have = take(q, e, 0);
   cp_async_commit();
   while (have) {
     TQEntry q2;
     bool more = false;
+    e += stride;
     if constexpr (NB == 2) {
-      more = take(q2, b ^ 1);
+      more = take(q2, e, b ^ 1);
       cp_async_commit();
       cp_async_wait<1>();                            // this entry's parent has arrived (the next may be in flight)
     } else {
@@ -1475,21 +1591,37 @@ __global__ void __launch_bounds__(TB_WARPS * 32) k_tbound(const __grid_constant_
         for (int i = 0; i < spp->nsym; i++) conjmask |= (unsigned)(spp->symconj[i] != 0) << i;
       }
     }
-    const DevSpec &sp = BATCHED ? *spp : sps[w];
+    const DevSpec &sp = *spp;
     const NodeMeta pm = a.meta[q.p];
-    int T = 0;
+    auto alive = [&](int T, int s2) {
+      return sp.lite ? q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem
+                     : combine(q.k > q.hs ? q.k : q.hs, T, q.c2, __popc(q.ntriv[s2])) <= rem;
+    };
+    bool ovf;
+    (void)warp_child<NQ, ST>(P, C, q.g[0], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
+    __syncwarp();
+    int T;
+    bool packed = false;
+    if constexpr (PACKED) packed = sp.unit && NQ + q.k <= PACK_MAX;
+    if (packed) {
+#pragma unroll
+      for (int j = 0; j < (E >= 32 ? E / 32 : 1); j++)
+        if (lane + 32 * j < E) sY[w][lane + 32 * j] = pack_entry(C[lane + 32 * j]);
+      __syncwarp();
+      T = packed_tbound<NQ>(sY[w], q.k, lane, [&](int t) { return !alive(t, 0) && (q.n < 2 || !alive(t, 1)); });
+    } else {
+      T = PACKED ? warp_tbound_slim<NQ, ST>(C, q.k, lane) : ptm_bound<NQ, ST>(C, q.k, lane);
+    }
+    c.teval++;
     for (int s2 = 0; s2 < q.n; s2++) {
-      bool ovf;
-      __syncwarp();
-      (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
-      __syncwarp();
-      if (s2 == 0) { T = ptm_bound<NQ, ST>(C, q.k, lane); c.teval++; }
-      bool alive;
-      if (sp.lite) alive = q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem;
-      else alive = combine(q.k > q.hs ? q.k : q.hs, T, q.c2, __popc(q.ntriv[s2])) <= rem;
-      if (!alive) { c.dead++; continue; }
+      if (!alive(T, s2)) { c.dead++; continue; }
       c.alive++;
       if (!keep) continue;
+      if (s2) {                                      // the sibling's residual
+        __syncwarp();
+        (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);
+        __syncwarp();
+      }
       uint64_t k1, k2;
       warp_class_key<NQ, ST>(C, q.k, sp.nsym, conjmask, sp.symperm, W, lane, k1, k2);
       unsigned long long slot = 0;
@@ -1511,7 +1643,7 @@ __global__ void __launch_bounds__(TB_WARPS * 32) k_tbound(const __grid_constant_
     }
     __syncwarp();                                    // every lane is done with this buffer before it is refilled
     if constexpr (NB == 1) {
-      more = take(q2, 0);
+      more = take(q2, e, 0);
       cp_async_commit();
     }
     have = more;
@@ -3382,6 +3514,22 @@ int Engine::Impl::run_mitm(const HostSpec &hs, const Options &opt, const std::fu
   return rc;
 }
 
+// M M^dag = 2^k I exactly (an N x N matrix of Z[w] entries over sqrt2^k); large coefficients count as not unitary
+bool unitary(const Zw *M, int N, int k) {
+  if (k < 0 || k > 40) return false;
+  constexpr int64_t LIM = (int64_t)1 << 20;
+  for (int e = 0; e < N * N; e++)
+    for (int64_t v : {M[e].a, M[e].b, M[e].c, M[e].d})
+      if (v > LIM || v < -LIM) return false;
+  for (int r = 0; r < N; r++)
+    for (int r2 = 0; r2 < N; r2++) {
+      Zw s{0, 0, 0, 0};
+      for (int c = 0; c < N; c++) s = zadd(s, zmul(M[r * N + c], zconj(M[r2 * N + c])));
+      if (!zeq(s, Zw{r == r2 ? (int64_t)1 << k : 0, 0, 0, 0})) return false;
+    }
+  return true;
+}
+
 // host part of the device spec: every field, plus the gate-matrix (gi) and goal (gl) tables to place on the device
 template <int NQ>
 DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool nogoal, std::vector<int4> &gi,
@@ -3453,6 +3601,8 @@ DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool no
       gl[2 * (r * N + c)] = make_longlong2(r == c ? 1 : 0, 0);
       gl[2 * (r * N + c) + 1] = make_longlong2(0, 0);
     }
+  sp.unit = !hs.states && unitary(hs.target.data(), N, hs.tk);
+  for (int g = 0; g < hs.G; g++) sp.unit = sp.unit && unitary(hs.ginv[g].data(), 1 << hs.gnq[g], hs.gik[g]);
   sp.states = hs.states;
   sp.m = hs.states ? hs.m : N;
   if (hs.states) {                     // the goal: the reference's rows over sqrt2^gk, compared exactly

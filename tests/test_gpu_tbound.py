@@ -1,0 +1,60 @@
+"""The T bound's packed form (unitary residuals with qubits + exponent up to 7: four components to a register, the
+entries that are already dead left early) and the general form beside it, through whole searches against the C
+restatement: targets whose residuals lie on both sides of the limit, and a target that is not unitary (general form
+throughout). Counts are whole numbers and must be equal."""
+import random
+
+import pytest
+
+import cheese_b200 as cz
+from cheese_b200 import workloads
+from conftest import run_oracle, spec_text
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    e = cz.Engine(0)
+    yield e
+    e.close()
+
+
+def target(seed):
+    """a circuit rich in H and T gates: residual exponents 4 (2 qubits) and 5 (3 qubits) at the root"""
+    rng = random.Random(seed)
+    n = 3 if seed % 3 else 2
+    circ = []
+    for _ in range(rng.randint(10, 16)):
+        g = rng.choice(["h", "h", "h", "h", "cx", "cx", "t", "t"])
+        circ.append((g, tuple(rng.sample(range(n), 2)) if g == "cx" else (rng.randrange(n),)))
+    return n, circ
+
+
+@pytest.mark.parametrize("seed,exponent,budget", [(85, 5, 10), (509, 5, 12), (581, 5, 12), (2740, 5, 12),
+                                                  (303, 4, 10), (2046, 4, 10)])
+def test_exponents_around_the_packed_limit(engine, oracle_bin, tmp_path, seed, exponent, budget):
+    n, circ = target(seed)
+    assert workloads.unitary(n, circ)[0] == exponent
+    text = workloads.make_spec(n, circ, budget)
+    p = tmp_path / "t.spec"
+    p.write_text(text)
+    rc, lines = run_oracle(oracle_bin, p, [])
+    out = engine.search(text)
+    assert (out.rc, out.lines()) == (rc, lines)
+    assert out.raw.t_evals > 0
+
+
+def test_target_that_is_not_unitary(engine, oracle_bin, tmp_path):
+    text = spec_text("toffoli")
+    head, rest = text.split("\ntarget ", 1)
+    rows = rest.split("\n")
+    for r in range(1, 9):                       # the rows of the target, every entry times 3
+        rows[r] = " ".join(str(3 * int(v)) for v in rows[r].split())
+    text = head + "\ntarget " + "\n".join(rows)
+    p = tmp_path / "t.spec"
+    p.write_text(text)
+    rc, lines = run_oracle(oracle_bin, p, ["--depth", "9"])
+    out = engine.search(text, depth=9)
+    assert (out.rc, out.lines()) == (rc, lines)
+    assert out.raw.t_evals > 0
