@@ -61,6 +61,8 @@ CZ_HD bool fits32(int64_t v) { return v >= INT32_MIN && v <= INT32_MAX; }
 //  GF_TDIAG:    one-qubit diagonal with an odd w-power ratio (all such gates on a qubit give the same T bound:
 //               they differ by a power of S, a Clifford)
 //  GF_RANK2:    two-qubit gate of operator-Schmidt rank <= 2 over F_p (cx, cz: the CX bound moves by at most 1)
-enum GateFlag : uint8_t { GF_CLIFFORD = 1, GF_ONEQ = 2, GF_MONAFF = 4, GF_TDIAG = 8, GF_RANK2 = 16 };
+//  GF_UNITMON:  monomial with w-power entries over sqrt2^0: the entries of S g^-1 are those of S, columns permuted and
+//               multiplied by units, so the exponent stays (device specs only)
+enum GateFlag : uint8_t { GF_CLIFFORD = 1, GF_ONEQ = 2, GF_MONAFF = 4, GF_TDIAG = 8, GF_RANK2 = 16, GF_UNITMON = 32 };
 
 }  // namespace cz

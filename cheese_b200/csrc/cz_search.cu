@@ -33,6 +33,7 @@
 #include <map>
 #include <mutex>
 #include <stdexcept>
+#include <type_traits>
 
 #include "cz_engine.h"
 #include "cz_sort.cuh"
@@ -46,8 +47,11 @@ constexpr int RC_STOP = -3;        // levels(): stopped after the requested leve
 constexpr int EXP_WARPS = 8;       // warps per expand block
 constexpr int EXP_MINB = 4;        // expand blocks per SM: 32 warps (64 registers; latency-bound code, measured
                                    // 6 % faster than 2 blocks of 128 registers despite small spills)
+constexpr int EXPB_MINB = 3;       // batched: 3 blocks of 80 registers as fast as 4 of 64 with more spills, or 2
 constexpr int INHERIT_KMAX = 60;
 enum GateKind : uint8_t { GK_GENERAL = 0, GK_ONEQ = 1, GK_PERM = 2 };   // the T bound is computed exactly (mod 2^32 / 2^64) only while 2(n + k) <= 128
+
+constexpr uint8_t QC_NONE = 0xff;
 
 // ---------------- device-side spec ----------------
 struct DevSpec {
@@ -61,6 +65,8 @@ struct DevSpec {
   uint8_t gmask[GMAX];                 // qubits a gate acts on
   uint8_t gkind[GMAX];                 // GK_*: how the child update multiplies by the gate
   uint8_t gph[GMAX][4];                // one-qubit unit gates: w-power of ginv[m][lc] at [2 m + lc] (8: zero)
+  uint8_t gmono[GMAX][8];              // GF_UNITMON gates: column c of S g^-1 is column src of S times w^p: src | p << 4
+  uint8_t qcut[3];                     // per qubit: bit offset in NodeMeta.needs of the cut around it, QC_NONE if none
   uint8_t gperm[GMAX][8];              // permutation gates: local column lc takes local row gperm[lc]
   int goal_id;                         // the goal is the identity with exponent 0 (unitary targets)
   int8_t gnq[GMAX], gik[GMAX];
@@ -302,7 +308,7 @@ template <typename ST> __device__ __forceinline__ int4 pack_entry(const Z4<ST> &
 }
 // OR of the output bytes of pair f (0 for f = 0); the point map as in tbound_round
 template <int NQ, bool IDENT>
-__device__ __forceinline__ unsigned packed_round(const int4 *Y, int f) {
+__device__ __forceinline__ unsigned packed_round(const int4 *Y, const int *X, int f) {
   constexpr int E = 1 << (2 * NQ), HP = E / 2;
   if (f == 0) return 0;
   const int lomask = IDENT ? E - 1 : ((f & HP) ? E - 1 : (f & -f) - 1);
@@ -311,7 +317,7 @@ __device__ __forceinline__ unsigned packed_round(const int4 *Y, int f) {
   for (int i = 0; i < HP; i++) {
     const int e = IDENT ? i : (i & lomask) | ((i & ~lomask) << 1);
     const int4 y = Y[e];
-    const int x = Y[e ^ f].x;
+    const int x = X[e ^ f];              // the first words again, one per bank
     int s = __dp4a(x, y.w, 0);
     s = __dp4a(x, y.z, s << 8);
     s = __dp4a(x, y.y, s << 8);
@@ -343,20 +349,20 @@ __device__ __forceinline__ void unpack_or(unsigned o, unsigned &O1, unsigned &O2
   O2 = ((o | (o >> 8)) & 0x7fu) << 1;
   O1 = O2 | (((o >> 16) | (o >> 24)) & 0x7fu);
 }
-// T bound of the residual packed in Y (E words). At 3 qubits the 32 pairs f >= 32 come first: `dead(T)` says whether
-// a bound of T already decides the entry (bounds only grow with further pairs); then the rest is left out and T is a
-// lower bound. On the deep proofs 92 % of the entries are dead and these 32 pairs show it for every one of them.
-template <int NQ, typename Dead>
-__device__ __forceinline__ int packed_tbound(const int4 *Y, int k, int lane, Dead dead) {
+// T bound of the residual packed in Y and X (E words). At 3 qubits the 32 pairs f >= 32 come first: a bound above thr
+// already decides the entry (bounds only grow with further pairs); then the rest is left out and the result is a
+// lower bound above thr. On the deep proofs 92 % of the entries are dead and these 32 pairs show it for every one.
+template <int NQ>
+__device__ __forceinline__ int packed_tbound(const int4 *Y, const int *X, int k, int lane, int thr) {
   constexpr int E = 1 << (2 * NQ), PL = E > 32 ? E / 32 : 1;
   unsigned o = 0, O1, O2;
   if constexpr (E == 64) {
-    o = __reduce_or_sync(FULL, packed_round<NQ, true>(Y, 32 + lane));
+    o = __reduce_or_sync(FULL, packed_round<NQ, true>(Y, X, 32 + lane));
     unpack_or(o, O1, O2);
     const int T = bound_of<NQ>(O1, O2, k);
-    if (dead(T)) return T;
+    if (T > thr) return T;
   }
-  o |= packed_round<NQ, false>(Y, lane < E ? lane : 0);
+  o |= packed_round<NQ, false>(Y, X, lane < E ? lane : 0);
   // f = 0: alpha + 2^16 beta over all E points across the warp (|alpha| <= 2^7, |beta| < 2^7)
   int v[PL];
 #pragma unroll
@@ -436,9 +442,10 @@ template <typename ST> __device__ __forceinline__ uint32_t to_fp(const Z4<ST> &x
 // (output bit, input bit) of the cut qubit, columns those of the other qubits. The matrices of 32 / (E/4) cuts are
 // eliminated side by side, one column per lane: per row a ballot finds the group's pivot column, and the rows
 // below are reduced by it. Returns the bound and packs the child's needs (2 bits per cut) into needs_out.
-template <int NQ, typename ST>
-__device__ __forceinline__ int warp_cx_bound(const Z4<ST> *S, const DevSpec &sp, int lane, int gmask, int needs_in,
-                                          int &needs_out) {
+// elem(o, i): the F_p image of the residual's entry in row o, column i.
+template <int NQ, typename Elem>
+__device__ __forceinline__ int warp_cx_elems(Elem elem, const DevSpec &sp, int lane, int gmask, int needs_in,
+                                             int &needs_out) {
   constexpr int N = 1 << NQ, CC = N * N / 4 > 0 ? N * N / 4 : 1, SLOTS = 32 / CC, ALLQ = N - 1;
   static_assert(NQ <= 3, "cuts of one qubit: 4 x E/4 matrices within a warp");
   const bool inherit = sp.ncuts <= 4 && gmask;
@@ -466,7 +473,7 @@ __device__ __forceinline__ int warp_cx_bound(const Z4<ST> *S, const DevSpec &sp,
         if ((A >> q) & 1) { o |= ((rr >> 1) & 1) << q; i |= (rr & 1) << q; }
         else { o |= ((col >> (NQ - 1 + nb)) & 1) << q; i |= ((col >> nb) & 1) << q; nb++; }
       }
-      v[rr] = mycut >= 0 ? to_fp(S[o * N + i], sp) : 0u;
+      v[rr] = mycut >= 0 ? elem(o, i) : 0u;
     }
     const unsigned group = (CC >= 32 ? FULL : ((1u << CC) - 1u)) << (slot * CC);
     int rank = 0;
@@ -503,14 +510,16 @@ __device__ __forceinline__ int warp_cx_bound(const Z4<ST> *S, const DevSpec &sp,
   return sp.have_table && idx < sp.ncx ? __ldg(&sp.cxtable[idx]) : mx;
 }
 
-__device__ __forceinline__ int combine(int h, int t, int c2, int supp) {   // cheese.cu:599-607
-  int best = 1 << 30;
-  const int hi = c2 > supp ? c2 : supp;
-  for (int c = c2; c <= hi; c++) {
-    const int one = (h + t > supp - 2 * c) ? h + t : supp - 2 * c;
-    if (c + one < best) best = c + one;
-  }
-  return best;
+template <int NQ, typename ST>
+__device__ __forceinline__ int warp_cx_bound(const Z4<ST> *S, const DevSpec &sp, int lane, int gmask, int needs_in,
+                                             int &needs_out) {
+  return warp_cx_elems<NQ>([&](int o, int i) { return to_fp(S[(o << NQ) + i], sp); }, sp, lane, gmask, needs_in, needs_out);
+}
+
+// the least c + max(h + t, supp - 2 c) over c >= c2 (cheese.cu:599-607): the second term falls by 2 per step of c until
+// it meets h + t, so the least c with supp - 2 c <= h + t is best, or c2 if that is larger
+__device__ __forceinline__ int combine(int h, int t, int c2, int supp) {
+  return max(c2, (max(supp - h - t, 0) + 1) >> 1) + h + t;
 }
 
 // x times w^p (p < 8): a signed rotation of the coefficients
@@ -530,6 +539,19 @@ __device__ __forceinline__ int4 mul_unit32(int4 x, int p) {
   int4 y = (p & 2) ? make_int4(-x.z, -x.w, x.x, x.y) : x;
   y = (p & 1) ? make_int4(-y.w, y.x, y.y, y.z) : y;
   return (p & 4) ? make_int4(-y.x, -y.y, -y.z, -y.w) : y;
+}
+
+// the same for any limb type
+template <typename ST> __device__ __forceinline__ Z4<ST> unit_mul(const Z4<ST> &x, int p) {
+  Z4<ST> y = (p & 2) ? Z4<ST>{(ST)-x.c, (ST)-x.d, x.a, x.b} : x;
+  y = (p & 1) ? Z4<ST>{(ST)-y.d, y.a, y.b, y.c} : y;
+  return (p & 4) ? Z4<ST>{(ST)-y.a, (ST)-y.b, (ST)-y.c, (ST)-y.d} : y;
+}
+// entry lane + 32 j of P g^-1 for a GF_UNITMON gate, mono = its gmono byte for the lane's column (entries lane and
+// lane + 32 are in one column)
+template <int NQ, typename ST> __device__ __forceinline__ Z4<ST> mono_entry(const Z4<ST> *P, int mono, int lane, int j) {
+  constexpr int N = 1 << NQ;
+  return unit_mul(P[((lane & ~(N - 1)) | (mono & 15)) + 32 * j], mono >> 4);
 }
 
 // normalise the lane's two entries (sqrt2 division while every entry allows it) and store them; returns k
@@ -558,6 +580,26 @@ struct I4 { int a, b, c, d; };
 __device__ __forceinline__ bool zdiv2ok(const I4 &x) { return !((x.a - x.c) & 1) && !((x.b - x.d) & 1); }
 __device__ __forceinline__ I4 zdown(const I4 &x) { return {(x.b - x.d) >> 1, (x.a + x.c) >> 1, (x.b + x.d) >> 1, (x.c - x.a) >> 1}; }
 __device__ __forceinline__ bool fits32(int) { return true; }
+
+// one-qubit unit gate: the two outputs of a column pair (entries ei of P), w-powers ph of the inverse at [2 m + lc]
+template <typename ST> __device__ __forceinline__ void oneq_pair(const Z4<ST> *P, const int (&ei)[2], const uint8_t *ph, I4 (&v)[2]) {
+  const int4 *P4 = (const int4 *)P;
+  const int4 x0 = P4[ei[0]], x1 = P4[ei[1]], z = make_int4(0, 0, 0, 0);
+  const int p00 = ph[0], p01 = ph[1], p10 = ph[2], p11 = ph[3];
+  const int4 a0 = p00 < 8 ? mul_unit32(x0, p00) : z, a1 = p10 < 8 ? mul_unit32(x1, p10) : z;
+  const int4 b0 = p01 < 8 ? mul_unit32(x0, p01) : z, b1 = p11 < 8 ? mul_unit32(x1, p11) : z;
+  v[0] = I4{a0.x + a1.x, a0.y + a1.y, a0.z + a1.z, a0.w + a1.w};
+  v[1] = I4{b0.x + b1.x, b0.y + b1.y, b0.z + b1.z, b0.w + b1.w};
+}
+// sqrt2 division of the warp's entries (zeros divide) while every one allows it; returns the exponent
+__device__ __forceinline__ int normalise_pair(I4 (&v)[2], int k) {
+  while (k > 0 && __all_sync(FULL, zdiv2ok(v[0]) && zdiv2ok(v[1]))) {
+    v[0] = zdown(v[0]);
+    v[1] = zdown(v[1]);
+    k--;
+  }
+  return k;
+}
 
 // child residual C = P g^-1, general gate: multiplies the local matrix out over Z[w] in int64
 template <int NQ, typename ST>
@@ -630,13 +672,7 @@ __device__ __forceinline__ int warp_child(const Z4<ST> *P, Z4<ST> *C, int g, int
     if (lane < E / 2) {
       ei[0] = ((lane & ~lo) << 1) | (lane & lo);
       ei[1] = ei[0] | (1 << q);
-      const int4 x0 = P4[ei[0]], x1 = P4[ei[1]];
-      const int p00 = sp.gph[g][0], p01 = sp.gph[g][1], p10 = sp.gph[g][2], p11 = sp.gph[g][3];
-      const int4 z = make_int4(0, 0, 0, 0);
-      const int4 a0 = p00 < 8 ? mul_unit32(x0, p00) : z, a1 = p10 < 8 ? mul_unit32(x1, p10) : z;
-      const int4 b0 = p01 < 8 ? mul_unit32(x0, p01) : z, b1 = p11 < 8 ? mul_unit32(x1, p11) : z;
-      v[0] = I4{a0.x + a1.x, a0.y + a1.y, a0.z + a1.z, a0.w + a1.w};
-      v[1] = I4{b0.x + b1.x, b0.y + b1.y, b0.z + b1.z, b0.w + b1.w};
+      oneq_pair(P, ei, sp.gph[g], v);
     }
   } else {   // GK_PERM
     const int nq = sp.gnq[g];
@@ -925,42 +961,35 @@ template <typename ST> __device__ __forceinline__ void entry_hash(const Z4<ST> &
   ha = fmix32(lo0 ^ hi);
   hb = fmix32(lo1 + (hi ^ 0x1b873593u));
 }
-template <int NQ, typename ST>
-__device__ __forceinline__ void warp_class_key(const Z4<ST> *S, int k, int nsym, unsigned conjmask, const uint8_t (*perm)[8],
-                                            const uint64_t *W, int lane, uint64_t &k1, uint64_t &k2) {
-  constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
-  static_assert(SYMMAX <= 16, "the reduce-scatter holds 16 elements x (A, B)");
-  uint32_t fa[EPL], fb[EPL], ca[EPL], cb[EPL];
-  int row[EPL], col[EPL];
+// x: the lane's two entries, at positions ei (negative: none; every position in one lane); weight(s, e): W[pi_s(e)].
+template <int NQ, typename ST, typename Weight>
+__device__ __forceinline__ void warp_key_entries(const Z4<ST> (&x)[2], const int (&ei)[2], int k, int nsym, unsigned conjmask,
+                                                 Weight weight, int lane, uint64_t &k1, uint64_t &k2) {
+  static_assert(SYMMAX == 12, "the reduce-scatter halves 12 elements twice and keeps 3 per lane");
+  uint32_t fa[2], fb[2], ca[2], cb[2];
 #pragma unroll
-  for (int j = 0; j < EPL; j++) {
-    const int e = lane + 32 * j;
-    fa[j] = fb[j] = ca[j] = cb[j] = 0;
-    row[j] = (e >> NQ) & (N - 1);
-    col[j] = e & (N - 1);
-    if (e >= E) continue;
-    const Z4<ST> x = S[e];
-    entry_hash(x, fa[j], fb[j]);
-    entry_hash(zcj(x), ca[j], cb[j]);
+  for (int j = 0; j < 2; j++) {
+    entry_hash(x[j], fa[j], fb[j]);
+    entry_hash(zcj(x[j]), ca[j], cb[j]);
+    if (ei[j] < 0) fa[j] = fb[j] = ca[j] = cb[j] = 0;
   }
-  uint32_t v[32];
+  uint32_t v[24];                            // A of element s at s, B at 12 + s
 #pragma unroll
-  for (int s = 0; s < 16; s++) {
-    v[s] = v[16 + s] = 0;
+  for (int s = 0; s < 12; s++) {
+    v[s] = v[12 + s] = 0;
     if (s >= nsym) continue;
     const bool cj = (conjmask >> s) & 1;
 #pragma unroll
-    for (int j = 0; j < EPL; j++) {
-      if (lane + 32 * j >= E) continue;
-      const uint64_t w = W[perm[s][row[j]] * N + perm[s][col[j]]];
+    for (int j = 0; j < 2; j++) {
+      const uint64_t w = weight(s, max(ei[j], 0));
       v[s] += (cj ? ca[j] : fa[j]) * (uint32_t)w;
-      v[16 + s] += (cj ? cb[j] : fb[j]) * (uint32_t)(w >> 32);
+      v[12 + s] += (cj ? cb[j] : fb[j]) * (uint32_t)(w >> 32);
     }
   }
-  // reduce-scatter: at offset o a lane keeps the half of its values on its side of lane bit o and adds the
-  // partner's copy of that half
+  // reduce-scatter: at offset o a lane keeps the half of its values on its side of lane bit o and adds the partner's
+  // copy of that half: A or B by bit 4, six elements by bit 3, three by bit 2, summed over bits 1 and 0
 #pragma unroll
-  for (int o = 16, n = 16; o; o >>= 1, n >>= 1) {
+  for (int o = 16, n = 12; o >= 4; o >>= 1, n >>= 1) {
     const bool up = lane & o;
 #pragma unroll
     for (int i = 0; i < n; i++) {
@@ -968,32 +997,59 @@ __device__ __forceinline__ void warp_class_key(const Z4<ST> *S, int k, int nsym,
       v[i] = keep + __shfl_xor_sync(FULL, give, o);
     }
   }
-  const uint32_t other = __shfl_xor_sync(FULL, v[0], 16);   // lane s < 16: A_s here, B_s from lane 16 + s
-  uint64_t x1 = ~0ULL, x2 = ~0ULL;
-  if (lane < nsym) {
-    x1 = fmix64((((uint64_t)v[0] << 32) | other) + (uint64_t)k * 0xa0761d6478bd642fULL);
-    x2 = fmix64(x1 ^ 0xe7037ed1a0b428dbULL);
-  }
 #pragma unroll
-  for (int m = 16; m; m >>= 1) {
-    const uint64_t o1 = __shfl_xor_sync(FULL, x1, m), o2 = __shfl_xor_sync(FULL, x2, m);
-    if (o1 < x1 || (o1 == x1 && o2 < x2)) { x1 = o1; x2 = o2; }
+  for (int i = 0; i < 3; i++) {
+    v[i] += __shfl_xor_sync(FULL, v[i], 2);
+    v[i] += __shfl_xor_sync(FULL, v[i], 1);
   }
-  k1 = x1; k2 = x2;
+  const int r = lane & 3, el = 6 * ((lane >> 3) & 1) + 3 * ((lane >> 2) & 1) + r;   // the lane's element (r < 3)
+  const uint32_t mine = r == 0 ? v[0] : (r == 1 ? v[1] : v[2]);
+  const uint32_t other = __shfl_xor_sync(FULL, mine, 16);                           // lanes < 16: A here, B there
+  uint64_t x1 = ~0ULL;
+  if (lane < 16 && r < 3 && el < nsym) x1 = fmix64((((uint64_t)mine << 32) | other) + (uint64_t)k * 0xa0761d6478bd642fULL);
+  const uint32_t hi = __reduce_min_sync(FULL, (uint32_t)(x1 >> 32));
+  const uint32_t lo = __reduce_min_sync(FULL, (uint32_t)(x1 >> 32) == hi ? (uint32_t)x1 : ~0u);
+  k1 = ((uint64_t)hi << 32) | lo;
+  k2 = fmix64(k1 ^ 0xe7037ed1a0b428dbULL);
+}
+// of the residual S in shared memory, the weights by position W through the group's basis maps
+template <int NQ, typename ST>
+__device__ __forceinline__ void warp_class_key(const Z4<ST> *S, int k, int nsym, unsigned conjmask, const uint8_t (*perm)[8],
+                                               const uint64_t *W, int lane, uint64_t &k1, uint64_t &k2) {
+  constexpr int N = 1 << NQ, E = N * N;
+  Z4<ST> x[2];
+  int ei[2];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    ei[j] = lane + 32 * j < E ? lane + 32 * j : -1;
+    x[j] = ei[j] >= 0 ? S[ei[j]] : Z4<ST>{0, 0, 0, 0};
+  }
+  warp_key_entries<NQ, ST>(x, ei, k, nsym, conjmask,
+                           [&](int s, int e) { return W[perm[s][e >> NQ] * N + perm[s][e & (N - 1)]]; }, lane, k1, k2);
 }
 
 template <int NQ, typename ST> struct ExpandSmem {
-  static constexpr int E = (1 << NQ) * (1 << NQ);
-  Z4<ST> P[EXP_WARPS][E];
+  static constexpr int E = (1 << NQ) * (1 << NQ), NB = sizeof(ST) == 4 ? 2 : 1;
+  Z4<ST> P[EXP_WARPS][NB][E];      // a warp's parent, and its next one arriving
   Z4<ST> C[EXP_WARPS][E];
-  uint64_t W[E];
-  uint8_t perm[SYMMAX][8];
+  uint64_t Wt[SYMMAX][E];          // the class key's weights per group element, W[pi_s(e)]
+  uint32_t F[EXP_WARPS][E];        // the parent's entries in F_p
 };
 
 // the class key's position weights: (weight A, weight B), both odd
+__device__ __forceinline__ uint64_t key_weight(int pos) {
+  return fmix64(0x243f6a8885a308d3ULL + (uint64_t)pos * 0x13198a2e03707345ULL) | 0x0000000100000001ULL;
+}
 __device__ __forceinline__ void init_weights(uint64_t *W, int E) {
-  for (int i = threadIdx.x; i < E; i += blockDim.x)
-    W[i] = fmix64(0x243f6a8885a308d3ULL + (uint64_t)i * 0x13198a2e03707345ULL) | 0x0000000100000001ULL;
+  for (int i = threadIdx.x; i < E; i += blockDim.x) W[i] = key_weight(i);
+}
+// the same for every element of the symmetry group, through its basis maps
+template <int NQ> __device__ __forceinline__ void init_group_weights(uint64_t (*Wt)[(1 << NQ) * (1 << NQ)], const DevSpec &sp) {
+  constexpr int N = 1 << NQ, E = N * N;
+  for (int i = threadIdx.x; i < sp.nsym * E; i += blockDim.x) {
+    const int s = i / E, e = i % E;
+    Wt[s][e] = key_weight(sp.symperm[s][e >> NQ] * N + sp.symperm[s][e & (N - 1)]);
+  }
 }
 
 // ---------------- the level kernel ----------------
@@ -1030,24 +1086,43 @@ template <typename ST> struct ExpandOut {
 
 // every child of parent p (residual already in P): window rules, exact prechecks, child residual, bounds, class key,
 // survivor append. sp is the parent's spec (kernel parameter or a shared copy), sps its shared-memory address for
-// the out-of-line helpers; child index = p * GS + g.
+// the out-of-line helpers; child index = p * GS + g; F: the warp's room for the parent's F_p image; weight: the class
+// key's weights.
 // PART: 0 every candidate; 1 the one-qubit gates; 2 the multi-qubit gates. The plain level runs the two parts as
 // two launches: each warp then walks the code of one kind of child (instruction fetch is the level kernel's main
 // stall; measured 3 % faster than one launch), at the price of reading each parent twice. (Three parts, the odd
 // diagonals on their own, measured slower than one.)
-template <int NQ, typename ST, bool STATES = false, int PART = 0>
-__device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *sps, const uint8_t (*perm)[8],
-                                              unsigned conjmask, const uint64_t *W,
-                                              const Z4<ST> *P, Z4<ST> *C, unsigned long long p, const NodeMeta pm,
-                                              int rem, bool keep, int GS, const ExpandOut<ST> &o, WarpTally &c,
-                                              int lane) {
+//
+// Most children never have their residual computed. When the cut around a gate's qubit has F_p Schmidt rank >= 2 the
+// parent is no product there, so no gate on that qubit alone makes it act trivially: the support of a one-qubit child is
+// the parent's. A unit monomial (x z s sdg t tdg) keeps the exponent, one-qubit gates the CX bound, affine monomials
+// the H structure and Cliffords the T bound, so such a child's bounds are the parent's own: the Clifford ones are decided
+// one per lane, the odd diagonals queued one per lane. A two-qubit permutation (cx) changes only the ranks of the cuts it
+// crosses; they are eliminated straight from the parent's F_p image (computed once per parent) with its columns permuted.
+// Only survivors' entries are then formed, in registers, for the class key. Deep
+// proofs (budget 12, two targets, 2.74 M parents): both parts 19.9 -> 12.6 ms; bound by issue (80 %) and, for the one-qubit
+// part, by instruction fetch.
+template <int NQ, typename ST, bool STATES = false, int PART = 0, typename Weight>
+__device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *sps, Weight weight, unsigned conjmask,
+                                              const Z4<ST> *P, Z4<ST> *C, uint32_t *F, unsigned long long p,
+                                              const NodeMeta pm, int rem, bool keep, int GS, const ExpandOut<ST> &o,
+                                              WarpTally &c, int lane) {
   constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
   const int G = sp.G;
   const int g1 = pm.g1 == 0xff ? -1 : pm.g1, g2 = pm.g2 == 0xff ? -1 : pm.g2;
   const int kP = pm.k, TP = pm.T, c2P = pm.c2, hsP = (pm.hsn & 1) ? 2 : 0, ntP = (pm.hsn >> 1) & 7;
   const int suppP = __popc(ntP);
-  const bool pre_ok = sp.standard && !sp.states && kP < INHERIT_KMAX;
+  const bool pre_ok = !STATES && sp.standard && !sp.states && kP < INHERIT_KMAX;
+  // the cut around qubit q has rank >= 2 (needs as packed in NodeMeta)
+  auto entangled = [&](int q, int needs) { const int b = sps->qcut[q]; return b != QC_NONE && ((needs >> b) & 3) != 0; };
   unsigned long long pend[3] = {0, 0, 0};    // per qubit: 1 + queue entry of its deferred odd-diagonal child
+  auto put_entry = [&](unsigned long long e, int ga, int gb, int n, int k, int c2, int needs, int hs, int ntriv) {
+    TQEntry q;
+    q.p = p; q.k = (int16_t)k; q.n = (uint8_t)n; q.g[0] = (uint8_t)ga; q.g[1] = (uint8_t)gb; q.c2 = (uint8_t)c2;
+    q.needs = (uint8_t)needs; q.hs = (uint8_t)hs; q.ntriv[0] = (uint8_t)ntriv; q.ntriv[1] = n > 1 ? (uint8_t)ntriv : 0;
+    q.pad[0] = q.pad[1] = q.pad[2] = q.pad[3] = 0;
+    o.tq[e] = q;
+  };
   // queue a deferred T evaluation: a second odd diagonal on the same qubit joins its sibling's entry
   auto defer = [&](int g, int k, int c2, int needs, int hs, int ntriv, int q0, bool tdiag) {
     if (tdiag && pend[q0]) {
@@ -1060,126 +1135,224 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
     if (lane == 0) e = atomicAdd(&o.st->n_tq, 1ULL);
     e = __shfl_sync(FULL, e, 0);
     if (e >= o.tqcap) return;                // counted: the host redoes the level with room for every entry
-    if (lane == 0) {
-      TQEntry q;
-      q.p = p; q.k = (int16_t)k; q.n = 1; q.g[0] = (uint8_t)g; q.g[1] = 0xff; q.c2 = (uint8_t)c2;
-      q.needs = (uint8_t)needs; q.hs = (uint8_t)hs; q.ntriv[0] = (uint8_t)ntriv; q.ntriv[1] = 0;
-      q.pad[0] = q.pad[1] = q.pad[2] = q.pad[3] = 0;
-      o.tq[e] = q;
-    }
+    if (lane == 0) put_entry(e, g, 0xff, 1, k, c2, needs, hs, ntriv);
     if (tdiag) pend[q0] = e + 1;
   };
   // the fates decided without the child's residual, one candidate per lane: window cuts (W2, W3) and the exact
   // prechecks. Lower bounds on the child's bounds from the parent's: k drops by at most the gate's sqrt2 exponent;
   // H structure, T and CX bounds are unchanged by monomial-affine / Clifford / one-qubit gates; an odd diagonal
   // changes T by at most 1; a gate of Schmidt rank 2 changes the CX bound by at most 1; support changes only on
-  // the gate's qubits. combine is monotone in every argument, so exceeding the budget with these proves the child
-  // dead (the goal has all bounds 0 and is never removed here). The other children are evaluated in order.
-  unsigned long long full = 0;
+  // the gate's qubits (not at all under a one-qubit gate on an entangled one). combine is monotone in every argument,
+  // so exceeding the budget with these proves the child dead (the goal has all bounds 0 and is never removed here).
+  // The other children are decided as their kind allows, or evaluated in order.
+  enum { NONE, W2, W3, DEADP, QUEUE, FULLC, ALIVEP, RANKS, HADA };
+  const bool need_b = sp.standard != 0 && !sp.states;
   for (int g0 = 0; g0 < G; g0 += 32) {
     const int g = g0 + lane;
-    int fate = 0;                            // 0: no candidate, 1: W2 cut, 2: W3 cut, 3: dead by precheck, 4: full
+    int fate = NONE, q0 = 0;
     if (g < G && (PART == 0 || ((sp.gflags[g] & GF_ONEQ) != 0) == (PART == 1))) {
-      fate = 4;
-      if (g1 >= 0 && __ldg(&sp.bad2[g1 * G + g])) fate = 1;
+      fate = FULLC;
+      if (g1 >= 0 && __ldg(&sp.bad2[g1 * G + g])) fate = W2;
       else if (g2 >= 0) {
         const uint32_t tri = ((uint32_t)g2 * G + (uint32_t)g1) * G + (uint32_t)g;
-        if ((__ldg(&sp.bad3[tri >> 5]) >> (tri & 31)) & 1) fate = 2;
+        if ((__ldg(&sp.bad3[tri >> 5]) >> (tri & 31)) & 1) fate = W3;
       }
-      if (fate == 4 && pre_ok) {
+      if (fate == FULLC && pre_ok) {
         const uint8_t fl = sps->gflags[g];
+        q0 = sps->gq[g][0];
         const int ik = sps->gik[g] > 0 ? sps->gik[g] : 0;
+        const bool oneq = fl & GF_ONEQ, ent = oneq && entangled(q0, pm.needs);
         int hlo = kP - ik;
         if ((fl & GF_MONAFF) && hsP > hlo) hlo = hsP;
         const int tlo = (fl & GF_CLIFFORD) ? TP : ((fl & GF_TDIAG) ? TP - 1 : 0);
-        const int clo = (fl & GF_ONEQ) ? c2P : ((fl & GF_RANK2) ? c2P - 1 : 0);
-        const int slo = suppP - sps->gnq[g];
-        if (combine(max(hlo, 0), max(tlo, 0), max(clo, 0), max(slo, 0)) > rem) fate = 3;
-      }
-    }
-    c.w2 += __popc(__ballot_sync(FULL, fate == 1));
-    c.w3 += __popc(__ballot_sync(FULL, fate == 2));
-    c.child += __popc(__ballot_sync(FULL, fate >= 3));
-    c.dead += __popc(__ballot_sync(FULL, fate == 3));
-    full |= (unsigned long long)__ballot_sync(FULL, fate == 4) << g0;
-  }
-  const bool need_b = sp.standard != 0 && !sp.states;
-  for (; full; full &= full - 1) {
-    const int g = __ffsll((long long)full) - 1;
-    const uint8_t fl = sp.gflags[g];
-    const int gm = sp.gmask[g], q0 = sp.gq[g][0];
-    bool ovf;
-    c.full++;
-    const int k = warp_child<NQ, ST, PART>(P, C, g, kP, sp, sps, lane, ovf);
-    if (ovf) { c.ovf = true; continue; }
-    const bool need_hs = need_b && !(fl & GF_MONAFF);
-    // the child is the goal only if the parent equals the gate, i.e. acts on no other qubit (unitary targets)
-    const Cheap ch = warp_cheap<NQ, ST>(C, k, sp, lane, (ntP & ~gm) == 0 || !need_b, need_hs, need_b ? gm : 0, ntP);
-    if (ch.goal) {
-      if (sp.nogoal) c.dead++;
-      else { c.found++; const unsigned long long oi = p * (unsigned long long)GS + g; if (oi < c.first) c.first = oi; }
-      continue;
-    }
-    const bool inheritT = (fl & GF_CLIFFORD) && k <= INHERIT_KMAX && kP <= INHERIT_KMAX;
-    const bool cacheT = (fl & GF_TDIAG) && k <= INHERIT_KMAX;
-    bool alive = true;
-    int T = 0, c2 = 0, hs = 0, needs = 0;
-    if constexpr (STATES) {                    // state targets (cheese.cu:683-716): no inherited bounds
-      if (sp.standard || sp.lite) {
-        int h = k;
-        if (!sp.lite) warp_state_cheap<NQ, ST>(C, k, *sps, lane, h, c2);
-        if (combine(h, 0, c2, 0) > rem) alive = false;
-        else {
-          T = warp_state_t<NQ, ST>(C, *sps, lane); c.teval++;
-          alive = combine(h, T, c2, 0) <= rem;
+        const int clo = oneq ? c2P : ((fl & GF_RANK2) ? c2P - 1 : 0);
+        const int slo = ent ? suppP : suppP - sps->gnq[g];
+        if (combine(max(hlo, 0), max(tlo, 0), max(clo, 0), max(slo, 0)) > rem) fate = DEADP;
+        else if (!sp.lite && (fl & (GF_UNITMON | GF_MONAFF)) == (GF_UNITMON | GF_MONAFF)) {
+          if (PART != 2 && ent) {
+            if (fl & GF_CLIFFORD) fate = ALIVEP;             // every bound above was exact
+            else if (fl & GF_TDIAG) fate = QUEUE;
+          } else if (PART != 1 && !oneq && (fl & GF_CLIFFORD) && sps->gkind[g] == GK_PERM && sps->gnq[g] == 2 &&
+                     (ntP & ~sps->gmask[g])) {               // (else the child may be the goal)
+            fate = RANKS;
+          }
+        } else if (PART != 2 && !sp.lite && sp.unit && ent && (fl & GF_CLIFFORD) && sps->gkind[g] == GK_ONEQ &&
+                   sizeof(ST) == 4 && kP <= 56) {
+          fate = HADA;
         }
       }
-    } else if (sp.lite) {
-      if (k > rem) alive = false;
-      else {
-        if (inheritT) T = TP;
-        else { defer(g, k, 0, 0, 0, 0, q0, cacheT && (fl & GF_ONEQ) && k == kP); continue; }
-        alive = k + (T + sp.tdiv - 1) / sp.tdiv <= rem;
+    }
+    c.w2 += __popc(__ballot_sync(FULL, fate == W2));
+    c.w3 += __popc(__ballot_sync(FULL, fate == W3));
+    c.child += __popc(__ballot_sync(FULL, fate >= DEADP));
+    c.dead += __popc(__ballot_sync(FULL, fate == DEADP));
+    unsigned todo = __ballot_sync(FULL, fate >= FULLC);
+    if constexpr (!STATES && PART != 2) {
+      const unsigned m = __ballot_sync(FULL, fate == ALIVEP);
+      if (!keep) { c.alive += __popc(m); todo &= ~m; }        // counted only
+      if (__ballot_sync(FULL, fate == QUEUE)) {
+        // the odd diagonals of one qubit two by two (their T bounds agree: they differ by a power of S)
+        const unsigned peers = __match_any_sync(FULL, fate == QUEUE ? q0 : 8), below = (1u << lane) - 1;
+        const bool lead = fate == QUEUE && !(__popc(peers & below) & 1);
+        const unsigned leads = __ballot_sync(FULL, lead);
+        unsigned long long e = 0;
+        if (lane == 0) e = atomicAdd(&o.st->n_tq, (unsigned long long)__popc(leads));
+        e = __shfl_sync(FULL, e, 0) + __popc(leads & below);
+        if (lead && e < o.tqcap) {           // (entries past the room are counted: the host redoes the level)
+          const unsigned after = peers & ~below & ~(1u << lane);
+          put_entry(e, g, after ? g0 + __ffs(after) - 1 : 0xff, after ? 2 : 1, kP, c2P, pm.needs, hsP, ntP);
+        }
       }
-    } else if (need_b) {
-      hs = need_hs ? ch.hs : hsP;
-      const int h = k > hs ? k : hs;
-      const int supp = __popc(ch.ntriv);
-      if (PART == 1 || (PART == 0 && (fl & GF_ONEQ))) { c2 = c2P; needs = pm.needs; }
-      else c2 = warp_cx_bound<NQ, ST>(C, *sps, lane, gm, pm.needs, needs);
-      if (combine(h, 0, c2, supp) > rem) alive = false;
-      else {
-        if (inheritT) T = TP;
-        else {
-          // siblings share an entry only when every bound but support is the parent's (one-qubit monomial gates)
-          const bool share = cacheT && (fl & GF_ONEQ) && (fl & GF_MONAFF) && k == kP;
-          defer(g, k, c2, needs, hs, ch.ntriv, q0, share);
+    }
+    if constexpr (!STATES && PART != 1) {
+      if (__ballot_sync(FULL, fate == RANKS)) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < EPL; j++)
+          if (lane + 32 * j < E) F[lane + 32 * j] = to_fp(P[lane + 32 * j], *sps);
+        __syncwarp();
+      }
+    }
+    for (; todo; todo &= todo - 1) {
+      const int g = g0 + __ffs(todo) - 1;
+      int kind = __shfl_sync(FULL, fate, g - g0);
+      const uint8_t fl = sp.gflags[g];
+      const int gm = sp.gmask[g], gq0 = sp.gq[g][0];
+      // the child's bounds (the parent's until shown otherwise) and the lane's entries of its residual
+      int k = kP, T = TP, c2 = c2P, hs = hsP, needs = pm.needs, ntriv = ntP, ei[2] = {-1, -1};
+      Z4<ST> x[2] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+      bool alive = true;
+      if (!STATES && PART != 1 && kind == RANKS) {
+        const uint8_t *mono = sps->gmono[g];
+        c2 = warp_cx_elems<NQ>([&](int r, int i) { return F[(r << NQ) + (mono[i] & 15)]; }, *sps, lane, gm, pm.needs, needs);
+        ntriv = ntP | gm;
+        if (!entangled(gq0, needs) || !entangled(sps->gq[g][1], needs)) kind = FULLC;   // one may have become trivial
+        else alive = combine(max(kP, hsP), TP, c2, __popc(ntriv)) <= rem;
+      }
+      if (!STATES && PART != 2 && kind == HADA) {
+        // a Hadamard-like Clifford on an entangled qubit: only the exponent is open (and, for a small one, the H
+        // structure: a unitary residual of exponent 1 or more in normal form is not monomial)
+        if constexpr (sizeof(ST) == 4) {
+          const int lo = (1 << gq0) - 1;
+          I4 v[2] = {I4{0, 0, 0, 0}, I4{0, 0, 0, 0}};
+          if (lane < E / 2) {
+            ei[0] = ((lane & ~lo) << 1) | (lane & lo);
+            ei[1] = ei[0] | (1 << gq0);
+            oneq_pair(P, ei, sps->gph[g], v);
+          }
+          k = normalise_pair(v, kP + sps->gik[g]);
+          c.full++;
+          if (k < 1) {
+            ei[0] = ei[1] = -1;
+            kind = FULLC;
+            c.full--;
+          } else {
+            hs = 0;
+            alive = combine(k, TP, c2P, suppP) <= rem;
+#pragma unroll
+            for (int j = 0; j < 2; j++) x[j] = Z4<ST>{(ST)v[j].a, (ST)v[j].b, (ST)v[j].c, (ST)v[j].d};
+          }
+        }
+      } else if (kind != FULLC) {
+        if (alive && keep) {
+          const int mono = sps->gmono[g][lane & (N - 1)];
+#pragma unroll
+          for (int j = 0; j < EPL; j++)
+            if (lane + 32 * j < E) {
+              ei[j] = lane + 32 * j;
+              x[j] = mono_entry<NQ>(P, mono, lane, j);
+            }
+        }
+      }
+      if (kind == FULLC) {
+        bool ovf;
+        c.full++;
+        k = warp_child<NQ, ST, PART>(P, C, g, kP, sp, sps, lane, ovf);
+        if (ovf) { c.ovf = true; continue; }
+        const bool need_hs = need_b && !(fl & GF_MONAFF);
+        // the child is the goal only if the parent equals the gate, i.e. acts on no other qubit (unitary targets); the
+        // qubit of a one-qubit gate stays non-trivial when it is entangled
+        const int test_q = !need_b || (pre_ok && (fl & GF_ONEQ) && entangled(gq0, pm.needs)) ? 0 : gm;
+        const Cheap ch = warp_cheap<NQ, ST>(C, k, sp, lane, (ntP & ~gm) == 0 || !need_b, need_hs, test_q, ntP);
+        if (ch.goal) {
+          if (sp.nogoal) c.dead++;
+          else {
+            c.found++;
+            const unsigned long long oi = p * (unsigned long long)GS + g;
+            if (oi < c.first) c.first = oi;
+          }
           continue;
         }
-        alive = combine(h, T, c2, supp) <= rem;
+        const bool inheritT = (fl & GF_CLIFFORD) && k <= INHERIT_KMAX && kP <= INHERIT_KMAX;
+        const bool cacheT = (fl & GF_TDIAG) && k <= INHERIT_KMAX;
+        T = 0; c2 = 0; hs = 0; needs = 0;
+        ntriv = need_b ? ch.ntriv : 0;
+        if constexpr (STATES) {                    // state targets (cheese.cu:683-716): no inherited bounds
+          if (sp.standard || sp.lite) {
+            int h = k;
+            if (!sp.lite) warp_state_cheap<NQ, ST>(C, k, *sps, lane, h, c2);
+            if (combine(h, 0, c2, 0) > rem) alive = false;
+            else {
+              T = warp_state_t<NQ, ST>(C, *sps, lane); c.teval++;
+              alive = combine(h, T, c2, 0) <= rem;
+            }
+          }
+        } else if (sp.lite) {
+          if (k > rem) alive = false;
+          else {
+            if (inheritT) T = TP;
+            else { defer(g, k, 0, 0, 0, 0, gq0, cacheT && (fl & GF_ONEQ) && k == kP); continue; }
+            alive = k + (T + sp.tdiv - 1) / sp.tdiv <= rem;
+          }
+        } else if (need_b) {
+          hs = need_hs ? ch.hs : hsP;
+          const int h = k > hs ? k : hs;
+          const int supp = __popc(ch.ntriv);
+          if (PART == 1 || (PART == 0 && (fl & GF_ONEQ))) { c2 = c2P; needs = pm.needs; }
+          else c2 = warp_cx_bound<NQ, ST>(C, *sps, lane, gm, pm.needs, needs);
+          if (combine(h, 0, c2, supp) > rem) alive = false;
+          else {
+            if (inheritT) T = TP;
+            else {
+              // siblings share an entry only when every bound but support is the parent's (one-qubit monomial gates)
+              const bool share = cacheT && (fl & GF_ONEQ) && (fl & GF_MONAFF) && k == kP;
+              defer(g, k, c2, needs, hs, ch.ntriv, gq0, share);
+              continue;
+            }
+            alive = combine(h, T, c2, supp) <= rem;
+          }
+        }
+        if (alive && keep) {
+#pragma unroll
+          for (int j = 0; j < EPL; j++)
+            if (lane + 32 * j < E) {
+              ei[j] = lane + 32 * j;
+              x[j] = C[lane + 32 * j];
+            }
+        }
       }
-    }
-    if (!alive) { c.dead++; continue; }
-    c.alive++;
-    if (!keep) continue;
-    uint64_t k1, k2;
-    warp_class_key<NQ, ST>(C, k, sp.nsym, conjmask, perm, W, lane, k1, k2);
-    unsigned long long slot = 0;
-    if (lane == 0) slot = atomicAdd(&o.st->n_surv, 1ULL);
-    slot = __shfl_sync(FULL, slot, 0);
-    if (slot < o.cap) {
-      if (lane == 0) {
-        o.sh1[slot] = k1; o.sh2[slot] = k2; o.sidx[slot] = p * (unsigned long long)GS + g;
-        NodeMeta nm;
-        nm.k = (int16_t)k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = (uint8_t)c2; nm.g1 = (uint8_t)g; nm.g2 = pm.g1;
-        nm.hsn = (uint8_t)((hs == 2 ? 1 : 0) | ((need_b ? ch.ntriv : 0) << 1));
-        nm.needs = (uint8_t)needs;
-        o.smeta[slot] = nm;
+      if (!alive) { c.dead++; continue; }
+      c.alive++;
+      if (!keep) continue;
+      uint64_t k1, k2;
+      warp_key_entries<NQ, ST>(x, ei, k, sp.nsym, conjmask, weight, lane, k1, k2);
+      unsigned long long slot = 0;
+      if (lane == 0) slot = atomicAdd(&o.st->n_surv, 1ULL);
+      slot = __shfl_sync(FULL, slot, 0);
+      if (slot < o.cap) {
+        if (lane == 0) {
+          o.sh1[slot] = k1; o.sh2[slot] = k2; o.sidx[slot] = p * (unsigned long long)GS + g;
+          NodeMeta nm;
+          nm.k = (int16_t)k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = (uint8_t)c2; nm.g1 = (uint8_t)g; nm.g2 = pm.g1;
+          nm.hsn = (uint8_t)((hs == 2 ? 1 : 0) | (ntriv << 1));
+          nm.needs = (uint8_t)needs;
+          o.smeta[slot] = nm;
+        }
+      } else if (lane == 0) {
+        o.st->surv_overflow = 1;
       }
-    } else if (lane == 0) {
-      o.st->surv_overflow = 1;
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -1243,38 +1416,65 @@ __global__ void __launch_bounds__(EXP_WARPS * 32) k_goal_level(const DevSpec sp,
   }
 }
 
+// A warp's parents: taken from a counter two ahead, the residual one ahead (copied into shared memory by cp.async while
+// the current parent is expanded), so neither the counter nor the loads are waited for. body(p, P, meta).
+template <int NQ, typename ST, typename Body>
+__device__ __forceinline__ void walk_parents(ExpandSmem<NQ, ST> &sm, unsigned long long *counter, unsigned long long p0,
+                                             unsigned long long end, const Z4<ST> *R, const NodeMeta *meta, int w, int lane,
+                                             Body body) {
+  constexpr int E = (1 << NQ) * (1 << NQ), NB = ExpandSmem<NQ, ST>::NB, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
+  auto grab = [&]() { return lane == 0 ? p0 + atomicAdd(counter, 1ULL) : 0ULL; };
+  auto fetch = [&](unsigned long long p, int b, NodeMeta &m) {
+    if (p < end) {
+      const char *src = (const char *)(R + p * (unsigned long long)E);
+      char *dst = (char *)sm.P[w][b];
+      for (int i = lane; i < CHUNKS; i += 32) cp_async16(dst + 16 * i, src + 16 * i);
+      m = meta[p];
+    }
+    cp_async_commit();
+  };
+  unsigned long long p = __shfl_sync(FULL, grab(), 0), raw = grab();
+  NodeMeta m{}, mn{};
+  int b = 0;
+  fetch(p, 0, m);
+  while (p < end) {
+    const unsigned long long pn = __shfl_sync(FULL, raw, 0);
+    if (NB == 2) fetch(pn, b ^ 1, mn);
+    raw = grab();
+    if (NB == 2) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncwarp();
+    body(p, sm.P[w][b], m);
+    __syncwarp();
+    if (NB == 1) fetch(pn, 0, mn);
+    p = pn;
+    m = mn;
+    b ^= NB - 1;
+  }
+  cp_async_wait<0>();
+}
+
 template <int NQ, typename ST, bool STATES = false, int PART = 0>
 __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand(const DevSpec sp, const ExpandArgs<ST> a) {
-  constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
+  constexpr int E = (1 << NQ) * (1 << NQ);
   if (a.gshort && a.gshort->found && !a.gshort->ovf && a.gshort->count <= GOAL_LIST) return;   // the found level
   __shared__ ExpandSmem<NQ, ST> sm;
   __shared__ DevSpec s_sp;                     // the spec for out-of-line helpers (a shared address, no local copy)
   for (int i = threadIdx.x; i < (int)(sizeof(DevSpec) / 4); i += blockDim.x) ((int *)&s_sp)[i] = ((const int *)&sp)[i];
-  init_weights(sm.W, E);
-  for (int i = threadIdx.x; i < SYMMAX * 8; i += blockDim.x) sm.perm[i / 8][i % 8] = sp.symperm[i / 8][i % 8];
+  __syncthreads();
+  init_group_weights<NQ>(sm.Wt, s_sp);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Z4<ST> *P = sm.P[w], *C = sm.C[w];
   unsigned conjmask = 0;
   for (int i = 0; i < sp.nsym; i++) conjmask |= (unsigned)(sp.symconj[i] != 0) << i;
   const ExpandOut<ST> o{a.st, a.cap, a.sh1, a.sh2, a.sidx, a.smeta, a.tq, a.tqcap};
+  const auto weight = [&](int s, int e) { return sm.Wt[s][e & (E - 1)]; };
   WarpTally c;
-  for (;;) {
-    unsigned long long p = 0;
-    if (lane == 0) p = atomicAdd(PART == 2 ? &a.st->work2 : &a.st->work, 1ULL);
-    p = __shfl_sync(FULL, p, 0);
-    if ((long long)p >= a.m) break;
-#pragma unroll
-    for (int j = 0; j < EPL; j++) {
-      const int e = lane + 32 * j;
-      if (e < E) P[e] = a.R[p * E + e];
-    }
-    const NodeMeta pm = a.meta[p];
-    __syncwarp();
-    expand_parent<NQ, ST, STATES, PART>(sp, &s_sp, sm.perm, conjmask, sm.W, P, C, p, pm, a.rem, a.keep != 0, sp.G, o, c,
-                          lane);
-    __syncwarp();
-  }
+  walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, 0, (unsigned long long)a.m, a.R, a.meta, w, lane,
+                       [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm) {
+    expand_parent<NQ, ST, STATES, PART>(sp, &s_sp, weight, conjmask, P, sm.C[w], sm.F[w], p, pm, a.rem, a.keep != 0, sp.G,
+                                        o, c, lane);
+  });
   c.flush(a.st, lane);
 }
 
@@ -1390,10 +1590,11 @@ __global__ void __launch_bounds__(EXP_WARPS * 32) k_goal_level_batch(const DevSp
 }
 
 template <int NQ, typename ST>
-__global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand_batch(const BatchArgs<ST> a) {
+__global__ void __launch_bounds__(EXP_WARPS * 32, EXPB_MINB) k_expand_batch(const BatchArgs<ST> a) {
   constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
   __shared__ Z4<ST> sP[EXP_WARPS][E], sC[EXP_WARPS][E];
   __shared__ uint64_t W[E];
+  __shared__ uint32_t sF[EXP_WARPS][E];
   __shared__ DevSpec sps[EXP_WARPS];           // each warp's current job spec
   init_weights(W, E);
   __syncthreads();
@@ -1434,7 +1635,10 @@ __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand_batch(const
     }
     const NodeMeta pm = a.meta[p];
     __syncwarp();
-    expand_parent<NQ, ST>(sp, &sp, sp.symperm, conjmask, W, P, C, p, pm, rem, keep, BATCH_GS, o, c, lane);
+    const auto weight = [&](int s, int e) {
+      return W[sp.symperm[s][(e >> NQ) & (N - 1)] * N + sp.symperm[s][e & (N - 1)]];
+    };
+    expand_parent<NQ, ST>(sp, &sp, weight, conjmask, P, C, sF[w], p, pm, rem, keep, BATCH_GS, o, c, lane);
     __syncwarp();
   }
   if (job >= 0) c.flush(a.jst + job, lane);
@@ -1446,37 +1650,26 @@ __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand_batch(const
 template <int NQ, typename ST, int PART>
 __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand_solo(const DevSpec sp, const BatchArgs<ST> a,
                                                                          int job) {
-  constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
+  constexpr int E = (1 << NQ) * (1 << NQ);
   if (a.gshort && !a.gshort->ovf && a.gshort->count <= GOAL_LIST && a.jgoal[job].x > 0) return;   // its found level
   __shared__ ExpandSmem<NQ, ST> sm;
   __shared__ DevSpec s_sp;
   for (int i = threadIdx.x; i < (int)(sizeof(DevSpec) / 4); i += blockDim.x) ((int *)&s_sp)[i] = ((const int *)&sp)[i];
-  init_weights(sm.W, E);
-  for (int i = threadIdx.x; i < SYMMAX * 8; i += blockDim.x) sm.perm[i / 8][i % 8] = sp.symperm[i / 8][i % 8];
+  __syncthreads();
+  init_group_weights<NQ>(sm.Wt, s_sp);
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Z4<ST> *P = sm.P[w], *C = sm.C[w];
   unsigned conjmask = 0;
   for (int i = 0; i < sp.nsym; i++) conjmask |= (unsigned)(sp.symconj[i] != 0) << i;
   const int t = a.jt[job];
   const ExpandOut<ST> o{a.st, a.cap, a.sh1, a.sh2, a.sidx, a.smeta, a.tq, a.tqcap};
+  const auto weight = [&](int s, int e) { return sm.Wt[s][e & (E - 1)]; };
   WarpTally c;
-  for (;;) {
-    unsigned long long p = 0;
-    if (lane == 0) p = a.p0 + atomicAdd(PART == 2 ? &a.st->work2 : &a.st->work, 1ULL);
-    p = __shfl_sync(FULL, p, 0);
-    if ((long long)p >= a.m) break;
-#pragma unroll
-    for (int j = 0; j < EPL; j++) {
-      const int e = lane + 32 * j;
-      if (e < E) P[e] = a.R[p * E + e];
-    }
-    const NodeMeta pm = a.meta[p];
-    __syncwarp();
-    expand_parent<NQ, ST, false, PART>(sp, &s_sp, sm.perm, conjmask, sm.W, P, C, p, pm, sp.depth - t, t < sp.depth, BATCH_GS, o, c,
-                          lane);
-    __syncwarp();
-  }
+  walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, (unsigned long long)a.p0, (unsigned long long)a.m, a.R,
+                       a.meta, w, lane, [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm) {
+    expand_parent<NQ, ST, false, PART>(sp, &s_sp, weight, conjmask, P, sm.C[w], sm.F[w], p, pm, sp.depth - t, t < sp.depth,
+                                       BATCH_GS, o, c, lane);
+  });
   c.flush(a.jst + job, lane);
 }
 
@@ -1505,6 +1698,8 @@ __device__ __forceinline__ void warp_materialize(const Z4<ST> *R, const NodeMeta
 // children, finish their alive test, and write the survivors' records, as the level kernel would have. With jobs
 // (fjob != nullptr) the parent's job gives the spec, level and counters.
 constexpr int TB_WARPS = 8;
+constexpr int TB_MINB = 2;   // blocks per SM asked for: 2 (128 registers) 6.40 ms, 3 (80) 6.87 ms, 4 (64, spills) 6.51 ms
+                             // over the two budget 12 proofs
 template <typename ST> struct TBoundArgs {
   const Z4<ST> *R;
   const NodeMeta *meta;
@@ -1521,16 +1716,18 @@ template <typename ST> struct TBoundArgs {
   NodeMeta *smeta;
 };
 // One block's warps walk the queue with a fixed stride. Bound by issue: a dead entry (most are) is the child's update,
-// its packing and one packed round, about 800 instructions.
+// its packing and one packed round. 3.96 M entries of two budget 12 proofs: 32.7 ms with 32-bit components, 11.7 ms
+// packed, 6.4 ms with the diagonal update in registers, the general form in a walk of its own and one alive test.
 template <int NQ, typename ST, bool BATCHED = false>
-__global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? 3 : 1)
+__global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
     k_tbound(const __grid_constant__ DevSpec sp0, const TBoundArgs<ST> a) {
-  constexpr int N = 1 << NQ, E = N * N, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
+  constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
   constexpr bool PACKED = sizeof(ST) == 4;               // the packed T bound (int32 limbs)
   constexpr int NB = sizeof(ST) == 4 ? 2 : 1;            // int64 limbs: one buffer (shared memory), no overlap
   __shared__ __align__(16) Z4<ST> sP[TB_WARPS][NB][E];  // the entry's parent, and the next entry's arriving
   __shared__ Z4<ST> sC[TB_WARPS][E];
   __shared__ int4 sY[PACKED ? TB_WARPS : 1][PACKED ? E : 1];
+  __shared__ int sX[PACKED ? TB_WARPS : 1][PACKED ? E : 1];
   __shared__ uint64_t W[E];
   __shared__ DevSpec s_sp;
   const unsigned long long n = a.st->n_tq < a.tqcap ? a.st->n_tq : a.tqcap;
@@ -1548,7 +1745,15 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? 3 : 1)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   Z4<ST> *C = sC[w];
   const DevSpec *spp = &s_sp;
-  WarpTally c;
+  unsigned nalive = 0, ndead = 0, neval = 0;           // tallies of the current job (or the whole search)
+  auto flush = [&](DevStats *st) {
+    if (lane == 0) {
+      if (ndead) atomicAdd(&st->dead, (unsigned long long)ndead);
+      if (nalive) atomicAdd(&st->alive, (unsigned long long)nalive);
+      if (neval) atomicAdd(&st->t_evals, (unsigned long long)neval);
+    }
+    nalive = ndead = neval = 0;
+  };
   int job = -2, rem = a.rem;
   bool keep = a.keep != 0;
   // entries are read one ahead: the next entry's parent residual is copied into shared memory asynchronously
@@ -1561,98 +1766,135 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? 3 : 1)
     for (int i = lane; i < CHUNKS; i += 32) cp_async16(dst + 16 * i, src + 16 * i);
     return true;
   };
-  TQEntry q;
-  int b = 0;
-  unsigned long long e = (unsigned long long)blockIdx.x * TB_WARPS + w;
-  bool have = take(q, e, 0);
-  cp_async_commit();
-  while (have) {
-    TQEntry q2;
-    bool more = false;
-    e += stride;
-    if constexpr (NB == 2) {
-      more = take(q2, e, b ^ 1);
-      cp_async_commit();
-      cp_async_wait<1>();                            // this entry's parent has arrived (the next may be in flight)
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncwarp();
-    const Z4<ST> *P = sP[w][b];
-    if constexpr (BATCHED) {
-      const int pj = (int)a.fjob[q.p];
-      if (pj != job) {                               // the spec of this entry's job
-        if (job >= 0) c.flush(a.jst + job, lane);
-        job = pj;
-        spp = a.specs + job;
-        const int t = a.jt[job];
-        rem = spp->depth - t; keep = t < spp->depth;
-        conjmask = 0;
-        for (int i = 0; i < spp->nsym; i++) conjmask |= (unsigned)(spp->symconj[i] != 0) << i;
+  // one walk over the warp's entries with the packed form; those it does not take, if any, in a second walk with the
+  // general one (a call in the loop would cost the packed form its registers)
+  bool left = !PACKED;
+  auto walk = [&](auto general) {
+    constexpr bool GENERAL = decltype(general)::value;
+    TQEntry q;
+    int b = 0;
+    unsigned long long e = (unsigned long long)blockIdx.x * TB_WARPS + w;
+    bool have = take(q, e, 0);
+    cp_async_commit();
+    while (have) {
+      TQEntry q2;
+      bool more = false;
+      e += stride;
+      if constexpr (NB == 2) {
+        more = take(q2, e, b ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();                            // this entry's parent has arrived (the next may be in flight)
+      } else {
+        cp_async_wait<0>();
       }
-    }
-    const DevSpec &sp = *spp;
-    const NodeMeta pm = a.meta[q.p];
-    auto alive = [&](int T, int s2) {
-      return sp.lite ? q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem
-                     : combine(q.k > q.hs ? q.k : q.hs, T, q.c2, __popc(q.ntriv[s2])) <= rem;
-    };
-    bool ovf;
-    (void)warp_child<NQ, ST>(P, C, q.g[0], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
-    __syncwarp();
-    int T;
-    bool packed = false;
-    if constexpr (PACKED) packed = sp.unit && NQ + q.k <= PACK_MAX;
-    if (packed) {
-#pragma unroll
-      for (int j = 0; j < (E >= 32 ? E / 32 : 1); j++)
-        if (lane + 32 * j < E) sY[w][lane + 32 * j] = pack_entry(C[lane + 32 * j]);
       __syncwarp();
-      T = packed_tbound<NQ>(sY[w], q.k, lane, [&](int t) { return !alive(t, 0) && (q.n < 2 || !alive(t, 1)); });
-    } else {
-      T = PACKED ? warp_tbound_slim<NQ, ST>(C, q.k, lane) : ptm_bound<NQ, ST>(C, q.k, lane);
-    }
-    c.teval++;
-    for (int s2 = 0; s2 < q.n; s2++) {
-      if (!alive(T, s2)) { c.dead++; continue; }
-      c.alive++;
-      if (!keep) continue;
-      if (s2) {                                      // the sibling's residual
-        __syncwarp();
-        (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);
-        __syncwarp();
-      }
-      uint64_t k1, k2;
-      warp_class_key<NQ, ST>(C, q.k, sp.nsym, conjmask, sp.symperm, W, lane, k1, k2);
-      unsigned long long slot = 0;
-      if (lane == 0) slot = atomicAdd(&a.st->n_surv, 1ULL);
-      slot = __shfl_sync(FULL, slot, 0);
-      if (slot < a.cap) {
-        if (lane == 0) {
-          a.sh1[slot] = k1; a.sh2[slot] = k2; a.sidx[slot] = q.p * (unsigned long long)a.GS + q.g[s2];
-          NodeMeta nm;
-          nm.k = q.k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = q.c2; nm.g1 = q.g[s2]; nm.g2 = pm.g1;
-          nm.hsn = (uint8_t)((q.hs == 2 ? 1 : 0) | (q.ntriv[s2] << 1));
-          nm.needs = q.needs;
-          a.smeta[slot] = nm;
+      const Z4<ST> *P = sP[w][b];
+      if constexpr (BATCHED) {
+        const int pj = (int)a.fjob[q.p];
+        if (pj != job) {                               // the spec of this entry's job
+          if (job >= 0) flush(a.jst + job);
+          job = pj;
+          spp = a.specs + job;
+          const int t = a.jt[job];
+          rem = spp->depth - t; keep = t < spp->depth;
+          conjmask = 0;
+          for (int i = 0; i < spp->nsym; i++) conjmask |= (unsigned)(spp->symconj[i] != 0) << i;
         }
-      } else if (lane == 0) {
-        a.st->surv_overflow = 1;
       }
-      __syncwarp();
+      const DevSpec &sp = *spp;
+      const NodeMeta pm = a.meta[q.p];
+      // the largest T bound a child lives with: lane T tries T (combine is monotone in it), so one evaluation per child
+      int thr[2];
+      const int h = q.k > q.hs ? q.k : q.hs;
+#pragma unroll
+      for (int s2 = 0; s2 < 2; s2++) {
+        const bool ok = s2 < q.n && (sp.lite ? q.k + (lane + sp.tdiv - 1) / sp.tdiv <= rem
+                                             : combine(h, lane, q.c2, __popc(q.ntriv[s2])) <= rem);
+        thr[s2] = 31 - __clz((int)__ballot_sync(FULL, ok));
+      }
+      // the packed walk takes the children of one-qubit unit monomials (t, tdg): the parent's entries times units, so the
+      // exponent stays the parent's
+      const int col = lane & (N - 1);
+      bool packed = PACKED && sp.unit && NQ + q.k <= PACK_MAX && q.k == pm.k && (sp.gflags[q.g[0]] & GF_UNITMON);
+      const int mono0 = packed ? sp.gmono[q.g[0]][col] : 0;
+      if (q.n > 1) packed = packed && (sp.gflags[q.g[1]] & GF_UNITMON);
+      int mine = q.n;                                // the entry's children, none when the other walk takes it
+      if (packed == GENERAL) {
+        mine = 0;
+        left = true;
+      }
+      bool ovf;
+      int T = 0;
+      if (mine) neval++;
+      if constexpr (GENERAL) {
+        if (mine) {
+          (void)warp_child<NQ, ST>(P, C, q.g[0], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
+          __syncwarp();
+          T = PACKED ? warp_tbound_slim<NQ, ST>(C, q.k, lane) : ptm_bound<NQ, ST>(C, q.k, lane);
+        }
+      } else if (mine) {
+#pragma unroll
+        for (int j = 0; j < EPL; j++)
+          if (lane + 32 * j < E) {
+            const int4 y = pack_entry(mono_entry<NQ>(P, mono0, lane, j));
+            sY[w][lane + 32 * j] = y;
+            sX[w][lane + 32 * j] = y.x;
+          }
+        __syncwarp();
+        T = packed_tbound<NQ>(sY[w], sX[w], q.k, lane, max(thr[0], thr[1]));   // T <= 2 (NQ + k) < 31: thr is exact
+      }
+      for (int s2 = 0; s2 < mine; s2++) {
+        const bool alive = T < 31 ? T <= thr[s2]
+                                  : (sp.lite ? q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem
+                                             : combine(h, T, q.c2, __popc(q.ntriv[s2])) <= rem);
+        if (!alive) { ndead++; continue; }
+        nalive++;
+        if (!keep) continue;
+        if constexpr (GENERAL) {
+          if (s2) {                                    // the sibling's residual
+            __syncwarp();
+            (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < EPL; j++)
+            if (lane + 32 * j < E) C[lane + 32 * j] = mono_entry<NQ>(P, sp.gmono[q.g[s2]][col], lane, j);
+        }
+        __syncwarp();
+        uint64_t k1, k2;
+        warp_class_key<NQ, ST>(C, q.k, sp.nsym, conjmask, sp.symperm, W, lane, k1, k2);
+        unsigned long long slot = 0;
+        if (lane == 0) slot = atomicAdd(&a.st->n_surv, 1ULL);
+        slot = __shfl_sync(FULL, slot, 0);
+        if (slot < a.cap) {
+          if (lane == 0) {
+            a.sh1[slot] = k1; a.sh2[slot] = k2; a.sidx[slot] = q.p * (unsigned long long)a.GS + q.g[s2];
+            NodeMeta nm;
+            nm.k = q.k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = q.c2; nm.g1 = q.g[s2]; nm.g2 = pm.g1;
+            nm.hsn = (uint8_t)((q.hs == 2 ? 1 : 0) | (q.ntriv[s2] << 1));
+            nm.needs = q.needs;
+            a.smeta[slot] = nm;
+          }
+        } else if (lane == 0) {
+          a.st->surv_overflow = 1;
+        }
+        __syncwarp();
+      }
+      __syncwarp();                                    // every lane is done with this buffer before it is refilled
+      if constexpr (NB == 1) {
+        more = take(q2, e, 0);
+        cp_async_commit();
+      }
+      have = more;
+      q = q2;
+      b ^= NB - 1;
     }
-    __syncwarp();                                    // every lane is done with this buffer before it is refilled
-    if constexpr (NB == 1) {
-      more = take(q2, e, 0);
-      cp_async_commit();
-    }
-    have = more;
-    q = q2;
-    b ^= NB - 1;
-  }
-  cp_async_wait<0>();
-  if constexpr (BATCHED) { if (job >= 0) c.flush(a.jst + job, lane); }
-  else c.flush(a.st, lane);
+    cp_async_wait<0>();
+  };
+  if constexpr (PACKED) walk(std::false_type{});
+  if (left) walk(std::true_type{});
+  if constexpr (BATCHED) { if (job >= 0) flush(a.jst + job); }
+  else flush(a.st);
 }
 
 // the root node's bounds (the target itself), inherited or bracketed by its children
@@ -2642,7 +2884,7 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       a.smeta = sMeta.as<NodeMeta>();
       a.tq = tq.as<TQEntry>(); a.tqcap = tqcap; a.gshort = gsd;
       const long long want = (m + EXP_WARPS - 1) / EXP_WARPS;
-      const long long grid = std::max<long long>(1, std::min<long long>(want, (long long)nsm * 2 * 8));
+      const long long grid = std::max<long long>(1, std::min<long long>(want, (long long)nsm * EXP_MINB));   // one wave
       if (opt.profile) ck(cudaEventRecord(ev[0], s), "event");
       if (hs.states) k_expand<NQ, ST, true><<<(unsigned)grid, EXP_WARPS * 32, 0, s>>>(sp, a);
       else {                                     // one-qubit gates, then the others: two smaller loop bodies
@@ -3588,6 +3830,31 @@ DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool no
       }
       if (perm) sp.gkind[g] = GK_PERM;
     }
+  }
+  for (int g = 0; g < hs.G; g++) {      // unit monomials: per column its source column and power
+    const int nq = hs.gnq[g], L = 1 << nq;
+    bool ok = hs.gik[g] == 0;
+    for (int c = 0; c < N && ok; c++) {
+      int lc = 0, cnt = 0;
+      for (int j = 0; j < nq; j++) lc |= ((c >> hs.gq[g][j]) & 1) << j;
+      for (int m = 0; m < L && ok; m++) {
+        const Zw z = hs.ginv[g][m * L + lc];
+        if (zzero(z)) continue;
+        int p = -1;
+        for (int w = 0; w < 8; w++) if (zeq(z, zwpow(w))) p = w;
+        int src = c;
+        for (int j = 0; j < nq; j++) src = (src & ~(1 << hs.gq[g][j])) | (((m >> j) & 1) << hs.gq[g][j]);
+        ok = p >= 0 && ++cnt == 1;
+        sp.gmono[g][c] = (uint8_t)(src | p << 4);
+      }
+      ok = ok && cnt == 1;
+    }
+    if (ok) sp.gflags[g] |= GF_UNITMON;
+  }
+  for (int q = 0; q < 3; q++) {
+    sp.qcut[q] = QC_NONE;
+    for (int i = 0; i < sp.ncuts && sp.ncuts <= 4; i++)
+      if (q < NQ && sp.rad[i] > 1 && (sp.cutmask[i] == 1 << q || sp.cutmask[i] == (N - 1) - (1 << q))) sp.qcut[q] = (uint8_t)(2 * i);
   }
   gi.assign((size_t)GMAX * 64, int4{0, 0, 0, 0});
   for (int g = 0; g < hs.G; g++)

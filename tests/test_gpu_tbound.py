@@ -58,3 +58,21 @@ def test_target_that_is_not_unitary(engine, oracle_bin, tmp_path):
     out = engine.search(text, depth=9)
     assert (out.rc, out.lines()) == (rc, lines)
     assert out.raw.t_evals > 0
+
+
+@pytest.mark.parametrize("sym", [True, False])
+@pytest.mark.parametrize("seed,n,length", [(1, 3, 6), (2, 3, 7), (3, 3, 5), (4, 2, 7), (5, 2, 6), (6, 3, 6), (7, 1, 5)])
+def test_children_decided_from_their_parent(engine, oracle_bin, tmp_path, seed, n, length, sym):
+    """every kind of candidate the level kernel tells apart: unit monomials with phases (y), two-qubit diagonals (cz),
+    non-affine permutations (ccx), Hadamards and cx, on targets that are products and entangled ones"""
+    rng = random.Random(seed)
+    gates = ["y", "t", "h", "s"] + (["cz", "cx"] if n > 1 else []) + (["ccx"] if n > 2 else [])
+    circ = [(g, tuple(rng.sample(range(n), {"cz": 2, "cx": 2, "ccx": 3}.get(g, 1)))) for g in
+            gates[:length] + [rng.choice(gates) for _ in range(max(0, length - len(gates)))]]
+    rng.shuffle(circ)
+    text = workloads.make_spec(n, circ, length)
+    p = tmp_path / "t.spec"
+    p.write_text(text)
+    rc, lines = run_oracle(oracle_bin, p, ["--depth", "5"] + ([] if sym else ["--no-sym"]))
+    out = engine.search(text, depth=5, sym=sym)
+    assert (out.rc, out.lines()) == (rc, lines), circ
