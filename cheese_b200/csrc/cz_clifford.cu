@@ -12,11 +12,10 @@
 //    element of a rank is computed back from the rank (unrank) for candidate enumeration and uniform draws;
 //  * BFS: one thread per symplectic part, whose reached sign vectors are one 64-bit mask (n = 3); a generator carries
 //    the whole mask, its bits permuted by XOR with the signs it adds;
-//  * beam step: dist(X) = dist(X^-1) (the generator set is closed under inverses), and X^-1 is the candidate
-//    (a column of the candidate table) composed with the inverse of the beam state's left part, a 4^n-entry row
-//    lookup table held in shared memory, so one evaluation is 2n lookups + a rank + one L2 byte load. The B
-//    smallest (cost, index) pairs are selected exactly by a cost histogram and an ordered compaction instead of
-//    sorting every packed cost;
+//  * beam step: dist(X) = dist(X^-1) (the generator set is closed under inverses), and X^-1 is the placement composed
+//    with the inverse of the beam state's left part, a 4^n-entry row lookup table held in shared memory. The 4^n sign
+//    vectors of a placement share one composition and one rank; rows of 4^n costs are screened by their least one, and
+//    only the placements up to the beam's threshold are listed and sorted;
 //  * read-back: one warp per segment, a lane per generator, ballot picks the first generator one step closer.
 // Candidates are ordered by their tableau value (the reference leaves their order to an atomic counter).
 #include <cuda_runtime.h>
@@ -40,7 +39,6 @@ namespace {
 
 constexpr int CL_T = 256;
 constexpr int HB = 2048;            // cost histogram bins
-constexpr int SEL_I = 16, SEL_CH = CL_T * SEL_I;
 constexpr int MAXBEAM = 255;
 constexpr int WORDMAX = 32;         // longest optimal word read back (13 at n = 3)
 
@@ -192,63 +190,50 @@ __global__ void __launch_bounds__(CL_T) k_cl_level(uint64_t *front, uint64_t *se
   if (threadIdx.x == 0 && total) atomicAdd(count, (unsigned long long)total);
 }
 
-// placements of a T on qubit q: every K with K Z_q' K^-1 = +-Z_q for some q' (clifford.cu:170-183)
+// placements of a T on qubit q: every K with K Z_q' K^-1 = +-Z_q for some q' (clifford.cu:170-183). The condition does
+// not see K's signs, so the placements are kept as symplectic parts (as tableaux without signs), 4^n placements each.
+template <int N> __device__ __forceinline__ int placed_qubit(uint64_t K, int q) {   // q', or -1
+  int qp = -1;
+  for (int i = 0; i < N; i++)
+    if ((Tb<N>::row(K, N + i) & Tb<N>::SYM) == (1u << (N + q))) qp = i;
+  return qp;
+}
 template <int N>
-__global__ void k_cl_cands(unsigned long long order, uint64_t *lists, unsigned long long capq,
-                           unsigned long long *cnt, int *ovf) {
-  using T = Tb<N>;
-  const int lane = threadIdx.x & 31;
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  const unsigned long long nit = (order + stride - 1) / stride;      // uniform trip count: full-warp ballots
-  for (unsigned long long it = 0; it < nit; it++) {
-    const unsigned long long r = it * stride + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = r < order;
-    const uint64_t K = valid ? T::unrank((uint32_t)r) : 0;   // every rank is an element (the BFS covers the group)
-#pragma unroll
-    for (int q = 0; q < N; q++) {
-      bool hit = false;
-      if (valid)
-        for (int qp = 0; qp < N; qp++)
-          hit |= (T::row(K, N + qp) & T::SYM) == (1u << (N + q));
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (!bal) continue;
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(&cnt[q], (unsigned long long)__popc(bal));
-      base = __shfl_sync(0xffffffffu, base, 0);
-      const unsigned long long pos = base + (unsigned)__popc(bal & ((1u << lane) - 1));
-      if (hit) {
-        if (pos < capq) lists[(unsigned long long)q * capq + pos] = K;
+__global__ void k_cl_cands(const uint64_t *part, uint64_t *lists, uint32_t capq, uint32_t *cnt, int *ovf) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < Sym<N>::ORDER; i += gridDim.x * blockDim.x) {
+    const uint64_t K = part[i];
+    for (int q = 0; q < N; q++)
+      if (placed_qubit<N>(K, q) >= 0) {
+        const uint32_t pos = atomicAdd(&cnt[q], 1u);
+        if (pos < capq) lists[(size_t)q * capq + pos] = K;
         else atomicOr(ovf, 1);
       }
-    }
   }
 }
-template <int N>
-__global__ void k_cl_cand_meta(const uint64_t *K, size_t n, int q, uint8_t *meta) {
-  using T = Tb<N>;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    uint8_t m = 0;
-    for (int qp = 0; qp < N; qp++) {
-      const uint32_t w = T::row(K[i], N + qp);
-      if ((w & T::SYM) == (1u << (N + q))) m = (uint8_t)(qp | ((w >> T::SB) << 2));
-    }
-    meta[i] = m;
+// per symplectic part the least distance over its sign vectors
+template <int N> __global__ void k_cl_least(const uint8_t *dist, uint8_t *least) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < Sym<N>::ORDER; i += gridDim.x * blockDim.x) {
+    uint32_t m = 0xffffffffu;
+    const uint32_t *row = (const uint32_t *)(dist + (size_t)i * Sym<N>::NS);
+#pragma unroll
+    for (int w = 0; w < Sym<N>::NS / 4; w++) m = __vminu4(m, row[w]);
+    m = __vminu4(m, m >> 16);
+    least[i] = (uint8_t)min(m & 0xffu, (m >> 8) & 0xffu);
   }
-}
-__global__ void k_cl_iota(uint32_t *v, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    v[i] = (uint32_t)i;
-}
-__global__ void k_cl_gather_u64(const uint64_t *src, const uint32_t *order, size_t n, uint64_t *dst) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = src[order[i]];
 }
 
-// beam step: cost of (state b, candidate c, flip f) at index (b * nc + c) * 2 + f, histogram relative to cmin
+// Beam step, first pass: one row per (state b, flip f, symplectic part g of the placements), the 4^n placements of the
+// part. With K's sign vector s, the rank of the composed tableau is at ^ s: composition adds K's signs to the table's,
+// and the flip (row X_q' times Z_q' times the T's sign, which cancels Z_q's) only adds a constant. So one composition and
+// one rank serve 4^n evaluations; the row's least cost comes from the part's least distance. Row i = (b * 2 + f) * ng + g
+// gets at[i] and rcost[i], and the least costs a histogram relative to cmin. A step with 16 states (2.2 M rows standing
+// for 142 M placements) takes 65 us, and 15 us to list the kept ones; one rank per placement took 3.0 ms, and 0.4 ms to
+// select.
+constexpr int BADCOST = 999;        // of a placement outside the table (the reference's)
 template <int N>
-__global__ void __launch_bounds__(CL_T) k_cl_beam(const uint64_t *Kc, const uint8_t *meta, unsigned long long nc, int nb,
-                                                  const uint8_t *tabs, const int *bcost, int dagger, int cmin,
-                                                  const uint8_t *dist, uint16_t *cost, unsigned *hist) {
+__global__ void __launch_bounds__(CL_T) k_cl_beam(const uint64_t *parts, uint32_t ng, int nb, int q, const uint8_t *tabs,
+                                                  const int *bcost, int dagger, int cmin, const uint8_t *least,
+                                                  uint32_t *at, uint16_t *rcost, unsigned *hist) {
   using T = Tb<N>;
   constexpr int TS = 1 << (2 * N);
   __shared__ uint8_t stab[MAXBEAM * TS];
@@ -258,27 +243,50 @@ __global__ void __launch_bounds__(CL_T) k_cl_beam(const uint64_t *Kc, const uint
   for (int i = threadIdx.x; i < nb; i += blockDim.x) sbc[i] = bcost[i];
   for (int i = threadIdx.x; i < HB; i += blockDim.x) sh[i] = 0;
   __syncthreads();
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += stride) {
-    const uint64_t K = Kc[c];
-    const int m = meta[c], qp = m & 3, dg = dagger ^ (m >> 2);
-    // the flipped placement's K o g^-1 (g = Sdg if the T is a dagger after the sign, else S): row X_qp -> +-Y_qp image
-    const uint64_t Kf = T::with_row(K, qp, T::image(K, 1u << qp, 1u << qp) ^ ((dg ? 0u : 1u) << T::SB));
-    for (int b = 0; b < nb; b++) {
-      const uint8_t *tb = stab + b * TS;
-#pragma unroll
-      for (int f = 0; f < 2; f++) {
-        const uint32_t r = T::rank(T::compose_tab(f ? Kf : K, tb));
-        const int dd = r == T::BAD ? 999 : (int)dist[r];
-        const int v = sbc[b] + dd;
-        cost[((unsigned long long)b * nc + c) * 2 + f] = (uint16_t)v;
-        atomicAdd(&sh[min(v - cmin, HB - 1)], 1u);
-      }
+  const uint32_t rows = (uint32_t)nb * 2 * ng, stride = gridDim.x * blockDim.x;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += stride) {
+    const uint32_t g = i % ng, bf = i / ng;
+    const int b = (int)(bf >> 1);
+    uint64_t K = parts[g];
+    if (bf & 1) {
+      // the flipped placement's K o g^-1 (g = Sdg if the T is a dagger after the sign, else S): row X_qp -> +-Y_qp image
+      const int qp = placed_qubit<N>(K, q);
+      K = T::with_row(K, qp, T::image(K, 1u << qp, 1u << qp) ^ ((dagger ? 0u : 1u) << T::SB));
     }
+    const uint32_t r = T::rank(T::compose_tab(K, stab + b * TS));
+    const int v = sbc[b] + (r == T::BAD ? BADCOST : (int)least[r >> (2 * N)]);
+    at[i] = r;
+    rcost[i] = (uint16_t)v;
+    atomicAdd(&sh[min(v - cmin, HB - 1)], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < HB; i += blockDim.x)
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
+}
+// second pass: the placements of cost <= thr as keys cost - cmin | b | K | f, in the order the beam keeps them in (cost,
+// then state, placement by tableau value, flip); *cnt counts all of them, the first cap are stored
+template <int N> constexpr int KEY_BITS = Tb<N>::RB * Tb<N>::ROWS + 1;      // of (K, f)
+template <int N>
+__global__ void __launch_bounds__(CL_T) k_cl_emit(const uint64_t *parts, uint32_t ng, uint32_t rows, const int *bcost,
+                                                  int cmin, int thr, const uint8_t *dist, const uint32_t *at,
+                                                  const uint16_t *rcost, uint64_t *keys, unsigned long long cap,
+                                                  unsigned long long *cnt) {
+  using T = Tb<N>;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+    if ((int)rcost[i] > thr) continue;
+    const uint32_t g = i % ng, bf = i / ng, r = at[i];
+    const int base = bcost[bf >> 1];
+    for (uint32_t sv = 0; sv < (uint32_t)Sym<N>::NS; sv++) {
+      const int v = base + (r == T::BAD ? BADCOST : (int)dist[r ^ sv]);
+      if (v > thr) continue;
+      uint64_t K = parts[g];
+#pragma unroll
+      for (int j = 0; j < 2 * N; j++) K |= (uint64_t)((sv >> j) & 1u) << (j * T::RB + T::SB);
+      const unsigned long long pos = atomicAdd(cnt, 1ULL);
+      if (pos < cap)
+        keys[pos] = ((uint64_t)(v - cmin) << (KEY_BITS<N> + 8)) | ((uint64_t)(bf >> 1) << KEY_BITS<N>) | (K << 1) | (bf & 1);
+    }
+  }
 }
 // histogram of the costs >= base (bins relative to base)
 __global__ void k_cl_hist(const uint16_t *cost, unsigned long long tot, int base, unsigned *hist) {
@@ -295,66 +303,6 @@ __global__ void k_cl_hist(const uint16_t *cost, unsigned long long tot, int base
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
-__device__ __forceinline__ unsigned blk_excl_scan256(unsigned v, unsigned &total) {
-  __shared__ unsigned ws[CL_T / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) ws[w] = inc;
-  __syncthreads();
-  unsigned pre = 0, tot = 0;
-#pragma unroll
-  for (int i = 0; i < CL_T / 32; i++) { if (i < w) pre += ws[i]; tot += ws[i]; }
-  __syncthreads();
-  total = tot;
-  return pre + inc - v;
-}
-// entries below the threshold (fewer than the beam) appended as (cost << 32 | index); per-chunk counts of the
-// entries at the threshold
-__global__ void __launch_bounds__(CL_T) k_cl_sel_count(const uint16_t *cost, unsigned long long tot, int thr,
-                                                       uint32_t *blkcnt, unsigned long long *below, unsigned *nbelow,
-                                                       int cap) {
-  const unsigned long long base = (unsigned long long)blockIdx.x * SEL_CH;
-  unsigned eq = 0;
-  for (int it = 0; it < SEL_I; it++) {
-    const unsigned long long i = base + (unsigned long long)it * CL_T + threadIdx.x;
-    if (i >= tot) break;
-    const int v = cost[i];
-    if (v == thr) eq++;
-    else if (v < thr) {
-      const unsigned p = atomicAdd(nbelow, 1u);
-      if ((int)p < cap) below[p] = ((unsigned long long)v << 32) | i;
-    }
-  }
-  unsigned total;
-  (void)blk_excl_scan256(eq, total);
-  if (threadIdx.x == 0) blkcnt[blockIdx.x] = total;
-}
-// the first `need` entries at the threshold, in index order
-__global__ void __launch_bounds__(CL_T) k_cl_sel_write(const uint16_t *cost, unsigned long long tot, int thr,
-                                                       const uint32_t *blkoff, unsigned need,
-                                                       unsigned long long *eqlist) {
-  unsigned run = blkoff[blockIdx.x];
-  if (run >= need) return;
-  const unsigned long long base = (unsigned long long)blockIdx.x * SEL_CH;
-  for (int it = 0; it < SEL_I && run < need; it++) {
-    const unsigned long long i = base + (unsigned long long)it * CL_T + threadIdx.x;
-    const unsigned flag = (i < tot && cost[i] == thr) ? 1u : 0u;
-    unsigned total;
-    const unsigned pos = run + blk_excl_scan256(flag, total);
-    if (flag && pos < need) eqlist[pos] = ((unsigned long long)thr << 32) | i;
-    run += total;
-  }
-}
-__global__ void k_cl_pick(const uint64_t *Kc, const uint8_t *meta, const unsigned long long *cidx, int m, uint64_t *oK,
-                          uint8_t *oM) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) { oK[i] = Kc[cidx[i]]; oM[i] = meta[cidx[i]]; }
-}
 template <int N>
 __global__ void k_cl_dist(const uint64_t *tab, size_t n, const uint8_t *dist, int *out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -414,11 +362,11 @@ void h_image_table(int n, uint64_t B, uint8_t *tab) {
 struct CTable {
   int n = 0;
   long long order = 0;
-  CBuf dist;
-  CBuf candK[3], candM[3];
-  unsigned long long ncand[3] = {0, 0, 0};
+  CBuf dist, least;                          // by rank; per symplectic part
+  CBuf cand[3];                              // per qubit: the symplectic parts of its placements
+  uint32_t ncand[3] = {0, 0, 0};
   CliffTableInfo info;
-  void release() { dist.release(); for (int q = 0; q < 3; q++) { candK[q].release(); candM[q].release(); } }
+  void release() { dist.release(); least.release(); for (CBuf &c : cand) c.release(); }
 };
 
 class CliffordContext {
@@ -427,7 +375,7 @@ class CliffordContext {
   cudaStream_t s;
   int nsm = 148;
   std::map<int, CTable *> tables;
-  CBuf ovf, cnt, cost, hist, below, nbelow, blk, blkoff, part, eql, tabs, bc, pk, pm, tmp, out, len;
+  CBuf ovf, cnt, at, cost, hist, keys, keys2, vals, vals2, shist, part, tabs, bc, pk, tmp, out, len;
   long long launches = 0;
   CliffordContext(int d, void *stream) : dev(d), s((cudaStream_t)stream) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -435,13 +383,13 @@ class CliffordContext {
   ~CliffordContext() {
     cudaSetDevice(dev);
     for (auto &kv : tables) { kv.second->release(); delete kv.second; }
-    for (CBuf *b : {&ovf, &cnt, &cost, &hist, &below, &nbelow, &blk, &blkoff, &part, &eql, &tabs, &bc, &pk, &pm, &tmp,
+    for (CBuf *b : {&ovf, &cnt, &at, &cost, &hist, &keys, &keys2, &vals, &vals2, &shist, &part, &tabs, &bc, &pk, &tmp,
                     &out, &len})
       b->release();
   }
   size_t trim() {                              // work buffers back to the device; resident tables stay
     size_t n = 0;
-    for (CBuf *b : {&cnt, &cost, &hist, &below, &nbelow, &blk, &blkoff, &part, &eql, &tabs, &bc, &pk, &pm, &tmp, &out,
+    for (CBuf *b : {&cnt, &at, &cost, &hist, &keys, &keys2, &vals, &vals2, &shist, &part, &tabs, &bc, &pk, &tmp, &out,
                     &len}) {
       n += b->cap;
       b->release();
@@ -456,9 +404,9 @@ class CliffordContext {
 
   CTable *table(int n, CliffTableInfo &info);
   template <int N> void build(CTable &t);
-  template <int N> void beam_step(CTable &t, int q, int dagger, const std::vector<uint64_t> &left,
-                                  const std::vector<int> &bcost, int beam, std::vector<unsigned long long> &picked,
-                                  std::vector<int> &pcost);
+  struct Placed { int b, f, cost; uint64_t K; int qp, neg; };   // a kept placement: state, flip, cost, K and its q', sign
+  template <int N> std::vector<Placed> beam_step(CTable &t, int q, int dagger, const std::vector<uint64_t> &left,
+                                                 const std::vector<int> &bcost, int beam);
   std::vector<int> dist_of(CTable &t, const std::vector<uint64_t> &x);
   void words(CTable &t, const std::vector<uint64_t> &x, std::vector<std::vector<int>> &w);
 };
@@ -512,43 +460,31 @@ void CliffordContext::build(CTable &t) {
   }
   inf.per_distance[0] = 1;
   inf.elements = (long long)total;
-  for (CBuf *m : {&part, &seen, &fa, &fb}) m->release();
-  if (total != order) throw std::logic_error("group order mismatch");
-  // placement candidates per qubit, ordered by tableau value
-  const unsigned long long capq = order / ((1ULL << (2 * N)) - 1) * N + 64;
+  for (CBuf *m : {&seen, &fa, &fb}) m->release();
+  if (total != order) { part.release(); throw std::logic_error("group order mismatch"); }
+  t.least.ensure(Sym<N>::ORDER);
+  k_cl_least<N><<<gp, CL_T, 0, s>>>(t.dist.as<uint8_t>(), t.least.as<uint8_t>());
+  // the placements' parts per qubit: Z_q comes from one of n rows, each with one of 4^n - 1 images
+  const uint32_t capq = Sym<N>::ORDER / ((1u << (2 * N)) - 1) * N;
   CBuf lists;
-  lists.ensure(capq * N * 8);
+  lists.ensure((size_t)capq * N * 8);
   clk(cudaMemsetAsync(cnt.p, 0, 64, s), "memset");
-  k_cl_cands<N><<<grid(order), CL_T, 0, s>>>(order, lists.as<uint64_t>(), capq,
-                                             cnt.as<unsigned long long>(), ovf.as<int>());
-  launches++;
+  k_cl_cands<N><<<gp, CL_T, 0, s>>>(part.as<uint64_t>(), lists.as<uint64_t>(), capq, cnt.as<uint32_t>(), ovf.as<int>());
+  launches += 2;
   clk(cudaGetLastError(), "candidates");
-  unsigned long long nc[3] = {0, 0, 0};
   int of = 0;
-  clk(cudaMemcpyAsync(nc, cnt.p, 24, cudaMemcpyDeviceToHost, s), "d2h");
+  clk(cudaMemcpyAsync(t.ncand, cnt.p, 12, cudaMemcpyDeviceToHost, s), "d2h");
   clk(cudaMemcpyAsync(&of, ovf.p, 4, cudaMemcpyDeviceToHost, s), "d2h");
   sync("candidates");
-  if (of) throw std::overflow_error("candidate buffer too small");
+  part.release();
+  if (of) { lists.release(); throw std::overflow_error("candidate buffer too small"); }
   for (int q = 0; q < N; q++) {
-    const size_t m = (size_t)nc[q];
-    t.ncand[q] = m;
-    t.candK[q].ensure(m * 8 + 8); t.candM[q].ensure(m + 8);
-    CBuf k1, v0, v1, hs, pt;
-    k1.ensure(m * 8 + 8); v0.ensure(m * 4 + 4); v1.ensure(m * 4 + 4);
-    hs.ensure(sort_hist_words(m) * 4 + 4); pt.ensure(scan_partials_words(sort_hist_words(m)) * 4 + 4);
-    uint64_t *k0 = lists.as<uint64_t>() + (size_t)q * capq;
-    k_cl_iota<<<grid(m), CL_T, 0, s>>>(v0.as<uint32_t>(), m);
-    SortScratch sc{hs.as<uint32_t>(), pt.as<uint32_t>(), hs.cap / 4, pt.cap / 4};
-    int ln = 0;
-    const bool f = radix_sort(k0, v0.as<uint32_t>(), k1.as<uint64_t>(), v1.as<uint32_t>(), m, 0,
-                              ((T::RB * T::ROWS + 7) / 8) * 8, sc, s, &ln);
-    launches += 1 + ln;
-    clk(cudaMemcpyAsync(t.candK[q].p, f ? (void *)k1.p : (void *)k0, m * 8, cudaMemcpyDeviceToDevice, s), "d2d");
-    k_cl_cand_meta<N><<<grid(m), CL_T, 0, s>>>(t.candK[q].as<uint64_t>(), m, q, t.candM[q].as<uint8_t>());
-    launches++;
-    clk(cudaGetLastError(), "candidate meta");
-    sync("candidates");
+    t.cand[q].ensure((size_t)t.ncand[q] * 8 + 8);
+    clk(cudaMemcpyAsync(t.cand[q].p, lists.as<uint64_t>() + (size_t)q * capq, (size_t)t.ncand[q] * 8,
+                        cudaMemcpyDeviceToDevice, s), "d2d");
   }
+  sync("candidates");
+  lists.release();
   inf.built = true;
   inf.seconds = cl_now() - t0;
 }
@@ -614,31 +550,34 @@ void CliffordContext::words(CTable &t, const std::vector<uint64_t> &x, std::vect
   }
 }
 
-// one beam step over the placements of a T gate on qubit q: the kept (cost << 32 | index) in (cost, index) order
+// one beam step over the placements of a T gate on qubit q: the kept ones, by (cost, state, placement, flip)
 template <int N>
-void CliffordContext::beam_step(CTable &t, int q, int dagger, const std::vector<uint64_t> &left,
-                                const std::vector<int> &bcost, int beam, std::vector<unsigned long long> &picked,
-                                std::vector<int> &pcost) {
+std::vector<CliffordContext::Placed> CliffordContext::beam_step(CTable &t, int q, int dagger, const std::vector<uint64_t> &left,
+                                                                const std::vector<int> &bcost, int beam) {
+  using T = Tb<N>;
   constexpr int TS = 1 << (2 * N);
   const int nb = (int)left.size();
-  const unsigned long long nc = t.ncand[q], tot = (unsigned long long)nb * nc * 2;
+  const uint32_t ng = t.ncand[q], rows = (uint32_t)nb * 2 * ng;
   std::vector<uint8_t> ht((size_t)nb * TS);
-  for (int b = 0; b < nb; b++) Tb<N>::image_table(Tb<N>::inverse(left[b]), ht.data() + (size_t)b * TS);
+  for (int b = 0; b < nb; b++) T::image_table(T::inverse(left[b]), ht.data() + (size_t)b * TS);
   int cmin = 1 << 30, cmax = 0;
   for (int v : bcost) { cmin = std::min(cmin, v); cmax = std::max(cmax, v); }
-  if (cmax + 999 > 65535) throw std::range_error("beam cost out of range");
-  tabs.ensure(ht.size()); bc.ensure(nb * 4); hist.ensure(HB * 4); cost.ensure(tot * 2 + 2);
+  if (cmax + BADCOST > 65535) throw std::range_error("beam cost out of range");
+  tabs.ensure(ht.size()); bc.ensure(nb * 4); hist.ensure(HB * 4); cost.ensure((size_t)rows * 2 + 2); at.ensure((size_t)rows * 4 + 4);
+  cnt.ensure(64);
   clk(cudaMemcpyAsync(tabs.p, ht.data(), ht.size(), cudaMemcpyHostToDevice, s), "h2d");
   clk(cudaMemcpyAsync(bc.p, bcost.data(), nb * 4, cudaMemcpyHostToDevice, s), "h2d");
   clk(cudaMemsetAsync(hist.p, 0, HB * 4, s), "memset");
-  k_cl_beam<N><<<grid(nc, 16), CL_T, 0, s>>>(t.candK[q].as<uint64_t>(), t.candM[q].as<uint8_t>(), nc, nb,
-                                              tabs.as<uint8_t>(), bc.as<int>(), dagger, cmin, t.dist.as<uint8_t>(),
-                                              cost.as<uint16_t>(), hist.as<unsigned>());
+  k_cl_beam<N><<<grid(rows, 16), CL_T, 0, s>>>(t.cand[q].as<uint64_t>(), ng, nb, q, tabs.as<uint8_t>(), bc.as<int>(), dagger,
+                                                cmin, t.least.as<uint8_t>(), at.as<uint32_t>(), cost.as<uint16_t>(),
+                                                hist.as<unsigned>());
   launches++;
   clk(cudaGetLastError(), "beam step");
-  const unsigned long long keep = std::min<unsigned long long>((unsigned long long)beam, tot);
-  // threshold: the cost of the keep-th smallest entry
-  unsigned long long nlow = 0;   // entries below the threshold
+  // a threshold with at least `keep` placements at or below it: the cost of the keep-th smallest row's best (every row
+  // has a placement of its least cost), or every row when there are fewer
+  const unsigned long long keep = std::min<unsigned long long>((unsigned long long)beam, (unsigned long long)rows * Sym<N>::NS);
+  const unsigned long long krows = std::min<unsigned long long>(keep, rows);
+  unsigned long long nlow = 0;
   int base = cmin, thr = -1;
   std::vector<unsigned> hh(HB);
   for (;;) {
@@ -647,40 +586,64 @@ void CliffordContext::beam_step(CTable &t, int q, int dagger, const std::vector<
     unsigned long long cum = nlow;
     int k = 0;
     for (; k < HB - 1; k++) {
-      if (cum + hh[k] >= keep) break;
+      if (cum + hh[k] >= krows) break;
       cum += hh[k];
     }
-    if (k < HB - 1) { thr = base + k; nlow = cum; break; }
+    if (k < HB - 1) { thr = base + k; break; }
     nlow = cum;                      // everything below base + HB - 1 is kept: zoom into the overflow bin
     base += HB - 1;
     clk(cudaMemsetAsync(hist.p, 0, HB * 4, s), "memset");
-    k_cl_hist<<<grid(tot, 16), CL_T, 0, s>>>(cost.as<uint16_t>(), tot, base, hist.as<unsigned>());
+    k_cl_hist<<<grid(rows, 16), CL_T, 0, s>>>(cost.as<uint16_t>(), rows, base, hist.as<unsigned>());
     launches++;
   }
-  const unsigned long long nblk = (tot + SEL_CH - 1) / SEL_CH;
-  const unsigned need = (unsigned)(keep - nlow);
-  below.ensure(MAXBEAM * 8 + 8); nbelow.ensure(4); blk.ensure(nblk * 4 + 4); blkoff.ensure(nblk * 4 + 4);
-  part.ensure(scan_partials_words(nblk) * 4 + 4); eql.ensure(MAXBEAM * 8 + 8);
-  clk(cudaMemsetAsync(nbelow.p, 0, 4, s), "memset");
-  k_cl_sel_count<<<(unsigned)nblk, CL_T, 0, s>>>(cost.as<uint16_t>(), tot, thr, blk.as<uint32_t>(),
-                                                  below.as<unsigned long long>(), nbelow.as<unsigned>(), MAXBEAM);
-  exclusive_scan(blk.as<uint32_t>(), blkoff.as<uint32_t>(), nblk, part.as<uint32_t>(), nullptr, s);
-  k_cl_sel_write<<<(unsigned)nblk, CL_T, 0, s>>>(cost.as<uint16_t>(), tot, thr, blkoff.as<uint32_t>(), need,
-                                                  eql.as<unsigned long long>());
-  launches += 5;
-  clk(cudaGetLastError(), "beam selection");
-  unsigned nbel = 0;
-  std::vector<unsigned long long> hb(MAXBEAM), he(need);
-  clk(cudaMemcpyAsync(&nbel, nbelow.p, 4, cudaMemcpyDeviceToHost, s), "d2h");
-  clk(cudaMemcpyAsync(hb.data(), below.p, MAXBEAM * 8, cudaMemcpyDeviceToHost, s), "d2h");
-  if (need) clk(cudaMemcpyAsync(he.data(), eql.p, need * 8, cudaMemcpyDeviceToHost, s), "d2h");
+  if (keep > krows) thr = cmax + BADCOST;            // fewer rows than the beam keeps: all their placements
+  // every placement up to the threshold (few: the tail of the costs is thin), sorted; a second round when they are more
+  // than the room
+  int kb = 0;
+  while ((thr - cmin) >> kb) kb++;
+  const int bits = KEY_BITS<N> + 8 + kb;
+  if (bits > 64) throw std::range_error("beam cost out of range");
+  unsigned long long room = std::max<unsigned long long>(keys.cap / 8, 1ULL << 16), m = 0;
+  for (;;) {
+    keys.ensure(room * 8);
+    room = keys.cap / 8;
+    clk(cudaMemsetAsync(cnt.p, 0, 8, s), "memset");
+    k_cl_emit<N><<<grid(rows, 16), CL_T, 0, s>>>(t.cand[q].as<uint64_t>(), ng, rows, bc.as<int>(), cmin, thr,
+                                                 t.dist.as<uint8_t>(), at.as<uint32_t>(), cost.as<uint16_t>(),
+                                                 keys.as<uint64_t>(), room, cnt.as<unsigned long long>());
+    launches++;
+    clk(cudaGetLastError(), "beam placements");
+    clk(cudaMemcpyAsync(&m, cnt.p, 8, cudaMemcpyDeviceToHost, s), "d2h");
+    sync("beam placements");
+    if (m <= room) break;
+    room = m;
+  }
+  if (m < keep) throw std::logic_error("beam selection count mismatch");
+  keys2.ensure(m * 8 + 8); vals.ensure(m * 4 + 4); vals2.ensure(m * 4 + 4);
+  shist.ensure(sort_hist_words(m) * 4 + 4); part.ensure(scan_partials_words(sort_hist_words(m)) * 4 + 4);
+  SortScratch sc{shist.as<uint32_t>(), part.as<uint32_t>(), shist.cap / 4, part.cap / 4};
+  int ln = 0;
+  const bool fl = radix_sort(keys.as<uint64_t>(), vals.as<uint32_t>(), keys2.as<uint64_t>(), vals2.as<uint32_t>(), (size_t)m, 0,
+                             (bits + 7) / 8 * 8, sc, s, &ln);
+  launches += ln;
+  std::vector<uint64_t> hk(keep);
+  clk(cudaMemcpyAsync(hk.data(), fl ? keys2.p : keys.p, keep * 8, cudaMemcpyDeviceToHost, s), "d2h");
   sync("beam selection");
-  if (nbel != nlow) throw std::logic_error("beam selection count mismatch");
-  std::vector<unsigned long long> all(hb.begin(), hb.begin() + nbel);
-  all.insert(all.end(), he.begin(), he.end());
-  std::sort(all.begin(), all.end());
-  picked.clear(); pcost.clear();
-  for (unsigned long long e : all) { picked.push_back(e & 0xffffffffULL); pcost.push_back((int)(e >> 32)); }
+  std::vector<Placed> out;
+  for (uint64_t k : hk) {
+    Placed p;
+    p.f = (int)(k & 1);
+    p.K = (k >> 1) & ((1ULL << (KEY_BITS<N> - 1)) - 1);
+    p.b = (int)((k >> KEY_BITS<N>) & 0xff);
+    p.cost = cmin + (int)(k >> (KEY_BITS<N> + 8));
+    p.qp = p.neg = 0;
+    for (int i = 0; i < N; i++) {
+      const uint32_t w = T::row(p.K, N + i);
+      if ((w & T::SYM) == (1u << (N + q))) { p.qp = i; p.neg = (int)(w >> T::SB); }
+    }
+    out.push_back(p);
+  }
+  return out;
 }
 
 // ---------------- jobs ----------------
@@ -783,35 +746,18 @@ int cliffopt_run(CliffordContext *c, const CliffJob &J, int beam,
       const int q = J.tq[j];
       std::vector<uint64_t> left(Kprev.size());
       for (size_t b = 0; b < Kprev.size(); b++) left[b] = j == 0 ? D[j] : h_compose(n, Kprev[b], D[j]);
-      std::vector<unsigned long long> picked;
-      std::vector<int> pcost;
-      if (n == 1) c->beam_step<1>(tab, q, J.td[j], left, bcost, beam, picked, pcost);
-      else if (n == 2) c->beam_step<2>(tab, q, J.td[j], left, bcost, beam, picked, pcost);
-      else c->beam_step<3>(tab, q, J.td[j], left, bcost, beam, picked, pcost);
-      const unsigned long long nc = tab.ncand[q];
-      const int m = (int)picked.size();
-      if (m == 0) throw std::logic_error("no placement candidates");
-      std::vector<unsigned long long> cidx(m);
-      for (int i = 0; i < m; i++) cidx[i] = (picked[i] % (2 * nc)) >> 1;
-      c->tmp.ensure(m * 8 + 8); c->pk.ensure(m * 8 + 8); c->pm.ensure(m + 8);
-      clk(cudaMemcpyAsync(c->tmp.p, cidx.data(), m * 8, cudaMemcpyHostToDevice, c->s), "h2d");
-      k_cl_pick<<<(m + 63) / 64, 64, 0, c->s>>>(tab.candK[q].as<uint64_t>(), tab.candM[q].as<uint8_t>(),
-                                                c->tmp.as<unsigned long long>(), m, c->pk.as<uint64_t>(), c->pm.as<uint8_t>());
-      c->launches++;
-      std::vector<uint64_t> pK(m);
-      std::vector<uint8_t> pM(m);
-      clk(cudaMemcpyAsync(pK.data(), c->pk.p, m * 8, cudaMemcpyDeviceToHost, c->s), "d2h");
-      clk(cudaMemcpyAsync(pM.data(), c->pm.p, m, cudaMemcpyDeviceToHost, c->s), "d2h");
-      c->sync("beam pick");
-      hist[j].resize(m);
-      Kprev.assign(m, 0);
-      bcost = pcost;
-      for (int i = 0; i < m; i++) {
-        const unsigned long long c2 = picked[i] % (2 * nc);
-        hist[j][i] = Pick{(int)(picked[i] / (2 * nc)), (int)(c2 & 1), pK[i], pM[i] & 3, pM[i] >> 2};
-        Kprev[i] = pK[i];
+      const std::vector<CliffordContext::Placed> kept =
+          n == 1 ? c->beam_step<1>(tab, q, J.td[j], left, bcost, beam)
+                 : n == 2 ? c->beam_step<2>(tab, q, J.td[j], left, bcost, beam) : c->beam_step<3>(tab, q, J.td[j], left, bcost, beam);
+      if (kept.empty()) throw std::logic_error("no placement candidates");
+      Kprev.clear();
+      bcost.clear();
+      for (const auto &p : kept) {
+        hist[j].push_back(Pick{p.b, p.f, p.K, p.qp, p.neg});
+        Kprev.push_back(p.K);
+        bcost.push_back(p.cost);
       }
-      if (on_step) on_step(j, CliffStep{(long long)nc, pcost.empty() ? 0 : pcost[0]});
+      if (on_step) on_step(j, CliffStep{(long long)tab.ncand[q] << (2 * n), bcost[0]});
     }
     int best = 0;
     if (t > 0) {

@@ -191,3 +191,28 @@ def test_cli_errors(tmp_path):
     assert p.returncode == 2 and "unknown Clifford gate foo" in p.stderr
     p = subprocess.run([str(BIN)], capture_output=True, text=True, timeout=60)
     assert p.returncode == 3
+
+
+@pytest.mark.parametrize("n,tcount,beam", [(1, 3, 1), (1, 3, 255), (2, 4, 1), (2, 3, 255), (2, 2, 100)])
+def test_beam_sizes_match_the_restatement(eng, tmp_path, n, tcount, beam):
+    """the smallest beam, and beams with more states than rows of sign vectors (n = 1: every placement is kept)"""
+    import subprocess
+    from cheese_b200 import tcwork
+    from conftest import ORACLE_DIR
+    oracle = ORACLE_DIR / "_ref" / "clifford-oracle"
+    if not oracle.exists():
+        subprocess.run(["make", "-C", str(ORACLE_DIR), "oracle"], check=True, capture_output=True)
+    rng = random.Random(100 * n + 10 * tcount + beam)
+    for i in range(4):
+        if n == 1:
+            segs = [[(rng.choice(["h", "s", "sdg", "x", "z"]), (0,)) for _ in range(6)] for _ in range(tcount + 1)]
+            job = tcwork.cliffopt_job(1, [(0, rng.randrange(2)) for _ in range(tcount)], segs)
+        else:
+            job = tcwork.random_clifford_job(rng, n, 12, tcount)
+        p = tmp_path / f"j{i}.job"
+        p.write_text(job)
+        want = subprocess.run([str(oracle), str(p), "--beam", str(beam)], capture_output=True, text=True, timeout=300)
+        rc, res, out, steps = eng.cliffopt(job, beam=beam)
+        assert rc == want.returncode == 0
+        assert out == want.stdout.splitlines()[1:]
+        assert [s[2] for s in steps] == [int(v) for v in re.findall(r"best partial (\d+)", want.stderr)]
