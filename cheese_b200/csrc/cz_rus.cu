@@ -21,12 +21,12 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <sstream>
 #include <stdexcept>
 
 #include "cz_rus.h"
 #include "cz_rus_node.h"
 #include "cz_sort.cuh"
+#include "cz_text.h"
 
 namespace cz {
 
@@ -244,6 +244,7 @@ class RusContext {
   std::map<std::pair<int, uint64_t>, Table *> tables;   // resident: (K, fingerprint)
   uint64_t spec_fp = 0;                                 // the fixed tables currently on the device
   Buf tr, ts, perm, sign, bygen, ovf, roots;
+  Tree search;                                          // the search's tree: its buffers stay for the next search
   Buf h1, h2, k0, k1, v0, v1, hist, part, keep, pos, kept, hits, cls, flag, total, fm2, g1, g2, p2, q2;
   long long launches = 0;
   RusContext(int d, void *stream) : dev(d), s((cudaStream_t)stream) {
@@ -253,6 +254,7 @@ class RusContext {
     cudaSetDevice(dev);
     for (auto &kv : tables) { kv.second->release(); delete kv.second; }
     for (Buf *b : all()) b->release();
+    search.release();
   }
   std::vector<Buf *> work() {
     return {&roots, &h1, &h2, &k0, &k1, &v0, &v1, &hist, &part, &keep, &pos, &kept, &hits, &cls, &flag, &total, &fm2,
@@ -266,6 +268,9 @@ class RusContext {
   size_t trim() {
     size_t n = 0;
     for (Buf *b : work()) { n += b->cap; b->release(); }
+    for (std::vector<Buf> *v : {&search.par, &search.gat}) for (Buf &b : *v) n += b.cap;
+    n += search.FM.cap + search.F1.cap + search.F2.cap;
+    search.release();
     return n;
   }
   unsigned grid(long long n) const {
@@ -277,8 +282,7 @@ class RusContext {
     rck(cudaStreamSynchronize(s), "sync");
     if (v) throw std::overflow_error("coefficient overflow (int32)");
   }
-  RDev upload(const RSpec &sp) {
-    const uint64_t fp = table_fingerprint(sp);
+  RDev upload(const RSpec &sp, uint64_t fp) {
     if (fp != spec_fp || !bygen.p) {
       std::vector<int8_t> t8(sp.tr.begin(), sp.tr.end()), s8(sp.ts.begin(), sp.ts.end());
       std::vector<int> bg(1 << 20, -1);
@@ -422,13 +426,14 @@ class RusContext {
                                32, sc, s, nullptr);
     if (nk > 1) launches += 20;
     const uint64_t *kidx = fk ? k1.as<uint64_t>() : kept.as<uint64_t>();
-    T.par.emplace_back(); T.gat.emplace_back(); T.n.push_back(nk);
-    T.par.back().ensure(nk * 4 + 4); T.gat.back().ensure(nk + 4);
+    T.n.push_back(nk);
+    if ((int)T.par.size() <= t) { T.par.resize(t + 1); T.gat.resize(t + 1); }   // (a kept tree has its levels' buffers)
+    T.par[t].ensure(nk * 4 + 4); T.gat[t].ensure(nk + 4);
     fm2.ensure((size_t)nk * MS * 4 + 16); g1.ensure(nk * 8 + 8); g2.ensure(nk * 8 + 8);
     if (nk) {
       k_rus_materialise<<<grid(nk), RT, 0, s>>>(kidx, nk, T.FM.as<int>(), sp, fm2.as<int>(), g1.as<uint64_t>(),
-                                                g2.as<uint64_t>(), T.par.back().as<uint32_t>(),
-                                                T.gat.back().as<uint8_t>(), ovf.as<int>());
+                                                g2.as<uint64_t>(), T.par[t].as<uint32_t>(),
+                                                T.gat[t].as<uint8_t>(), ovf.as<int>());
       launches++;
       rck(cudaGetLastError(), "materialise");
     }
@@ -451,14 +456,14 @@ class RusContext {
       fresh = hf;
       p2.ensure(fresh * 4 + 4); q2.ensure(fresh + 4); fm2.ensure((size_t)fresh * MS * 4 + 16);
       g1.ensure(fresh * 8 + 8); g2.ensure(fresh * 8 + 8);
-      k_rus_compact<<<grid(nk), RT, 0, s>>>(flag.as<uint32_t>(), pos.as<uint32_t>(), nk, T.par.back().as<uint32_t>(),
-                                            T.gat.back().as<uint8_t>(), T.FM.as<int>(), T.F1.as<uint64_t>(),
+      k_rus_compact<<<grid(nk), RT, 0, s>>>(flag.as<uint32_t>(), pos.as<uint32_t>(), nk, T.par[t].as<uint32_t>(),
+                                            T.gat[t].as<uint8_t>(), T.FM.as<int>(), T.F1.as<uint64_t>(),
                                             T.F2.as<uint64_t>(), p2.as<uint32_t>(), q2.as<uint8_t>(), fm2.as<int>(),
                                             g1.as<uint64_t>(), g2.as<uint64_t>());
       launches++;
       rck(cudaGetLastError(), "compact");
-      std::swap(T.par.back(), p2);
-      std::swap(T.gat.back(), q2);
+      std::swap(T.par[t], p2);
+      std::swap(T.gat[t], q2);
       std::swap(T.FM, fm2);
       std::swap(T.F1, g1);
       std::swap(T.F2, g2);
@@ -572,9 +577,8 @@ class RusContext {
     return true;
   }
 
-  Table *table(const RDev &sp, const RSpec &spec, const RusOptions &opt,
+  Table *table(const RDev &sp, const RSpec &spec, uint64_t fp, const RusOptions &opt,
                const std::function<void(const RusLevel &)> &cb, RusResult &res) {
-    const uint64_t fp = table_fingerprint(spec);
     const auto key = std::make_pair(opt.table_k, fp);
     char path[512];
     std::snprintf(path, sizeof path, "%s/rus-table-k%d.cz.bin", opt.cache_dir.c_str(), opt.table_k);
@@ -615,13 +619,15 @@ class RusContext {
     rck(cudaSetDevice(dev), "cudaSetDevice");
     const long long l0 = launches;
     res.maxt = opt.maxt;
-    const RDev sp = upload(spec);
-    Table *tab = table(sp, spec, opt, cb, res);
+    const uint64_t fp = table_fingerprint(spec);
+    const RDev sp = upload(spec, fp);
+    Table *tab = table(sp, spec, fp, opt, cb, res);
     res.table_cosets = tab->ns;
     res.table_levels = tab->D.top();
     const int Dtop = tab->D.top();
-    Tree T;
-    try {
+    Tree &T = search;
+    T.n.assign(1, 0);
+    {
       std::vector<int> mats;
       for (int r = 0; r < spec.nroot; r++) {
         const std::vector<int> m = packed(spec.re[r], spec.rx.data() + (size_t)r * NE, spec.ry.data() + (size_t)r * NE);
@@ -676,11 +682,7 @@ class RusContext {
         }
         if (j + Dtop >= opt.maxt) break;
       }
-      T.release();
       res.rc = rc;
-    } catch (...) {
-      T.release();
-      throw;
     }
     res.launches = launches - l0;
     res.total_seconds = now_s() - t0;
@@ -689,47 +691,47 @@ class RusContext {
 };
 
 int parse_rspec(const char *text, size_t len, RSpec &s, std::string &err) {
-  std::istringstream in(std::string(text, len));
+  TextCursor in{text, text + len};
   std::string tok;
   int ver = 0;
-  if (!(in >> tok) || tok != "rus-spec" || !(in >> ver)) { err = "not a rus spec"; return 2; }
+  if (!in.word(tok) || tok != "rus-spec" || !in.stream_int(ver)) { err = "not a rus spec"; return 2; }
   bool have_t = false, have_c = false;
   auto read_mat = [&](std::vector<int> &x, std::vector<int> &y, int &e) {
-    if (!(in >> e)) return false;
+    if (!in.stream_int(e)) return false;
     for (int i = 0; i < NE; i++) {
       int a, b;
-      if (!(in >> a >> b)) return false;
+      if (!in.stream_int(a) || !in.stream_int(b)) return false;
       x.push_back(a); y.push_back(b);
     }
     return true;
   };
-  while (in >> tok) {
+  while (in.word(tok)) {
     if (tok == "table-root") {
       s.tx.clear(); s.ty.clear();
       if (!read_mat(s.tx, s.ty, s.te)) { err = "bad table-root"; return 2; }
       have_t = true;
     } else if (tok == "roots") {
       int m = 0;
-      if (!(in >> m) || m < 0 || m > (1 << 20)) { err = "bad roots"; return 2; }
+      if (!in.stream_int(m) || m < 0 || m > (1 << 20)) { err = "bad roots"; return 2; }
       s.nroot = m; s.rx.clear(); s.ry.clear(); s.re.assign(m, 0);
       for (int r = 0; r < m; r++)
         if (!read_mat(s.rx, s.ry, s.re[r])) { err = "bad roots"; return 2; }
     } else if (tok == "rotations") {
       int m = 0;
-      if (!(in >> m) || m < 0 || m > 64) { err = "bad rotations"; return 2; }
+      if (!in.stream_int(m) || m < 0 || m > 64) { err = "bad rotations"; return 2; }
       s.tr.assign((size_t)m * NR, 0); s.ts.assign((size_t)m * NR, 0);
       for (int i = 0; i < m * NR; i++)
-        if (!(in >> s.tr[i] >> s.ts[i]) || s.tr[i] < -1 || s.tr[i] >= NR || s.ts[i] < -1 || s.ts[i] > 1) {
+        if (!in.stream_int(s.tr[i]) || !in.stream_int(s.ts[i]) || s.tr[i] < -1 || s.tr[i] >= NR || s.ts[i] < -1 || s.ts[i] > 1) {
           err = "bad rotations"; return 2;
         }
     } else if (tok == "cliffords") {
       int m = 0;
-      if (!(in >> m)) { err = "bad cliffords"; return 2; }
+      if (!in.stream_int(m)) { err = "bad cliffords"; return 2; }
       if (m != NCL) { err = "expected 11520 Cliffords"; return 2; }
       s.perm.assign((size_t)m * NR, 0); s.sign.assign((size_t)m * NR, 0);
       for (int i = 0; i < m * NR; i++) {
         int p, g;
-        if (!(in >> p >> g) || p < 0 || p >= NR || (g != 1 && g != -1)) { err = "bad cliffords"; return 2; }
+        if (!in.stream_int(p) || !in.stream_int(g) || p < 0 || p >= NR || (g != 1 && g != -1)) { err = "bad cliffords"; return 2; }
         s.perm[i] = (uint8_t)p; s.sign[i] = (int8_t)g;
       }
       have_c = true;
@@ -741,13 +743,13 @@ int parse_rspec(const char *text, size_t len, RSpec &s, std::string &err) {
     }
   }
   if (!s.nroot || !have_t || s.tr.size() != (size_t)NG * NR || !have_c) { err = "incomplete spec"; return 2; }
-  std::vector<int> bygen(1 << 20, -1);
+  std::vector<bool> seen(1 << 20, false);
   const int G[4] = {1, 3, 4, 12};
   for (int c = 0; c < NCL; c++) {
     int key = 0;
     for (int g = 0; g < 4; g++) key |= ((s.perm[c * NR + G[g]] << 1) | (s.sign[c * NR + G[g]] < 0)) << (5 * g);
-    if (bygen[key] >= 0) { err = "Clifford table: generator images not unique"; return 2; }
-    bygen[key] = c;
+    if (seen[key]) { err = "Clifford table: generator images not unique"; return 2; }
+    seen[key] = true;
   }
   return 0;
 }

@@ -1,5 +1,6 @@
 // Spec parsing, symmetry group and gate properties (host side of the boundary).
 #include "cz_spec.h"
+#include "cz_text.h"
 
 #include <algorithm>
 #include <cctype>
@@ -17,22 +18,12 @@ namespace {
 
 // whitespace tokenizer with std::istream-like failure: a failed numeric read poisons the stream
 struct Reader {
-  const char *p, *end;
+  TextCursor in;
   bool fail = false;
-  bool tok(std::string &s) {
-    while (p < end && std::isspace((unsigned char)*p)) p++;
-    if (p >= end) return false;
-    const char *b = p;
-    while (p < end && !std::isspace((unsigned char)*p)) p++;
-    s.assign(b, p);
-    return true;
-  }
+  bool tok(std::string &s) { return in.word(s); }
   int64_t num() {
-    std::string s;
-    if (fail || !tok(s)) { fail = true; return 0; }
-    char *e;
-    const long long v = std::strtoll(s.c_str(), &e, 10);
-    if (e == s.c_str()) { fail = true; return 0; }
+    long long v = 0;
+    if (fail || !in.word_number(v)) { fail = true; return 0; }
     return v;
   }
   Zw zw() { Zw z; z.a = num(); z.b = num(); z.c = num(); z.d = num(); return z; }

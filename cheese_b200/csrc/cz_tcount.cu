@@ -24,6 +24,7 @@
 #include <stdexcept>
 
 #include "cz_sort.cuh"
+#include "cz_text.h"
 #include "cz_tcount.h"
 
 namespace cz {
@@ -926,22 +927,12 @@ Table *TcountContext::table(const TDev &si, const TSpec &sp, const TcOptions &op
 
 int parse_tspec(const char *text, size_t len, TSpec &s, std::string &err) {
   s = TSpec{};
-  const char *p = text, *end = text + len;
-  auto tok = [&](std::string &out) {
-    while (p < end && std::isspace((unsigned char)*p)) p++;
-    if (p >= end) return false;
-    const char *b = p;
-    while (p < end && !std::isspace((unsigned char)*p)) p++;
-    out.assign(b, p);
-    return true;
-  };
+  TextCursor in{text, text + len};
+  auto tok = [&](std::string &out) { return in.word(out); };
   bool fail = false;
   auto num = [&]() -> long long {
-    std::string t;
-    if (fail || !tok(t)) { fail = true; return 0; }
-    char *e;
-    const long long v = std::strtoll(t.c_str(), &e, 10);
-    if (e == t.c_str()) { fail = true; return 0; }
+    long long v = 0;
+    if (fail || !in.word_number(v)) { fail = true; return 0; }
     return v;
   };
   std::string t;
