@@ -259,6 +259,121 @@ __device__ bool blk_same(const TSm &s, int ea, int eb, int P) {
   return blk_same_counted(s, P);                  // a hash group holds different columns: count exact matches
 }
 
+// ---------------- one warp per child ----------------
+// A child of a parent matrix M (entries (x, y) for x + y sqrt2, row-major) under rotation p: row a is M[a] sqrt2 = (2y, x)
+// where the rotation commutes (tr < 0), else M[a] - s M[r]; then d divisions by sqrt2, (x, y) -> (y, x / 2), as long as
+// every x is even: with vx, vy the least 2-adic valuations of the x and the y, d = min(2 vx, 2 vy + 1, e). Lane l holds
+// columns l and l + 32. The key is blk_colkey's: column hashes of the sign-normalised columns, summed.
+constexpr int NO_ORDER = INT32_MIN;            // a child's exponent where its columns were not ordered
+template <int LP> struct WarpChild {
+  static constexpr int P = 1 << LP, CPL = P > 32 ? 2 : 1;
+  static constexpr int LIMIT = 1 << 30;        // entries below this cannot overflow in one peel
+
+  // row a of the child before the divisions, the lane's column c
+  template <typename Mat>
+  __device__ __forceinline__ static int2 entry(const Mat &M, int a, int c, int r, int sg) {
+    const int2 m = M(a, c);
+    if (r < 0) return make_int2(2 * m.y, m.x);
+    const int2 o = M(r, c);
+    return make_int2(m.x - sg * o.x, m.y - sg * o.y);
+  }
+  __device__ __forceinline__ static int2 divided(int2 v, int d) {
+    const int k = d >> 1;
+    return (d & 1) ? make_int2(v.y >> k, v.x >> (k + 1)) : make_int2(v.x >> k, v.y >> k);
+  }
+  // the number of divisions of the child of exponent ie + 1 before them (warp-uniform)
+  template <typename Mat>
+  __device__ __forceinline__ static int divisions(const Mat &M, int ie, const int8_t *tr, const int8_t *ts, int lane) {
+    int X = 0, Y = 0;
+#pragma unroll 8
+    for (int a = 0; a < P; a++) {
+      const int r = __ldg(&tr[a]), sg = __ldg(&ts[a]);
+#pragma unroll
+      for (int j = 0; j < CPL; j++) {
+        const int c = lane + 32 * j;
+        if (c >= P) continue;
+        const int2 v = entry(M, a, c, r, sg);
+        X |= v.x; Y |= v.y;
+      }
+    }
+    X = (int)__reduce_or_sync(FULLM, (unsigned)X);
+    Y = (int)__reduce_or_sync(FULLM, (unsigned)Y);
+    const int vx = X ? __ffs(X) - 1 : 1 << 20, vy = Y ? __ffs(Y) - 1 : 1 << 20;
+    return min(min(2 * vx, 2 * vy + 1), ie + 1);
+  }
+  // the child's column hashes (t1, t2 per lane column), signs and key
+  template <typename Mat>
+  __device__ __forceinline__ static void key(const Mat &M, int e, int d, const int8_t *tr, const int8_t *ts, const ulonglong2 *w,
+                                             int lane, uint64_t (&t1)[CPL], int (&sign)[CPL], uint64_t &k1, uint64_t &k2) {
+    uint64_t p1[CPL], p2[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) { p1[j] = p2[j] = 0; sign[j] = 0; }
+#pragma unroll 4
+    for (int a = 0; a < P; a++) {
+      const int r = __ldg(&tr[a]), sg = __ldg(&ts[a]);
+      const ulonglong2 wa = w[a];
+#pragma unroll
+      for (int j = 0; j < CPL; j++) {
+        const int c = lane + 32 * j;
+        if (c >= P) continue;
+        const int2 v = divided(entry(M, a, c, r, sg), d);
+        if (sign[j] == 0 && (v.x | v.y)) sign[j] = (v.x > 0 || (v.x == 0 && v.y > 0)) ? 1 : -1;
+        const uint64_t h = (uint64_t)(uint32_t)(sign[j] * v.x) | ((uint64_t)(uint32_t)(sign[j] * v.y) << 32);
+        p1[j] += h * wa.x;
+        p2[j] += h * wa.y;
+      }
+    }
+    uint64_t s1 = 0, s2 = 0;
+#pragma unroll
+    for (int j = 0; j < CPL; j++) {
+      t1[j] = ~0ULL;
+      if (lane + 32 * j >= P) continue;
+      if (sign[j] == 0) sign[j] = 1;
+      t1[j] = fmix(p1[j] + 0x632be59bd9b4e019ULL);
+      s1 += t1[j];
+      s2 += fmix(p2[j] ^ 0x8cb92ba72f3d8dd7ULL);
+    }
+#pragma unroll
+    for (int m = 16; m; m >>= 1) { s1 += __shfl_xor_sync(FULLM, s1, m); s2 += __shfl_xor_sync(FULLM, s2, m); }
+    k1 = fmix(s1 + (uint64_t)(int64_t)e * 0xa0761d6478bd642fULL);
+    k2 = fmix(s2 ^ ((uint64_t)(int64_t)e * 0xe7037ed1a0b428dbULL + 0x5555ULL));
+  }
+  // the columns in the order of their hashes (58 bits, then the column: equal columns stay together): a bitonic sort of
+  // 64 elements, element i at lane i % 32, word i / 32. Word j of lane l gets the column at place l + 32 j, bit 7 its sign.
+  __device__ __forceinline__ static void order(const uint64_t (&t1)[CPL], const int (&sign)[CPL], int lane, uint8_t (&out)[CPL]) {
+    uint64_t k[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) k[j] = lane + 32 * j < P ? (t1[j] & ~63ULL) | (uint64_t)(lane + 32 * j) : ~0ULL;
+#pragma unroll
+    for (int size = 2; size <= 32 * CPL; size <<= 1) {
+#pragma unroll
+      for (int o = size >> 1; o; o >>= 1) {
+        if (o == 32) {                         // within the lane
+          if constexpr (CPL == 2) {
+            if (k[0] > k[1]) { const uint64_t t = k[0]; k[0] = k[1]; k[1] = t; }
+          }
+          continue;
+        }
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+          const uint64_t other = __shfl_xor_sync(FULLM, k[j], o);
+          const bool up = ((lane + 32 * j) & size) == 0, low = (lane & o) == 0;
+          k[j] = (k[j] < other) == (up == low) ? k[j] : other;
+        }
+      }
+    }
+    unsigned neg[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) neg[j] = __ballot_sync(FULLM, lane + 32 * j < P && sign[j] < 0);
+#pragma unroll
+    for (int j = 0; j < CPL; j++) {
+      const int c = (int)(k[j] & 63);
+      const unsigned m = CPL == 2 && c >= 32 ? neg[CPL - 1] : neg[0];
+      out[j] = (uint8_t)(c | (((m >> (c & 31)) & 1u) << 7));
+    }
+  }
+};
+
 // ---------------- kernels ----------------
 // keys of the nodes [0, n) of level t of tree H (the root when t = 0)
 __global__ void __launch_bounds__(TC_T) k_tc_keys(const TDev sp, const THist H, int t, long long n, uint64_t *k1o,
@@ -273,26 +388,70 @@ __global__ void __launch_bounds__(TC_T) k_tc_keys(const TDev sp, const THist H, 
   }
 }
 
-// child o = parent i * G + (p - 1): parent i of level tp, peeled by rotation p. With pmx, each parent's matrix and
-// exponent are kept (2 P^2 ints at pmx + 2 P^2 i, pe[i]) so the exact dedupe rebuilds a child with one peel.
-__global__ void __launch_bounds__(TC_T, 2) k_tc_children(const TDev sp, const THist H, int tp, long long m, uint64_t *k1o,
-                                                      uint64_t *k2o, int *ovf, int *pmx, int *pe) {
-  const TSm s = tsm_carve(sp.P);
-  const int G = sp.G, PP = sp.P * sp.P;
-  for (long long i = blockIdx.x; i < m; i += gridDim.x) {
+// child o = parent i * G + (p - 1): parent i of level tp, peeled by rotation p. A CTA rebuilds its parent in shared memory,
+// then each of its warps takes one rotation at a time; `split` CTAs share a parent when a level has few. With pmx, each
+// parent's matrix and exponent are kept (P^2 int2 at pmx + P^2 i, pe[i]) and per child its exponent (ce) and its columns in
+// the order of their hashes (co), so the exact dedupe compares two children column by column without searching.
+// Bound by issue (about 4000 instructions a child). One CTA per child, step by step, took 32 ns a child on
+// the B200; a warp per child 10 ns (380,000 children of two queries of T count 7: 12.2 -> 3.8 ms).
+template <int LP>
+__global__ void __launch_bounds__(TC_T) k_tc_children(const TDev sp, const THist H, int tp, long long m, int split,
+                                                      uint64_t *k1o, uint64_t *k2o, int *ovf, int2 *pmx, int *pe, uint8_t *co,
+                                                      int *ce) {
+  using W = WarpChild<LP>;
+  constexpr int P = W::P, PP = P * P;
+  const TSm s = tsm_carve(P);
+  int2 *M = (int2 *)s.bx;                      // the parent, entries interleaved (over the unused second matrix)
+  __shared__ ulonglong2 w[MAXP];
+  __shared__ int big;
+  for (int i = threadIdx.x; i < P; i += blockDim.x) w[i] = make_ulonglong2(s.w1[i], s.w2[i]);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, G = sp.G;
+  const auto mat = [&](int a, int c) { return M[a * P + c]; };
+  for (long long job = blockIdx.x; job < m * split; job += gridDim.x) {
+    const long long i = job / split;
+    const int part = (int)(job % split);
+    if (threadIdx.x == 0) big = 0;
     blk_path(H, tp, (uint32_t)i, s.seq);
     const int e = blk_build(s.ax, s.ay, sp, s.seq, tp, ovf);
-    if (pmx) {
-      int *dst = pmx + (size_t)i * 2 * PP;
-      for (int x = threadIdx.x; x < PP; x += blockDim.x) { dst[x] = s.ax[x]; dst[PP + x] = s.ay[x]; }
-      if (threadIdx.x == 0) pe[i] = e;
+    bool large = false;
+    for (int x = threadIdx.x; x < PP; x += blockDim.x) {
+      const int2 v = make_int2(s.ax[x], s.ay[x]);
+      large |= v.x >= W::LIMIT || v.x <= -W::LIMIT || v.y >= W::LIMIT || v.y <= -W::LIMIT;
+      M[x] = v;
+      if (pmx && part == 0) pmx[(size_t)i * PP + x] = v;
     }
-    for (int p = 1; p <= G; p++) {
-      const int ec = blk_peel(s.ax, s.ay, e, s.bx, s.by, p, sp, ovf);
-      uint64_t k1, k2;
-      blk_colkey(s.bx, s.by, ec, sp.P, s.fb, s.sb, s.b1, s.b2, s, k1, k2);
-      if (threadIdx.x == 0) { k1o[i * G + p - 1] = k1; k2o[i * G + p - 1] = k2; }
+    if (pmx && part == 0 && threadIdx.x == 0) pe[i] = e;
+    if (large) big = 1;
+    __syncthreads();
+    if (big) {                                 // entries so large that a peel may leave 32 bits: checked, a child at a time
+      for (int p = 1 + part; p <= G; p += split) {
+        const int ec = blk_peel(s.ax, s.ay, e, s.bx, s.by, p, sp, ovf);
+        uint64_t k1, k2;
+        blk_colkey(s.bx, s.by, ec, P, s.fb, s.sb, s.b1, s.b2, s, k1, k2);
+        const size_t o = (size_t)i * G + p - 1;
+        if (threadIdx.x == 0) { k1o[o] = k1; k2o[o] = k2; if (pmx) ce[o] = NO_ORDER; }
+      }
+      __syncthreads();
+      continue;
     }
+    for (int p = 1 + part * (TC_T / 32) + wp; p <= G; p += split * (TC_T / 32)) {
+      const int8_t *tr = sp.tr + (p - 1) * P, *ts = sp.ts + (p - 1) * P;
+      const int d = W::divisions(mat, e, tr, ts, lane), ec = e + 1 - d;
+      uint64_t t1[W::CPL], k1, k2;
+      int sign[W::CPL];
+      W::key(mat, ec, d, tr, ts, w, lane, t1, sign, k1, k2);
+      const size_t o = (size_t)i * G + p - 1;
+      if (lane == 0) { k1o[o] = k1; k2o[o] = k2; }
+      if (pmx) {
+        uint8_t ord[W::CPL];
+        W::order(t1, sign, lane, ord);
+#pragma unroll
+        for (int j = 0; j < W::CPL; j++)
+          if (lane + 32 * j < P) co[o * P + lane + 32 * j] = ord[j];
+        if (lane == 0) ce[o] = ec;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -319,54 +478,72 @@ __global__ void k_tc_split(const uint64_t *keys, const uint32_t *vals, size_t n,
     else check[atomicAdd(&st->n_work, 1ULL)] = (uint32_t)i;
   }
 }
-// one CTA per listed member: is it exactly the coset of its run's first member (equal h2 and the same multiset of
-// columns)? Children are rebuilt from their kept parents with one peel. A member that is not counts as unresolved:
-// the level is then deduped by the sequential resolver instead, which handles any mix of cosets in a run.
+// one warp per listed member: is it exactly the coset of its run's first member (equal h2 and exponent, and equal columns
+// up to sign in the order of their hashes)? Children's entries are recomputed from their kept parents. A member that is not,
+// be it for columns whose hashes agree by chance, counts as unresolved: the level is then deduped by the sequential
+// resolver instead, which handles any mix of cosets in a run. Bound by L2 (64 KB of parents a member); one CTA per member
+// with both children rebuilt, hashed and matched took 125 ns a member on the B200, this 11 ns (114,000 members: 14.3 -> 1.25 ms).
+template <int LP>
 __global__ void __launch_bounds__(TC_T) k_tc_dupcheck(const TDev sp, const uint64_t *keys, const uint32_t *vals,
                                                       size_t n, const uint32_t *check, const uint64_t *h2,
-                                                      const int *pmx, const int *pe, TcStats *st,
-                                                      unsigned long long *unresolved, int *ovf) {
-  const TSm s = tsm_carve(sp.P);
-  const int G = sp.G, PP = sp.P * sp.P;
+                                                      const int2 *pmx, const int *pe, const uint8_t *co, const int *ce,
+                                                      TcStats *st, unsigned long long *unresolved) {
+  using W = WarpChild<LP>;
+  constexpr int P = W::P, PP = P * P;
+  const int G = sp.G, lane = threadIdx.x & 31;
   const unsigned long long nw = st->n_work;
-  auto child = [&](uint32_t v, int *mx, int *my) {
-    const int *src = pmx + (size_t)(v / G) * 2 * PP;
-    for (int x = threadIdx.x; x < PP; x += blockDim.x) { mx[x] = src[x]; my[x] = src[PP + x]; }
-    __syncthreads();
-    return blk_peel(mx, my, pe[v / G], mx, my, (int)(v % G) + 1, sp, ovf);
-  };
-  for (unsigned long long w = blockIdx.x; w < nw; w += gridDim.x) {
+  unsigned long long bad = 0;
+  for (unsigned long long w = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5; w < nw;
+       w += ((unsigned long long)gridDim.x * blockDim.x) >> 5) {
     const uint32_t i = check[w];
     const uint64_t key = keys[i];
     size_t lo = 0, hi = i;                       // the run's first position: lower bound of the key
     while (lo < hi) { const size_t mid = (lo + hi) / 2; if (keys[mid] < key) lo = mid + 1; else hi = mid; }
-    const uint32_t v0 = vals[lo], vi = vals[i];
-    bool same = h2[v0] == h2[vi];
+    const uint32_t v0 = vals[lo], v1 = vals[i];
+    bool same = h2[v0] == h2[v1] && ce[v0] == ce[v1] && ce[v0] != NO_ORDER;
     if (same) {
-      const int ea = child(v0, s.ax, s.ay);
-      uint64_t k1, k2;
-      blk_colkey(s.ax, s.ay, ea, sp.P, s.fa, s.sa, s.a1, s.a2, s, k1, k2);
-      const int eb = child(vi, s.bx, s.by);
-      blk_colkey(s.bx, s.by, eb, sp.P, s.fb, s.sb, s.b1, s.b2, s, k1, k2);
-      same = blk_same(s, ea, eb, sp.P);
+      const int2 *A = pmx + (size_t)(v0 / G) * PP, *B = pmx + (size_t)(v1 / G) * PP;
+      const int pa = (int)(v0 % G), pb = (int)(v1 % G);
+      const int8_t *tra = sp.tr + pa * P, *tsa = sp.ts + pa * P, *trb = sp.tr + pb * P, *tsb = sp.ts + pb * P;
+      const int da = pe[v0 / G] + 1 - ce[v0], db = pe[v1 / G] + 1 - ce[v1];
+      const auto ma = [&](int a, int c) { return __ldg(&A[a * P + c]); };
+      const auto mb = [&](int a, int c) { return __ldg(&B[a * P + c]); };
+      int ca[W::CPL], cb[W::CPL];
+#pragma unroll
+      for (int j = 0; j < W::CPL; j++) {
+        ca[j] = lane + 32 * j < P ? co[(size_t)v0 * P + lane + 32 * j] : 0;
+        cb[j] = lane + 32 * j < P ? co[(size_t)v1 * P + lane + 32 * j] : 0;
+      }
+#pragma unroll 4
+      for (int a = 0; a < P; a++) {
+        const int ra = __ldg(&tra[a]), sa = __ldg(&tsa[a]), rb = __ldg(&trb[a]), sb = __ldg(&tsb[a]);
+#pragma unroll
+        for (int j = 0; j < W::CPL; j++) {
+          if (lane + 32 * j >= P) continue;
+          const int2 x = W::divided(W::entry(ma, a, ca[j] & 63, ra, sa), da);
+          const int2 y = W::divided(W::entry(mb, a, cb[j] & 63, rb, sb), db);
+          const int f = (ca[j] ^ cb[j]) & 128 ? -1 : 1;
+          same = same && x.x == f * y.x && x.y == f * y.y;
+        }
+      }
     }
-    if (!same && threadIdx.x == 0) atomicAdd(unresolved, 1ULL);
-    __syncthreads();
+    if (!__all_sync(FULLM, same)) bad++;
   }
+  if (lane == 0 && bad) atomicAdd(unresolved, bad);
 }
 
 // one CTA per run of equal key prefixes: order by (h1, h2, index), keep the first member of every exact coset
 __global__ void __launch_bounds__(TC_T) k_tc_resolve(const TDev sp, const THist H, int tp, const uint2 *work,
                                                      const uint32_t *vals, const uint64_t *h1, const uint64_t *h2,
                                                      uint32_t *tmp, uint64_t *kept, TcStats *st, int *ovf,
-                                                     const int *pmx, const int *pe) {
+                                                     const int2 *pmx, const int *pe) {
   const TSm s = tsm_carve(sp.P);
   const int G = sp.G, PP = sp.P * sp.P;
   // child v of level tp + 1 into (mx, my): its parent's kept matrix peeled once, or rebuilt from the base
   auto child = [&](uint32_t v, int *mx, int *my) {
     if (pmx) {
-      const int *src = pmx + (size_t)(v / G) * 2 * PP;
-      for (int x = threadIdx.x; x < PP; x += blockDim.x) { mx[x] = src[x]; my[x] = src[PP + x]; }
+      const int2 *src = pmx + (size_t)(v / G) * PP;
+      for (int x = threadIdx.x; x < PP; x += blockDim.x) { mx[x] = src[x].x; my[x] = src[x].y; }
       __syncthreads();
       return blk_peel(mx, my, pe[v / G], mx, my, (int)(v % G) + 1, sp, ovf);
     }
@@ -440,18 +617,34 @@ __global__ void k_tc_gather(const uint64_t *kidx, size_t nk, int G, const uint64
   }
 }
 
-// node j of level t of (sq, Hq) against the table (st, Ht) with sorted keys S1/S2 and (idx, lvl): the entry of
-// an exactly equal coset with level <= maxc, the smallest such level first; -1 if none
-__global__ void __launch_bounds__(TC_T) k_tc_lookup(const TDev sq, const THist Hq, int t, const uint64_t *F1,
-                                                    const uint64_t *F2, long long n, const TDev st, const THist Ht,
-                                                    const uint64_t *S1, const uint64_t *S2, const uint32_t *Sidx,
-                                                    const uint32_t *Slvl, long long nd, int maxc, long long *hit,
-                                                    int *ovf) {
-  const TSm s = tsm_carve(sq.P);
-  for (long long j = blockIdx.x; j < n; j += gridDim.x) {
+// nodes [0, n) against the table's sorted keys S1/S2, one thread each: those with an entry of equal keys and level <= maxc
+// are listed for the exact comparison, with the first entry of equal S1 in hit; hit is -1 for the others
+__global__ void k_tc_find(const uint64_t *F1, const uint64_t *F2, long long n, const uint64_t *S1, const uint64_t *S2,
+                          const uint32_t *Slvl, long long nd, int maxc, long long *hit, uint32_t *list, unsigned *count) {
+  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
     const uint64_t f1 = F1[j], f2 = F2[j];
     long long lo = 0, hi = nd;                                        // first entry with S1 >= f1
     while (lo < hi) { const long long mid = (lo + hi) >> 1; if (S1[mid] < f1) lo = mid + 1; else hi = mid; }
+    bool found = false;
+    for (long long x = lo; x < nd && S1[x] == f1 && !found; x++) found = S2[x] == f2 && (int)Slvl[x] <= maxc;
+    hit[j] = found ? lo : -1;
+    if (found) list[atomicAdd(count, 1u)] = (uint32_t)j;
+  }
+}
+// listed node j of level t of (sq, Hq) against the table (st, Ht) with sorted keys S1/S2 and (idx, lvl): the entry of
+// an exactly equal coset with level <= maxc, the smallest such level first; -1 if none
+__global__ void __launch_bounds__(TC_T) k_tc_lookup(const TDev sq, const THist Hq, int t, const uint64_t *F1,
+                                                    const uint64_t *F2, const uint32_t *list, const unsigned *count,
+                                                    const TDev st, const THist Ht, const uint64_t *S1, const uint64_t *S2,
+                                                    const uint32_t *Sidx, const uint32_t *Slvl, long long nd, int maxc,
+                                                    long long *hit, int *ovf) {
+  const unsigned n = *count;
+  if (blockIdx.x >= n) return;
+  const TSm s = tsm_carve(sq.P);
+  for (unsigned l = blockIdx.x; l < n; l += gridDim.x) {
+    const long long j = list[l], lo = hit[j];
+    const uint64_t f1 = F1[j], f2 = F2[j];
+    __syncthreads();                                                  // everyone has read hit[j]
     long long res = -1;
     int rl = 1 << 30;
     bool built = false;
@@ -523,7 +716,7 @@ struct Tree {
   Buf F1, F2;                      // keys of the top level
   int top() const { return (int)n.size() - 1; }
   THist hist() const {
-    if (par.size() != n.size() || gat.size() != n.size()) throw std::logic_error("tree levels out of step");
+    if (par.size() < n.size() || gat.size() < n.size()) throw std::logic_error("tree levels out of step");
     THist H{};
     for (int l = 1; l <= top() && l <= MAXT; l++) { H.par[l] = par[l].as<uint32_t>(); H.gat[l] = gat[l].as<uint8_t>(); }
     return H;
@@ -546,7 +739,9 @@ class TcountContext {
   std::map<std::pair<int, int>, Table *> tables;   // resident: (n, K)
   Buf bx, by, ix, iy, tr, ts, ovf, stats;
   Buf h1, h2, k0, k1, v0, v1, hist, part, work, tmp, kept, hits;
-  Buf pmat, pexp;                                  // parents' matrices and exponents of the level being grown
+  Buf pmat, pexp, cord, cexp;                      // parents' matrices and exponents, children's column orders and exponents
+  Buf list;                                        // a lookup's count and listed nodes
+  Tree search;                                     // the search's tree: its buffers stay for the next search
   long long launches = 0;
   TcountContext(int d, void *stream) : dev(d), s((cudaStream_t)stream) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -556,16 +751,19 @@ class TcountContext {
     for (auto &kv : tables) { kv.second->D.release(); kv.second->S1.release(); kv.second->S2.release();
                               kv.second->Sidx.release(); kv.second->Slvl.release(); delete kv.second; }
     for (Buf *b : {&bx, &by, &ix, &iy, &tr, &ts, &ovf, &stats, &h1, &h2, &k0, &k1, &v0, &v1, &hist, &part, &work, &tmp,
-                   &kept, &hits, &pmat, &pexp})
+                   &kept, &hits, &pmat, &pexp, &cord, &cexp, &list})
       b->release();
+    search.release();
   }
   size_t trim() {                              // work buffers back to the device; resident tables stay
     size_t n = 0;
     for (Buf *b : {&bx, &by, &ix, &iy, &tr, &ts, &h1, &h2, &k0, &k1, &v0, &v1, &hist, &part, &work, &tmp, &kept, &hits,
-                   &pmat, &pexp}) {
+                   &pmat, &pexp, &cord, &cexp, &list, &search.F1, &search.F2}) {
       n += b->cap;
       b->release();
     }
+    for (std::vector<Buf> *v : {&search.par, &search.gat}) for (Buf &b : *v) n += b.cap;
+    search.release();
     return n;
   }
   size_t smem(int P) const { return tsm_bytes(P); }
@@ -586,6 +784,20 @@ class TcountContext {
     tck(cudaGetLastError(), "keys kernel");
   }
 
+  // nodes [0, n) of level t of (sq, T) against the table: hits[j] = the entry of its coset with level <= maxc, or -1
+  void lookup(const TDev &sq, const Tree &T, int t, long long n, const TDev &st, const THist &Ht, const Table &tab, int maxc) {
+    list.ensure((size_t)n * 4 + 16);
+    unsigned *count = list.as<unsigned>();
+    tck(cudaMemsetAsync(count, 0, 4, s), "memset");
+    k_tc_find<<<(unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, (long long)nsm * 16)), 256, 0, s>>>(
+        T.F1.as<uint64_t>(), T.F2.as<uint64_t>(), n, tab.S1.as<uint64_t>(), tab.S2.as<uint64_t>(), tab.Slvl.as<uint32_t>(),
+        tab.ns, maxc, hits.as<long long>(), count + 1, count);
+    k_tc_lookup<<<grid(n), TC_T, smem(sq.P), s>>>(sq, T.hist(), t, T.F1.as<uint64_t>(), T.F2.as<uint64_t>(), count + 1, count,
+                                                  st, Ht, tab.S1.as<uint64_t>(), tab.S2.as<uint64_t>(), tab.Sidx.as<uint32_t>(),
+                                                  tab.Slvl.as<uint32_t>(), tab.ns, maxc, hits.as<long long>(), ovf.as<int>());
+    launches += 2;
+  }
+
   // one more level of T (peels off sp's base); table: drop cosets already in tab. Returns the new nodes.
   long long grow(const TDev &sp, Tree &T, Table *tab, const std::function<void(const TcLevel &)> &cb) {
     const double t0 = now_s();
@@ -596,13 +808,18 @@ class TcountContext {
     h1.ensure(nc * 8); h2.ensure(nc * 8);
     // the parents' matrices, kept for the exact dedupe (up to 16 GB; beyond, children are rebuilt from the base)
     const size_t pm_bytes = (size_t)m * 2 * sp.P * sp.P * 4;
-    int *pmx = nullptr, *pe = nullptr;
+    int2 *pmx = nullptr;
+    int *pe = nullptr;
     if (pm_bytes <= ((size_t)16 << 30)) {
       pmat.ensure(pm_bytes + 16); pexp.ensure((size_t)m * 4 + 16);
-      pmx = pmat.as<int>(); pe = pexp.as<int>();
+      cord.ensure((size_t)nc * sp.P + 16); cexp.ensure((size_t)nc * 4 + 16);
+      pmx = pmat.as<int2>(); pe = pexp.as<int>();
     }
-    k_tc_children<<<grid(m), TC_T, smem(sp.P), s>>>(sp, T.hist(), tp, m, h1.as<uint64_t>(), h2.as<uint64_t>(), ovf.as<int>(),
-                                                    pmx, pe);
+    // few parents: several CTAs share one (every warp then takes one rotation); a grid of two CTAs per SM at least
+    const int split = (int)std::max<long long>(1, std::min<long long>((G + TC_T / 32 - 1) / (TC_T / 32), (long long)nsm * 2 / std::max<long long>(m, 1)));
+    const auto children = sp.lp == 2 ? k_tc_children<2> : sp.lp == 4 ? k_tc_children<4> : k_tc_children<6>;
+    children<<<grid(m * split), TC_T, smem(sp.P), s>>>(sp, T.hist(), tp, m, split, h1.as<uint64_t>(), h2.as<uint64_t>(),
+                                                       ovf.as<int>(), pmx, pe, cord.as<uint8_t>(), cexp.as<int>());
     launches++;
     tck(cudaGetLastError(), "children kernel");
     check_ovf();
@@ -628,8 +845,9 @@ class TcountContext {
       const uint32_t *sv = f ? v1.as<uint32_t>() : v0.as<uint32_t>();
       tck(cudaMemsetAsync(stats.p, 0, sizeof(TcStats) + 8, s), "memset");
       k_tc_split<<<gb, 256, 0, s>>>(sk, sv, n, kept.as<uint64_t>(), tmp.as<uint32_t>(), stats.as<TcStats>());
-      k_tc_dupcheck<<<(unsigned)nsm * 8, TC_T, smem(sp.P), s>>>(sp, sk, sv, n, tmp.as<uint32_t>(), h2.as<uint64_t>(),
-                                                                pmx, pe, stats.as<TcStats>(), unres, ovf.as<int>());
+      const auto dupcheck = sp.lp == 2 ? k_tc_dupcheck<2> : sp.lp == 4 ? k_tc_dupcheck<4> : k_tc_dupcheck<6>;
+      dupcheck<<<(unsigned)nsm * 8, TC_T, 0, s>>>(sp, sk, sv, n, tmp.as<uint32_t>(), h2.as<uint64_t>(), pmx, pe,
+                                                  cord.as<uint8_t>(), cexp.as<int>(), stats.as<TcStats>(), unres);
       launches += 2;
       tck(cudaGetLastError(), "dedupe");
       unsigned long long hu = 0;
@@ -663,22 +881,19 @@ class TcountContext {
                                sc, s, nullptr);
     if (nk > 1) launches += 20;
     const uint64_t *kidx = fk ? k1.as<uint64_t>() : kept.as<uint64_t>();
-    T.par.emplace_back(); T.gat.emplace_back(); T.n.push_back((long long)nk);
-    T.par.back().ensure(nk * 4 + 4); T.gat.back().ensure(nk + 4);
+    T.n.push_back((long long)nk);
+    if ((int)T.par.size() <= t) { T.par.resize(t + 1); T.gat.resize(t + 1); }   // (a kept tree has its levels' buffers)
+    T.par[t].ensure(nk * 4 + 4); T.gat[t].ensure(nk + 4);
     T.F1.ensure(nk * 8 + 8); T.F2.ensure(nk * 8 + 8);
     k_tc_gather<<<(unsigned)std::max<size_t>(1, std::min<size_t>((nk + 255) / 256, (size_t)nsm * 16)), 256, 0, s>>>(
-        kidx, nk, G, h1.as<uint64_t>(), h2.as<uint64_t>(), T.par.back().as<uint32_t>(),
-        T.gat.back().as<uint8_t>(), T.F1.as<uint64_t>(), T.F2.as<uint64_t>());
+        kidx, nk, G, h1.as<uint64_t>(), h2.as<uint64_t>(), T.par[t].as<uint32_t>(),
+        T.gat[t].as<uint8_t>(), T.F1.as<uint64_t>(), T.F2.as<uint64_t>());
     launches++;
     tck(cudaGetLastError(), "gather");
     long long fresh = (long long)nk;
     if (tab && nk) {   // drop cosets present at a lower level, then add the rest to the table
       hits.ensure(nk * 8);
-      k_tc_lookup<<<grid(nk), TC_T, smem(sp.P), s>>>(sp, T.hist(), t, T.F1.as<uint64_t>(), T.F2.as<uint64_t>(), (long long)nk,
-                                                      sp, T.hist(), tab->S1.as<uint64_t>(), tab->S2.as<uint64_t>(),
-                                                      tab->Sidx.as<uint32_t>(), tab->Slvl.as<uint32_t>(), tab->ns, t - 1,
-                                                      hits.as<long long>(), ovf.as<int>());
-      launches++;
+      lookup(sp, T, t, (long long)nk, sp, T.hist(), *tab, t - 1);
       tck(cudaGetLastError(), "table filter");
       check_ovf();
       std::vector<long long> hh(nk);
@@ -686,8 +901,8 @@ class TcountContext {
       std::vector<uint8_t> hg(nk);
       std::vector<uint64_t> a1(nk), a2(nk);
       tck(cudaMemcpyAsync(hh.data(), hits.p, nk * 8, cudaMemcpyDeviceToHost, s), "d2h");
-      tck(cudaMemcpyAsync(hp.data(), T.par.back().p, nk * 4, cudaMemcpyDeviceToHost, s), "d2h");
-      tck(cudaMemcpyAsync(hg.data(), T.gat.back().p, nk, cudaMemcpyDeviceToHost, s), "d2h");
+      tck(cudaMemcpyAsync(hp.data(), T.par[t].p, nk * 4, cudaMemcpyDeviceToHost, s), "d2h");
+      tck(cudaMemcpyAsync(hg.data(), T.gat[t].p, nk, cudaMemcpyDeviceToHost, s), "d2h");
       tck(cudaMemcpyAsync(a1.data(), T.F1.p, nk * 8, cudaMemcpyDeviceToHost, s), "d2h");
       tck(cudaMemcpyAsync(a2.data(), T.F2.p, nk * 8, cudaMemcpyDeviceToHost, s), "d2h");
       tck(cudaStreamSynchronize(s), "d2h");
@@ -699,8 +914,8 @@ class TcountContext {
       fresh = (long long)np.size();
       T.n.back() = fresh;
       if (fresh) {
-        tck(cudaMemcpyAsync(T.par.back().p, np.data(), fresh * 4, cudaMemcpyHostToDevice, s), "h2d");
-        tck(cudaMemcpyAsync(T.gat.back().p, ng.data(), fresh, cudaMemcpyHostToDevice, s), "h2d");
+        tck(cudaMemcpyAsync(T.par[t].p, np.data(), fresh * 4, cudaMemcpyHostToDevice, s), "h2d");
+        tck(cudaMemcpyAsync(T.gat[t].p, ng.data(), fresh, cudaMemcpyHostToDevice, s), "h2d");
         tck(cudaMemcpyAsync(T.F1.p, n1.data(), fresh * 8, cudaMemcpyHostToDevice, s), "h2d");
         tck(cudaMemcpyAsync(T.F2.p, n2.data(), fresh * 8, cudaMemcpyHostToDevice, s), "h2d");
         tck(cudaStreamSynchronize(s), "h2d");
@@ -980,8 +1195,8 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
     tck(cudaSetDevice(ctx->dev), "cudaSetDevice");
     const int P = sp.P, lp = 2 * sp.n;
     const size_t sm = ctx->smem(P);
-    for (const void *k : {(const void *)k_tc_keys, (const void *)k_tc_children, (const void *)k_tc_resolve,
-                          (const void *)k_tc_dupcheck, (const void *)k_tc_lookup})
+    for (const void *k : {(const void *)k_tc_keys, (const void *)k_tc_children<2>, (const void *)k_tc_children<4>,
+                          (const void *)k_tc_children<6>, (const void *)k_tc_resolve, (const void *)k_tc_lookup})
       tck(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), "smem attribute");
     ctx->bx.ensure(P * P * 4); ctx->by.ensure(P * P * 4); ctx->ix.ensure(P * P * 4); ctx->iy.ensure(P * P * 4);
     ctx->tr.ensure(P * P); ctx->ts.ensure(P * P); ctx->ovf.ensure(4);
@@ -1003,7 +1218,8 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
     Table *tab = ctx->table(si, sp, opt, on_level, res);
     res.table_cosets = tab->ns;
     res.table_levels = tab->D.top();
-    Tree T;                                                       // search: peel rotations off U
+    Tree &T = ctx->search;                                        // search: peel rotations off U
+    T.n.assign(1, 1);
     ctx->level_keys(su, T, 0);
     ctx->check_ovf();
     int rc = 1;
@@ -1012,11 +1228,7 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
       const long long n = T.n[j];
       const int maxc = std::min(tab->D.top(), opt.maxt - j);
       ctx->hits.ensure(n * 8);
-      k_tc_lookup<<<ctx->grid(n), TC_T, sm, ctx->s>>>(su, T.hist(), j, T.F1.as<uint64_t>(), T.F2.as<uint64_t>(), n, si,
-                                                      tab->D.hist(), tab->S1.as<uint64_t>(), tab->S2.as<uint64_t>(),
-                                                      tab->Sidx.as<uint32_t>(), tab->Slvl.as<uint32_t>(), tab->ns, maxc,
-                                                      ctx->hits.as<long long>(), ctx->ovf.as<int>());
-      ctx->launches++;
+      ctx->lookup(su, T, j, n, si, tab->D.hist(), *tab, maxc);
       tck(cudaGetLastError(), "lookup");
       ctx->check_ovf();
       std::vector<long long> hh(n);
@@ -1055,7 +1267,6 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
       }
       if (j + tab->D.top() >= opt.maxt) break;
     }
-    T.release();
     res.rc = rc;
   } catch (const std::overflow_error &e) {
     res.error = e.what();

@@ -137,3 +137,32 @@ def test_cli_errors(tmp_path):
     assert p.returncode == 3
     p = subprocess.run([str(BIN)], capture_output=True, text=True, timeout=60)
     assert p.returncode == 3 and "usage" in p.stderr
+
+
+@pytest.mark.parametrize("shift", [0, 12, 28, 29, 30])
+@pytest.mark.parametrize("n", [1, 2])
+def test_scaled_channels_match_the_restatement(n, shift):
+    """a channel matrix written with its entries and exponent scaled up: many divisions per peel, and entries on both
+    sides of the size from which a peel may leave 32 bits (reported as an overflow, exit 4)"""
+    import cheese_b200 as cz
+    from conftest import ORACLE_DIR
+    oracle = ORACLE_DIR / "_ref" / "tc-oracle"
+    if not oracle.exists():
+        subprocess.run(["make", "-C", str(ORACLE_DIR), "oracle"], check=True, capture_output=True)
+    circ = [("t", (0,)), ("h", (0,)), ("t", (0,))] + ([("cx", (0, 1)), ("t", (1,))] if n == 2 else [])
+    rows = cz.tspec_generate(n, circ).split("\n")
+    c = next(i for i, l in enumerate(rows) if l.startswith("channel"))
+    rows[c] = f"channel {int(rows[c].split()[1]) + 2 * shift}"
+    for i in range(c + 1, c + 1 + 4 ** n):
+        rows[i] = " ".join(str(int(v) << shift) for v in rows[i].split())
+    text = "\n".join(rows)
+    import tempfile
+    with tempfile.NamedTemporaryFile("w", suffix=".tspec") as f:
+        f.write(text)
+        f.flush()
+        want = subprocess.run([str(oracle), f.name, "--table", "1", "--max", "6"], capture_output=True, text=True)
+    e = cz.Engine()
+    rc, levels, res = e.tcount(text, table_k=1, maxt=6, cache_dir=None)
+    e.close()
+    assert rc == want.returncode
+    assert lines(levels, rc, res) == strip_seconds(want.stdout.splitlines())
