@@ -1,6 +1,6 @@
 // Device primitives of the frontier dedupe: exclusive scan and a stable LSD radix sort of (u64 key, u32 value)
-// pairs over a chosen bit range, 8-bit digits, one launch per digit pass (see radix_sort). All launches go to the
-// caller's stream.
+// pairs over a chosen bit range, 8-bit digits, one launch per digit pass (see radix_sort); small sorts count each pair's
+// place in one launch. All launches go to the caller's stream.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -308,6 +308,50 @@ __global__ void __launch_bounds__(OS_THREADS, 4) k_sort_onesweep(const uint64_t 
   }
 }
 
+// Small sorts in one launch: a pair's place is the number of smaller keys plus the number of equal keys before it,
+// counted directly. A block places 32 pairs (one per lane); its warps share the keys, read tile by tile into shared
+// memory, and a key is compared with 32 at once from a broadcast. n^2 / 32 compares, but no passes, no scratch and one
+// launch where the digit passes need 1 + passes and a memset: up to SORT_COUNT_MAX keys it is faster (32-bit
+// digits on the B200, us: 1000 keys 36 -> 11, 4000 43 -> 16, 8192 46 -> 25; 8193 by digit passes 45).
+constexpr int SORT_COUNT_MAX = 8192;
+constexpr int SC_THREADS = 256, SC_TILE = 1024;
+template <typename K>     // uint32_t when hi - lo <= 32, else uint64_t: the digits compared
+__global__ void __launch_bounds__(SC_THREADS) k_sort_count(const uint64_t *kin, const uint32_t *vin, uint64_t *kout, uint32_t *vout,
+                                                           int n, int lo, uint64_t mask, unsigned *err) {
+  constexpr int NW = SC_THREADS / 32, PER = SC_TILE / NW;
+  __shared__ K tile[SC_TILE];
+  __shared__ int part[NW][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i0 = blockIdx.x * 32, i = i0 + lane;
+  if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;      // the scratch's flag, as a digit sort clears it
+  const K mine = i < n ? (K)((kin[i] >> lo) & mask) : 0;
+  int cnt = 0;
+  for (int t0 = 0; t0 < n; t0 += SC_TILE) {
+    const int tn = min(SC_TILE, n - t0);
+    __syncthreads();
+    for (int x = threadIdx.x; x < tn; x += SC_THREADS) tile[x] = (K)((kin[t0 + x] >> lo) & mask);
+    __syncthreads();
+    const int a = w * PER, b = min(a + PER, tn);
+    if (t0 + b <= i0) {                                          // all before the block's pairs: equal keys count
+#pragma unroll 8
+      for (int x = a; x < b; x++) cnt += tile[x] <= mine;
+    } else if (t0 + a >= i0 + 32) {                              // all behind them
+#pragma unroll 8
+      for (int x = a; x < b; x++) cnt += tile[x] < mine;
+    } else {
+      for (int x = a; x < b; x++) cnt += tile[x] < mine || (tile[x] == mine && t0 + x < i);
+    }
+  }
+  part[w][lane] = cnt;
+  __syncthreads();
+  if (w == 0 && i < n) {
+    int pos = 0;
+#pragma unroll
+    for (int x = 0; x < NW; x++) pos += part[x][lane];
+    kout[pos] = kin[i];
+    vout[pos] = vin[i];
+  }
+}
+
 struct SortScratch {
   uint32_t *hist = nullptr;       // sort scratch: sort_hist_words(n) words
   uint32_t *partials = nullptr;   // scan partials: scan_partials_words(sort_hist_words(n)) words (large sorts)
@@ -320,6 +364,16 @@ struct SortScratch {
 inline bool radix_sort(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, size_t n, int lo, int hi,
                        const SortScratch &sc, cudaStream_t s, int *launches) {
   if (n <= 1 || hi <= lo) return false;
+  if (n <= (size_t)SORT_COUNT_MAX) {
+    unsigned *own = sc.err ? nullptr : sc.hist + 256 * OS_MAXPASS + OS_MAXPASS;
+    const unsigned nb = (unsigned)((n + 31) / 32);
+    if (hi - lo <= 32)
+      k_sort_count<uint32_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 32 ? 0xffffffffULL : (1ULL << (hi - lo)) - 1, own);
+    else
+      k_sort_count<uint64_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 64 ? ~0ULL : (1ULL << (hi - lo)) - 1, own);
+    if (launches) (*launches)++;
+    return true;
+  }
   const int npass = (hi - lo + 7) / 8;
   const size_t ntiles = sort_tiles(n);
   const bool scan = n >= OS_SCAN_MIN && sc.partials && sc.cap_part >= scan_partials_words(256 * ntiles);
