@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <array>
 #include <chrono>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -108,6 +109,7 @@ static_assert(sizeof(TQEntry) == 24, "T queue entry layout");
 template <typename ST> struct ExpandArgs {
   long long m;
   int t, rem, keep;
+  int split;                       // warps that share a parent's candidates
   const Z4<ST> *R;
   const NodeMeta *meta;
   DevStats *st;
@@ -1106,7 +1108,7 @@ template <int NQ, typename ST, bool STATES = false, int PART = 0, typename Weigh
 __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *sps, Weight weight, unsigned conjmask,
                                               const Z4<ST> *P, Z4<ST> *C, uint32_t *F, unsigned long long p,
                                               const NodeMeta pm, int rem, bool keep, int GS, const ExpandOut<ST> &o,
-                                              WarpTally &c, int lane) {
+                                              WarpTally &c, int lane, int split = 1, int sub = 0) {
   constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
   const int G = sp.G;
   const int g1 = pm.g1 == 0xff ? -1 : pm.g1, g2 = pm.g2 == 0xff ? -1 : pm.g2;
@@ -1150,7 +1152,10 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
   for (int g0 = 0; g0 < G; g0 += 32) {
     const int g = g0 + lane;
     int fate = NONE, q0 = 0;
-    if (g < G && (PART == 0 || ((sp.gflags[g] & GF_ONEQ) != 0) == (PART == 1))) {
+    // with several warps to a parent, this one's share: the odd diagonals by qubit (siblings share a queue entry), the
+    // other candidates by index
+    const bool share = split == 1 || (g < G && ((sps->gflags[g] & GF_TDIAG) ? sps->gq[g][0] : g) % split == sub);
+    if (g < G && share && (PART == 0 || ((sp.gflags[g] & GF_ONEQ) != 0) == (PART == 1))) {
       fate = FULLC;
       if (g1 >= 0 && __ldg(&sp.bad2[g1 * G + g])) fate = W2;
       else if (g2 >= 0) {
@@ -1417,15 +1422,18 @@ __global__ void __launch_bounds__(EXP_WARPS * 32) k_goal_level(const DevSpec sp,
 }
 
 // A warp's parents: taken from a counter two ahead, the residual one ahead (copied into shared memory by cp.async while
-// the current parent is expanded), so neither the counter nor the loads are waited for. body(p, P, meta).
+// the current parent is expanded), so neither the counter nor the loads are waited for. body(p, P, meta, sub). A level
+// with fewer parents than warps on the chip splits each parent's candidates over `split` warps (sub = 0 .. split - 1).
 template <int NQ, typename ST, typename Body>
 __device__ __forceinline__ void walk_parents(ExpandSmem<NQ, ST> &sm, unsigned long long *counter, unsigned long long p0,
                                              unsigned long long end, const Z4<ST> *R, const NodeMeta *meta, int w, int lane,
-                                             Body body) {
+                                             int split, Body body) {
   constexpr int E = (1 << NQ) * (1 << NQ), NB = ExpandSmem<NQ, ST>::NB, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
   auto grab = [&]() { return lane == 0 ? p0 + atomicAdd(counter, 1ULL) : 0ULL; };
-  auto fetch = [&](unsigned long long p, int b, NodeMeta &m) {
-    if (p < end) {
+  auto parent = [&](unsigned long long it) { return split == 1 ? it : (unsigned long long)((unsigned)it / (unsigned)split); };
+  auto fetch = [&](unsigned long long it, int b, NodeMeta &m) {
+    if (it < end) {
+      const unsigned long long p = parent(it);
       const char *src = (const char *)(R + p * (unsigned long long)E);
       char *dst = (char *)sm.P[w][b];
       for (int i = lane; i < CHUNKS; i += 32) cp_async16(dst + 16 * i, src + 16 * i);
@@ -1444,7 +1452,7 @@ __device__ __forceinline__ void walk_parents(ExpandSmem<NQ, ST> &sm, unsigned lo
     if (NB == 2) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncwarp();
-    body(p, sm.P[w][b], m);
+    body(parent(p), sm.P[w][b], m, split == 1 ? 0 : (int)((unsigned)p % (unsigned)split));
     __syncwarp();
     if (NB == 1) fetch(pn, 0, mn);
     p = pn;
@@ -1470,10 +1478,10 @@ __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand(const DevSp
   const ExpandOut<ST> o{a.st, a.cap, a.sh1, a.sh2, a.sidx, a.smeta, a.tq, a.tqcap};
   const auto weight = [&](int s, int e) { return sm.Wt[s][e & (E - 1)]; };
   WarpTally c;
-  walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, 0, (unsigned long long)a.m, a.R, a.meta, w, lane,
-                       [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm) {
+  walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, 0, (unsigned long long)a.m * a.split, a.R, a.meta, w,
+                       lane, a.split, [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm, int sub) {
     expand_parent<NQ, ST, STATES, PART>(sp, &s_sp, weight, conjmask, P, sm.C[w], sm.F[w], p, pm, a.rem, a.keep != 0, sp.G,
-                                        o, c, lane);
+                                        o, c, lane, a.split, sub);
   });
   c.flush(a.st, lane);
 }
@@ -1666,7 +1674,7 @@ __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand_solo(const 
   const auto weight = [&](int s, int e) { return sm.Wt[s][e & (E - 1)]; };
   WarpTally c;
   walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, (unsigned long long)a.p0, (unsigned long long)a.m, a.R,
-                       a.meta, w, lane, [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm) {
+                       a.meta, w, lane, 1, [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm, int) {
     expand_parent<NQ, ST, false, PART>(sp, &s_sp, weight, conjmask, P, sm.C[w], sm.F[w], p, pm, sp.depth - t, t < sp.depth,
                                        BATCH_GS, o, c, lane);
   });
@@ -1901,12 +1909,22 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
 template <int NQ, typename ST> __global__ void k_root(const DevSpec sp, const Z4<ST> *R, NodeMeta *meta, int tk) {
   constexpr int E = (1 << NQ) * (1 << NQ);
   __shared__ Z4<ST> S[E];
+  __shared__ int4 Y[E];
+  __shared__ int X[E];
   const int lane = threadIdx.x;
   for (int e = lane; e < E; e += 32) S[e] = R[e];
   __syncwarp();
   int T = 0, c2 = 0, needs = 0;
   Cheap ch{false, 0, 0};
-  if (sp.standard || sp.lite) T = ptm_bound<NQ, ST>(S, tk, lane);
+  if (sp.standard || sp.lite) {
+    if (sp.unit && NQ + tk <= PACK_MAX) {
+      for (int e = lane; e < E; e += 32) { Y[e] = pack_entry(S[e]); X[e] = Y[e].x; }
+      __syncwarp();
+      T = packed_tbound<NQ>(Y, X, tk, lane, INT_MAX);
+    } else {
+      T = ptm_bound<NQ, ST>(S, tk, lane);
+    }
+  }
   if (sp.standard) {
     c2 = warp_cx_bound<NQ, ST>(S, sp, lane, 0, 0, needs);
     ch = warp_cheap<NQ, ST>(S, tk, sp, lane, false, true, (1 << NQ) - 1, 0);
@@ -2760,9 +2778,9 @@ struct Engine::Impl {
     ck(cudaSetDevice(dev), "cudaSetDevice");
     ck(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     for (auto &e : ev) ck(cudaEventCreate(&e), "event");
-    ck(cudaMallocHost(&hstats, sizeof(DevStats)), "pinned");
+    ck(cudaMallocHost(&hstats, sizeof(DevStats) + sizeof(GoalShort)), "pinned");
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    stats.ensure(sizeof(DevStats));
+    stats.ensure(sizeof(DevStats) + sizeof(GoalShort));
   }
   size_t trim() {
     size_t n = 0;
@@ -2816,6 +2834,17 @@ struct Engine::Impl {
   void table_save(const std::string &path, const DistTable &D);
 };
 
+// the gates of child o (parent * G + gate) of level t, walked back through the tree's levels, first gate first
+struct TreeLevels { const uint32_t *par[DMAX + 1]; const uint8_t *gat[DMAX + 1]; };
+__global__ void k_walk_back(const __grid_constant__ TreeLevels tree, unsigned long long o, int G, int t, uint8_t *out) {
+  out[t - 1] = (uint8_t)(o % (unsigned)G);
+  uint32_t i = (uint32_t)(o / (unsigned)G);
+  for (int l = t - 1; l >= 1; l--) {
+    out[l - 1] = tree.gat[l][i];
+    i = tree.par[l][i];
+  }
+}
+
 template <int NQ, typename ST>
 int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &opt, int depth, int &t_start,
                          const std::function<void(const LevelStats &)> &cb, SearchResult &res, int stop) {
@@ -2829,6 +2858,18 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
     float ms = 0;
     if (cudaEventElapsedTime(&ms, ev[2], ev[3]) == cudaSuccess) res.dedupe_ms += ms;
     ded_pending = false;
+  };
+  auto walk_back = [&](unsigned long long o, int t) {  // (the statistics have been read: their buffers carry the gates)
+    TreeLevels tree{};
+    for (int l = 1; l < t; l++) { tree.par[l] = par[l].as<uint32_t>(); tree.gat[l] = gat[l].as<uint8_t>(); }
+    k_walk_back<<<1, 1, 0, s>>>(tree, o, G, t, stats.as<uint8_t>());
+    launches++;
+    ck(cudaGetLastError(), "walk");
+    ck(cudaMemcpyAsync(hstats, stats.p, (size_t)t, cudaMemcpyDeviceToHost, s), "d2h");
+    d2h += t;
+    ck(cudaStreamSynchronize(s), "walk");
+    const uint8_t *q = (const uint8_t *)hstats;
+    return std::vector<int>(q, q + t);
   };
   if ((int)level_n.size() < t_start) level_n.resize(t_start, 0);
   for (int t = t_start; t <= depth && t <= stop; t++) {
@@ -2853,16 +2894,16 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
     GoalShort *gsd = nullptr;
     GoalShort hgs{0, 0, ~0ULL, 0, 0};
     const bool goal_pass = hs.standard && !hs.states && !sp.nogoal && m > 0;
-    if (goal_pass) {
-      gshort.ensure(sizeof(GoalShort) + (size_t)GOAL_LIST * 4 + 64);
-      gsd = gshort.as<GoalShort>();
+    if (goal_pass) {                         // its header lies behind the level's statistics: one copy brings both back
+      gshort.ensure((size_t)GOAL_LIST * 4 + 64);
+      gsd = (GoalShort *)(dst + 1);
     }
     // the level's counters and the goal pass's header set on the device (a copy from pageable host memory would
     // wait for the stream)
     k_level_init<<<1, 32, 0, s>>>(gsd, stats.as<DevStats>());
     launches++;
     if (goal_pass) {
-      uint32_t *glist = (uint32_t *)(gsd + 1);
+      uint32_t *glist = gshort.as<uint32_t>();
       const unsigned gm_ = (unsigned)std::max<long long>(1, std::min<long long>((m + 255) / 256, (long long)nsm * 8));
       k_goal_candidates<<<gm_, 256, 0, s>>>(fMeta.as<NodeMeta>(), m, glist, gsd);
       k_goal_level<NQ, ST><<<(unsigned)nsm * 2, EXP_WARPS * 32, 0, s>>>(sp, fR.as<Z4<ST>>(), fMeta.as<NodeMeta>(), glist,
@@ -2883,7 +2924,10 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       a.sh1 = sH1.as<uint64_t>(); a.sh2 = sH2.as<uint64_t>(); a.sidx = sIdx.as<uint64_t>();
       a.smeta = sMeta.as<NodeMeta>();
       a.tq = tq.as<TQEntry>(); a.tqcap = tqcap; a.gshort = gsd;
-      const long long want = (m + EXP_WARPS - 1) / EXP_WARPS;
+      // fewer parents than the chip has warps: up to 8 warps share a parent's candidates (a 2-qubit search's level kernels
+      // are then a chain of 3 children instead of 16; eight searches: 1.16 -> 0.75 ms of level kernels)
+      a.split = (int)std::max<long long>(1, std::min<long long>(8, (long long)nsm * EXP_MINB * EXP_WARPS / std::max<long long>(m, 1)));
+      const long long want = (m * a.split + EXP_WARPS - 1) / EXP_WARPS;
       const long long grid = std::max<long long>(1, std::min<long long>(want, (long long)nsm * EXP_MINB));   // one wave
       if (opt.profile) ck(cudaEventRecord(ev[0], s), "event");
       if (hs.states) k_expand<NQ, ST, true><<<(unsigned)grid, EXP_WARPS * 32, 0, s>>>(sp, a);
@@ -2902,10 +2946,11 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       expand_launches++;
       ck(cudaGetLastError(), "expand kernel");
       if (opt.profile) ck(cudaEventRecord(ev[1], s), "event");
-      ck(cudaMemcpyAsync(hstats, dst, sizeof(DevStats), cudaMemcpyDeviceToHost, s), "d2h");
-      d2h += sizeof(DevStats);
-      if (gsd) { ck(cudaMemcpyAsync(&hgs, gsd, sizeof hgs, cudaMemcpyDeviceToHost, s), "d2h"); d2h += sizeof hgs; }
+      const size_t back = sizeof(DevStats) + (gsd ? sizeof(GoalShort) : 0);
+      ck(cudaMemcpyAsync(hstats, dst, back, cudaMemcpyDeviceToHost, s), "d2h");
+      d2h += (long long)back;
       ck(cudaStreamSynchronize(s), "expand");
+      if (gsd) hgs = *(const GoalShort *)(hstats + 1);
       read_dedupe();
       if (gsd && hgs.found && !hgs.ovf && hgs.count <= GOAL_LIST) break;   // the found level (kernels skipped)
       if (opt.profile) { float ms = 0; cudaEventElapsedTime(&ms, ev[0], ev[1]); res.expand_ms += ms; }
@@ -2916,17 +2961,7 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
     }
     if (gsd && hgs.found && !hgs.ovf && hgs.count <= GOAL_LIST) {   // found by the goal pass
       const unsigned long long o = hgs.first;
-      std::vector<int> c(t);
-      c[t - 1] = (int)(o % G);
-      uint32_t i = (uint32_t)(o / G);
-      for (int l = t - 1; l >= 1; l--) {
-        uint8_t gg; uint32_t pp;
-        ck(cudaMemcpy(&gg, gat[l].as<uint8_t>() + i, 1, cudaMemcpyDeviceToHost), "d2h");
-        ck(cudaMemcpy(&pp, par[l].as<uint32_t>() + i, 4, cudaMemcpyDeviceToHost), "d2h");
-        c[l - 1] = gg; i = pp;
-        d2h += 5;
-      }
-      res.circuit = c;
+      res.circuit = walk_back(o, t);
       res.n_found = (long long)hgs.found;
       res.levels = t;
       return RC_CIRCUIT;
@@ -2944,17 +2979,7 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
     res.prefixes += L.prefixes;
     if (h.found) {                                     // the lexicographically first circuit of this level
       const unsigned long long o = h.first_found;
-      std::vector<int> c(t);
-      c[t - 1] = (int)(o % G);
-      uint32_t i = (uint32_t)(o / G);
-      for (int l = t - 1; l >= 1; l--) {
-        uint8_t gg; uint32_t pp;
-        ck(cudaMemcpy(&gg, gat[l].as<uint8_t>() + i, 1, cudaMemcpyDeviceToHost), "d2h");
-        ck(cudaMemcpy(&pp, par[l].as<uint32_t>() + i, 4, cudaMemcpyDeviceToHost), "d2h");
-        c[l - 1] = gg; i = pp;
-        d2h += 5;
-      }
-      res.circuit = c;
+      res.circuit = walk_back(o, t);
       res.n_found = (long long)h.found;
       res.levels = t;
       return RC_CIRCUIT;
@@ -2973,9 +2998,10 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
         work.ensure(ns * sizeof(uint2)); tmp.ensure(ns * 4);
         k_sort_init<<<gb, 256, 0, s>>>(sH1.as<uint64_t>(), ns, k0.as<uint64_t>(), v0.as<uint32_t>());
         launches++;
+        int nl = 0;
         const bool f = radix_sort(k0.as<uint64_t>(), v0.as<uint32_t>(), k1.as<uint64_t>(), v1.as<uint32_t>(), ns, 32,
-                                  64, sc, s, nullptr);
-        launches += 1 + 4;   // the sort: upsweep + one launch per 8-bit pass
+                                  64, sc, s, &nl);
+        launches += nl;
         const uint64_t *sk = f ? k1.as<uint64_t>() : k0.as<uint64_t>();
         const uint32_t *sv = f ? v1.as<uint32_t>() : v0.as<uint32_t>();
         k_runs<<<gb, 256, 0, s>>>(sk, sv, ns, sIdx.as<uint64_t>(), kidx.as<uint64_t>(), kslot.as<uint32_t>(),
@@ -3022,9 +3048,10 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       int bits = 1;
       while (bits < 64 && ((unsigned long long)m * G) >> bits) bits++;
       const int hi = ((bits + 7) / 8) * 8;
+      int nl2 = 0;
       const bool f2 = radix_sort(kidx.as<uint64_t>(), kslot.as<uint32_t>(), k1.as<uint64_t>(), v1.as<uint32_t>(),
-                                 (size_t)distinct, 0, hi, sc, s, nullptr);
-      if (distinct > 1) launches += 1 + hi / 8;
+                                 (size_t)distinct, 0, hi, sc, s, &nl2);
+      launches += nl2;
       const uint64_t *ki = f2 ? k1.as<uint64_t>() : kidx.as<uint64_t>();
       const uint32_t *vi = f2 ? v1.as<uint32_t>() : kslot.as<uint32_t>();
       if ((int)par.size() <= t) { par.resize(t + 1); gat.resize(t + 1); }
@@ -4287,8 +4314,13 @@ __global__ void k_bsort_init(const uint64_t *h1, const uint64_t *sidx, size_t n,
 }
 
 __global__ void k_bcount(const uint64_t *kidx, size_t nk, const uint32_t *fjob, unsigned long long *jdist) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nk; i += (size_t)gridDim.x * blockDim.x)
-    atomicAdd(&jdist[fjob[kidx[i] / BATCH_GS]], 1ULL);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nk; i += (size_t)gridDim.x * blockDim.x) {
+    // the indices are in order, so a warp's 32 are mostly one job's: one addition per job in the warp (2.6 -> 0.3 ms
+    // over a batch of 96 jobs)
+    const uint32_t job = fjob[kidx[i] / BATCH_GS];
+    const unsigned peers = __match_any_sync(__activemask(), job);
+    if ((int)(threadIdx.x & 31) == __ffs((int)peers) - 1) atomicAdd(&jdist[job], (unsigned long long)__popc(peers));
+  }
 }
 // circuits of jobs that found the goal: child o at step s, at job level t; walked back through the tree of steps
 // s - 1 .. s0 (the job's first step). A node carried over a step its job waited has gate 0xff there.
