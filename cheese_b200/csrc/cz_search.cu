@@ -1701,6 +1701,62 @@ __device__ __forceinline__ void warp_materialize(const Z4<ST> *R, const NodeMeta
   __syncwarp();
 }
 
+// child index o = parent * GS + gate: below 2^32 by one 32-bit division
+__device__ __forceinline__ unsigned long long child_parent(unsigned long long o, int GS, int &g) {
+  const unsigned long long p = (o >> 32) ? o / (unsigned long long)GS : (unsigned long long)((unsigned)o / (unsigned)GS);
+  g = (int)(o - p * (unsigned long long)GS);
+  return p;
+}
+// The lane's entries of a survivor's residual, straight from its parent Pg in global memory: unit monomials read the
+// permuted entry, one-qubit unit gates their column pair; any other gate goes through warp_child and shared memory (P, C).
+// x[j] is the entry at ei[j] (negative: none); every position is in one lane.
+template <int NQ, typename ST>
+__device__ __forceinline__ void child_entries(const Z4<ST> *Pg, int kp, int g, const DevSpec &sp, Z4<ST> *P, Z4<ST> *C, int lane,
+                                              Z4<ST> (&x)[2], int (&ei)[2]) {
+  constexpr int N = 1 << NQ, E = N * N;
+  ei[0] = ei[1] = -1;
+  x[0] = x[1] = Z4<ST>{0, 0, 0, 0};
+  if (sp.gflags[g] & GF_UNITMON) {
+    const int mono = sp.gmono[g][lane & (N - 1)];
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (lane + 32 * j < E) {
+        ei[j] = lane + 32 * j;
+        x[j] = mono_entry<NQ>(Pg, mono, lane, j);
+      }
+    return;
+  }
+  if constexpr (sizeof(ST) == 4) {
+    if (sp.gkind[g] == GK_ONEQ && kp <= 56) {
+      const int q = sp.gq[g][0], lo = (1 << q) - 1;
+      I4 v[2] = {I4{0, 0, 0, 0}, I4{0, 0, 0, 0}};
+      if (lane < E / 2) {
+        ei[0] = ((lane & ~lo) << 1) | (lane & lo);
+        ei[1] = ei[0] | (1 << q);
+        oneq_pair(Pg, ei, sp.gph[g], v);
+      }
+      (void)normalise_pair(v, kp + sp.gik[g]);
+#pragma unroll
+      for (int j = 0; j < 2; j++) x[j] = Z4<ST>{(ST)v[j].a, (ST)v[j].b, (ST)v[j].c, (ST)v[j].d};
+      return;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    if (lane + 32 * j < E) P[lane + 32 * j] = Pg[lane + 32 * j];
+  __syncwarp();
+  bool ovf;
+  (void)warp_child<NQ, ST>(P, C, g, kp, sp, &sp, lane, ovf);
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    if (lane + 32 * j < E) {
+      ei[j] = lane + 32 * j;
+      x[j] = C[lane + 32 * j];
+    }
+}
+
 // ---------------- deferred T bounds ----------------
 // One warp per queued entry: recompute the child from its parent, evaluate the T bound once for the entry's
 // children, finish their alive test, and write the survivors' records, as the level kernel would have. With jobs
@@ -1984,53 +2040,129 @@ __global__ void k_runs(const uint64_t *keys, const uint32_t *slots, size_t n, co
   }
 }
 
+// are A (the lane's entries av at positions ei) and B (in shared memory) one class: some group element maps A to B
 template <int NQ, typename ST>
-__device__ bool warp_same_class(const Z4<ST> *A, const Z4<ST> *B, const DevSpec &sp, const uint8_t (*perm)[8], int lane) {
-  constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1;
-  Z4<ST> av[EPL];
-#pragma unroll
-  for (int j = 0; j < EPL; j++) { const int e = lane + 32 * j; if (e < E) av[j] = A[e]; }
+__device__ __forceinline__ bool warp_same_entries(const Z4<ST> (&av)[2], const int (&ei)[2], const Z4<ST> *B, const DevSpec &sp,
+                                                  const uint8_t (*perm)[8]) {
+  constexpr int N = 1 << NQ;
   for (int s = 0; s < sp.nsym; s++) {
     bool eq = true;
 #pragma unroll
-    for (int j = 0; j < EPL; j++) {
-      const int e = lane + 32 * j;
-      if (e >= E) continue;
+    for (int j = 0; j < 2; j++) {
+      if (ei[j] < 0) continue;
       const Z4<ST> v = sp.symconj[s] ? zcj(av[j]) : av[j];
-      if (!zq(v, B[perm[s][e >> NQ] * N + perm[s][e & (N - 1)]])) eq = false;
+      if (!zq(v, B[perm[s][ei[j] >> NQ] * N + perm[s][ei[j] & (N - 1)]])) eq = false;
     }
     if (__all_sync(FULL, eq)) return true;
   }
   return false;
 }
+template <int NQ, typename ST>
+__device__ bool warp_same_class(const Z4<ST> *A, const Z4<ST> *B, const DevSpec &sp, const uint8_t (*perm)[8], int lane) {
+  constexpr int E = (1 << NQ) * (1 << NQ);
+  Z4<ST> av[2];
+  int ei[2];
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    ei[j] = lane + 32 * j < E ? lane + 32 * j : -1;
+    av[j] = ei[j] >= 0 ? A[ei[j]] : Z4<ST>{0, 0, 0, 0};
+  }
+  return warp_same_entries<NQ, ST>(av, ei, B, sp, perm);
+}
 
 constexpr int RES_WARPS = 4;       // warps per resolve / materialize block
+constexpr int RES_MINB = 8;        // resolve blocks per SM: 8 (64 registers) 2.7 ms, 6 3.8 ms, 5 3.6 ms (two budget 12 proofs)
 template <int NQ, typename ST> struct ResolveSmem {
   static constexpr int E = (1 << NQ) * (1 << NQ);
   Z4<ST> A[RES_WARPS][E], B[RES_WARPS][E], P[RES_WARPS][E];
+  uint8_t ord[RES_WARPS][32];
 };
 
 // one warp per run: order members by (h1, h2, index), then keep the first member of every exact class. With jobs
 // (fjob != nullptr) members of different jobs are never one class and each job's spec and symmetry group apply.
+// A run of up to 32 members (nearly all have two or three) is held one member per lane: ordered by shuffles, its kept
+// members a bit mask, written with one counter update. Longer runs order themselves in tmp. Bound by the latency of a
+// run's loads (members, then parents): the two budget 12 proofs' runs took 4.5 ms with every run ordered in memory and its
+// members rebuilt through shared memory, 2.7 ms so.
 template <int NQ, typename ST>
-__global__ void __launch_bounds__(RES_WARPS * 32) k_resolve(const DevSpec sp, const DevSpec *specs, const uint32_t *fjob,
-                                                          int GS, const Z4<ST> *R, const NodeMeta *meta,
-                                                          const uint2 *work, const uint32_t *slots, const uint64_t *sh1,
-                                                          const uint64_t *sh2, const uint64_t *sidx,
-                                                          const NodeMeta *smeta, uint32_t *tmp, uint64_t *kidx,
-                                                          uint32_t *kslot, DevStats *st) {
+__global__ void __launch_bounds__(RES_WARPS * 32, sizeof(ST) == 4 ? RES_MINB : 4) k_resolve(
+    const DevSpec sp, const DevSpec *specs, const uint32_t *fjob, int GS, const Z4<ST> *R, const NodeMeta *meta,
+    const uint2 *work, const uint32_t *slots, const uint64_t *sh1, const uint64_t *sh2, const uint64_t *sidx,
+    const NodeMeta *smeta, uint32_t *tmp, uint64_t *kidx, uint32_t *kslot, DevStats *st) {
+  constexpr int E = (1 << NQ) * (1 << NQ);
   __shared__ ResolveSmem<NQ, ST> sm;
   __shared__ DevSpec s_sp;
+  const unsigned long long nwork = st->n_work;
+  if ((unsigned long long)blockIdx.x * RES_WARPS >= nwork) return;
   if (!specs)
     for (int i = threadIdx.x; i < (int)(sizeof(DevSpec) / 4); i += blockDim.x) ((int *)&s_sp)[i] = ((const int *)&sp)[i];
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  Z4<ST> *A = sm.A[w], *B = sm.B[w], *P = sm.P[w];
-  const unsigned long long nwork = st->n_work;
+  Z4<ST> *B = sm.B[w], *P = sm.P[w], *C = sm.A[w];
   const unsigned long long nw = (unsigned long long)gridDim.x * RES_WARPS;
+  // the exact comparison of two survivors of one job (child indices oa and ob)
+  auto same = [&](uint64_t oa, uint64_t ob, uint32_t job) {
+    const DevSpec &jsp = specs ? specs[job] : s_sp;
+    int ga, gb;
+    const unsigned long long pa = child_parent(oa, GS, ga), pb = child_parent(ob, GS, gb);
+    Z4<ST> xa[2], xb[2];
+    int ea[2], eb[2];
+    child_entries<NQ, ST>(R + pa * E, meta[pa].k, ga, jsp, P, C, lane, xa, ea);
+    child_entries<NQ, ST>(R + pb * E, meta[pb].k, gb, jsp, P, C, lane, xb, eb);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+      if (eb[j] >= 0) B[eb[j]] = xb[j];
+    __syncwarp();
+    const bool r = warp_same_entries<NQ, ST>(xa, ea, B, jsp, jsp.symperm);
+    __syncwarp();
+    return r;
+  };
+  auto job_of = [&](uint64_t o) { int g; return fjob ? fjob[child_parent(o, GS, g)] : 0u; };
   for (unsigned long long wi = blockIdx.x * RES_WARPS + w; wi < nwork; wi += nw) {
     const uint2 wk = work[wi];
     const unsigned start = wk.x, len = wk.y;
+    if (len <= 32) {
+      uint32_t slot = 0, job = 0;
+      uint64_t h1 = 0, h2 = 0, idx = 0;
+      int k = 0;
+      if ((unsigned)lane < len) {
+        slot = slots[start + lane];
+        h1 = sh1[slot]; h2 = sh2[slot]; idx = sidx[slot];
+        k = smeta[slot].k;
+        job = job_of(idx);
+      }
+      int rank = 0;
+      for (int b = 0; b < (int)len; b++) {
+        const uint64_t bh1 = __shfl_sync(FULL, h1, b), bh2 = __shfl_sync(FULL, h2, b), bix = __shfl_sync(FULL, idx, b);
+        rank += (bh1 < h1) || (bh1 == h1 && (bh2 < h2 || (bh2 == h2 && bix < idx)));
+      }
+      __syncwarp();
+      if ((unsigned)lane < len) sm.ord[w][rank] = (uint8_t)lane;
+      __syncwarp();
+      unsigned kept = 0, group = 0;                    // by lane: kept members; kept members of the current key
+      for (unsigned i = 0; i < len; i++) {
+        const int li = sm.ord[w][i];
+        if (i > 0) {
+          const int lp = sm.ord[w][i - 1];
+          if (__shfl_sync(FULL, h1, lp) != __shfl_sync(FULL, h1, li) || __shfl_sync(FULL, h2, lp) != __shfl_sync(FULL, h2, li))
+            group = 0;
+        }
+        const int ki = __shfl_sync(FULL, k, li);
+        const uint32_t ji = __shfl_sync(FULL, job, li);
+        unsigned cand = group & __ballot_sync(FULL, k == ki && job == ji);
+        bool dup = false;
+        for (; cand && !dup; cand &= cand - 1)
+          dup = same(__shfl_sync(FULL, idx, li), __shfl_sync(FULL, idx, __ffs((int)cand) - 1), ji);
+        if (!dup) group |= 1u << li;
+        kept |= group & (1u << li);
+      }
+      unsigned long long pos = 0;
+      if (lane == 0) pos = atomicAdd(&st->n_kept, (unsigned long long)__popc(kept));
+      pos = __shfl_sync(FULL, pos, 0) + __popc(kept & ((1u << lane) - 1));
+      if ((kept >> lane) & 1) { kidx[pos] = idx; kslot[pos] = slot; }
+      continue;
+    }
     for (unsigned a0 = 0; a0 < len; a0 += 32) {          // rank of member a among the run
       const unsigned ai = a0 + lane;
       uint64_t ah1 = 0, ah2 = 0, aix = 0;
@@ -2052,18 +2184,15 @@ __global__ void __launch_bounds__(RES_WARPS * 32) k_resolve(const DevSpec sp, co
         const uint32_t sp0 = tmp[start + i - 1] & 0x7fffffffu;
         if (sh1[sp0] != sh1[si] || sh2[sp0] != sh2[si]) gstart = i;
       }
-      const uint32_t ji = fjob ? fjob[sidx[si] / (unsigned long long)GS] : 0;
-      const DevSpec &jsp = specs ? specs[ji] : s_sp;
-      bool dup = false, haveA = false;
+      const uint32_t ji = job_of(sidx[si]);
+      bool dup = false;
       for (unsigned i2 = gstart; i2 < i && !dup; i2++) {
         const uint32_t t2 = tmp[start + i2];
         if (!(t2 & 0x80000000u)) continue;
         const uint32_t s2 = t2 & 0x7fffffffu;
         if (smeta[s2].k != smeta[si].k) continue;
-        if (fjob && fjob[sidx[s2] / (unsigned long long)GS] != ji) continue;
-        if (!haveA) { warp_materialize<NQ, ST>(R, meta, sidx[si], GS, jsp, &jsp, P, A, lane); haveA = true; }
-        warp_materialize<NQ, ST>(R, meta, sidx[s2], GS, jsp, &jsp, P, B, lane);
-        dup = warp_same_class<NQ, ST>(A, B, jsp, jsp.symperm, lane);
+        if (fjob && job_of(sidx[s2]) != ji) continue;
+        dup = same(sidx[si], sidx[s2], ji);
       }
       if (!dup && lane == 0) {
         tmp[start + i] = si | 0x80000000u;
@@ -2084,38 +2213,43 @@ __global__ void k_keep_all(const uint64_t *sidx, size_t n, uint64_t *kidx, uint3
 }
 
 // kept survivors (in index order) -> the next frontier: residual recomputed from the parent, bounds, tree links
-// (and job ids, with jobs). One warp per kept child; consecutive warps mostly share a parent.
+// (and job ids, with jobs). One warp per kept child; consecutive warps mostly share a parent, whose entries come straight
+// from L2. Bound by the latency of the chain index -> parent -> entries, and by the 1 KB written per node (3 qubits): 2.6 M
+// nodes of two budget 12 proofs took 2.2 ms through shared memory, 1.3 ms so.
 template <int NQ, typename ST>
-__global__ void __launch_bounds__(RES_WARPS * 32) k_materialize(const DevSpec sp, const DevSpec *specs,
-                                                              const uint32_t *fjob, int GS, const Z4<ST> *R,
-                                                              const NodeMeta *meta, const uint64_t *kidx,
-                                                              const uint32_t *kslot, size_t nk, const NodeMeta *smeta,
-                                                              Z4<ST> *R2, NodeMeta *meta2, uint32_t *par,
-                                                              uint8_t *gat, uint32_t *fjob2) {
-  constexpr int E = (1 << NQ) * (1 << NQ), EPL = E >= 32 ? E / 32 : 1;
+__global__ void __launch_bounds__(RES_WARPS * 32, sizeof(ST) == 4 ? 8 : 4) k_materialize(
+    const DevSpec sp, const DevSpec *specs, const uint32_t *fjob, int GS, const Z4<ST> *R, const NodeMeta *meta,
+    const uint64_t *kidx, const uint32_t *kslot, size_t nk, const NodeMeta *smeta, Z4<ST> *R2, NodeMeta *meta2, uint32_t *par,
+    uint8_t *gat, uint32_t *fjob2) {
+  constexpr int E = (1 << NQ) * (1 << NQ);
   __shared__ Z4<ST> sP[RES_WARPS][E], sC[RES_WARPS][E];
   __shared__ DevSpec s_sp;
   if (!specs)
     for (int i = threadIdx.x; i < (int)(sizeof(DevSpec) / 4); i += blockDim.x) ((int *)&s_sp)[i] = ((const int *)&sp)[i];
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (size_t j = blockIdx.x * (size_t)RES_WARPS + w; j < nk; j += (size_t)gridDim.x * RES_WARPS) {
-    const unsigned long long o = kidx[j];
-    const unsigned long long p = o / (unsigned long long)GS;
+  const size_t step = (size_t)gridDim.x * RES_WARPS;
+  size_t j = blockIdx.x * (size_t)RES_WARPS + w;
+  unsigned long long o = j < nk ? kidx[j] : 0;
+  for (; j < nk; j += step) {
+    const unsigned long long on = j + step < nk ? kidx[j + step] : 0;   // the next child's index, loaded ahead
+    int g;
+    const unsigned long long p = child_parent(o, GS, g);
     const uint32_t job = fjob ? fjob[p] : 0;
     const DevSpec &jsp = specs ? specs[job] : s_sp;
-    warp_materialize<NQ, ST>(R, meta, o, GS, jsp, &jsp, sP[w], sC[w], lane);
+    Z4<ST> x[2];
+    int ei[2];
+    child_entries<NQ, ST>(R + p * E, meta[p].k, g, jsp, sP[w], sC[w], lane, x, ei);
 #pragma unroll
-    for (int q = 0; q < EPL; q++) {
-      const int e = lane + 32 * q;
-      if (e < E) R2[j * E + e] = sC[w][e];
-    }
+    for (int q = 0; q < 2; q++)
+      if (ei[q] >= 0) R2[j * E + ei[q]] = x[q];
     if (lane == 0) {
       meta2[j] = smeta[kslot[j]];
       par[j] = (uint32_t)p;
-      gat[j] = (uint8_t)(o % (unsigned long long)GS);
+      gat[j] = (uint8_t)g;
       if (fjob2) fjob2[j] = job;
     }
+    o = on;
   }
 }
 
