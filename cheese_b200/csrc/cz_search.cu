@@ -67,6 +67,7 @@ struct DevSpec {
   uint8_t gkind[GMAX];                 // GK_*: how the child update multiplies by the gate
   uint8_t gph[GMAX][4];                // one-qubit unit gates: w-power of ginv[m][lc] at [2 m + lc] (8: zero)
   uint8_t gmono[GMAX][8];              // GF_UNITMON gates: column c of S g^-1 is column src of S times w^p: src | p << 4
+  int cuts3;                           // 3 qubits and exactly the three one-qubit cuts
   uint8_t qcut[3];                     // per qubit: bit offset in NodeMeta.needs of the cut around it, QC_NONE if none
   uint8_t gperm[GMAX][8];              // permutation gates: local column lc takes local row gperm[lc]
   int goal_id;                         // the goal is the identity with exponent 0 (unitary targets)
@@ -516,6 +517,49 @@ template <int NQ, typename ST>
 __device__ __forceinline__ int warp_cx_bound(const Z4<ST> *S, const DevSpec &sp, int lane, int gmask, int needs_in,
                                              int &needs_out) {
   return warp_cx_elems<NQ>([&](int o, int i) { return to_fp(S[(o << NQ) + i], sp); }, sp, lane, gmask, needs_in, needs_out);
+}
+
+// The same for a two-qubit column permutation of a 3-qubit residual with one cut around each qubit (sp.cuts3): the two
+// crossed cuts side by side, one per half warp, from the parent's F_p image F with its columns permuted (mono: source column
+// per column). A need only tells ranks 1, 2 and 3 or more apart, so three of the four rows are eliminated first and the last
+// one only where they left a rank below 3 (rarely): 54 instead of 132 instructions.
+__device__ __forceinline__ int warp_cx_pair(const uint32_t *F, const uint8_t *mono, const DevSpec &sp, int lane, int q0, int q1,
+                                            int needs_in, int &needs_out) {
+  const int q = lane < 16 ? q0 : q1, col = lane & 15, lo = (1 << q) - 1;
+  auto wide = [&](int x) { return ((x & ~lo) << 1) | (x & lo); };      // a 0 inserted at bit q
+  const int i0 = wide(col & 3), o0 = wide(col >> 2) << 3, s0 = mono[i0] & 15, s1 = mono[i0 | (1 << q)] & 15, o1 = o0 | (8 << q);
+  uint32_t v[3] = {F[o0 + s0], F[o0 + s1], F[o1 + s0]}, w = F[o1 + s1];
+  const unsigned half = lane < 16 ? 0xffffu : 0xffff0000u;
+  uint32_t pa[3];
+  int pl[3], rank = 0;
+  bool used[3];
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const unsigned bal = __ballot_sync(FULL, v[r] != 0) & half;
+    used[r] = bal != 0;
+    pl[r] = bal ? __ffs(bal) - 1 : lane;
+    rank += used[r];
+    pa[r] = __shfl_sync(FULL, v[r], pl[r]);
+#pragma unroll
+    for (int r2 = r + 1; r2 < 3; r2++) {
+      const uint32_t b = __shfl_sync(FULL, v[r2], pl[r]);
+      if (used[r]) v[r2] = subp(mont(pa[r], v[r2]), mont(b, v[r]));
+    }
+  }
+  if (!__all_sync(FULL, rank == 3)) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const uint32_t b = __shfl_sync(FULL, w, pl[r]);
+      if (used[r]) w = subp(mont(pa[r], w), mont(b, v[r]));
+    }
+    rank += (__ballot_sync(FULL, w != 0) & half) != 0;
+  }
+  const int need = rank <= 1 ? 0 : (rank == 2 ? 1 : 2);
+  const int n0 = __shfl_sync(FULL, need, 0), n1 = __shfl_sync(FULL, need, 16), b0 = sp.qcut[q0], b1 = sp.qcut[q1];
+  const int needs = (needs_in & ~(3 << b0) & ~(3 << b1)) | n0 << b0 | n1 << b1;
+  needs_out = needs;
+  const int c0 = needs & 3, c1 = (needs >> 2) & 3, c2 = (needs >> 4) & 3, idx = c0 + 3 * c1 + 9 * c2;
+  return sp.have_table && idx < sp.ncx ? __ldg(&sp.cxtable[idx]) : max(c0, max(c1, c2));
 }
 
 // the least c + max(h + t, supp - 2 c) over c >= c2 (cheese.cu:599-607): the second term falls by 2 per step of c until
@@ -1102,8 +1146,8 @@ template <typename ST> struct ExpandOut {
 // one per lane, the odd diagonals queued one per lane. A two-qubit permutation (cx) changes only the ranks of the cuts it
 // crosses; they are eliminated straight from the parent's F_p image (computed once per parent) with its columns permuted.
 // Only survivors' entries are then formed, in registers, for the class key. Deep
-// proofs (budget 12, two targets, 2.74 M parents): both parts 19.9 -> 12.6 ms; bound by issue (80 %) and, for the one-qubit
-// part, by instruction fetch.
+// proofs (budget 12, two targets, 2.74 M parents): both parts 19.9 -> 12.6 ms, 10.5 ms with the ranks of warp_cx_pair; bound by
+// issue (80 %) and, for the one-qubit part, by instruction fetch.
 template <int NQ, typename ST, bool STATES = false, int PART = 0, typename Weight>
 __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *sps, Weight weight, unsigned conjmask,
                                               const Z4<ST> *P, Z4<ST> *C, uint32_t *F, unsigned long long p,
@@ -1229,7 +1273,8 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
       bool alive = true;
       if (!STATES && PART != 1 && kind == RANKS) {
         const uint8_t *mono = sps->gmono[g];
-        c2 = warp_cx_elems<NQ>([&](int r, int i) { return F[(r << NQ) + (mono[i] & 15)]; }, *sps, lane, gm, pm.needs, needs);
+        if (NQ == 3 && sps->cuts3) c2 = warp_cx_pair(F, mono, *sps, lane, gq0, sps->gq[g][1], pm.needs, needs);
+        else c2 = warp_cx_elems<NQ>([&](int r, int i) { return F[(r << NQ) + (mono[i] & 15)]; }, *sps, lane, gm, pm.needs, needs);
         ntriv = ntP | gm;
         if (!entangled(gq0, needs) || !entangled(sps->gq[g][1], needs)) kind = FULLC;   // one may have become trivial
         else alive = combine(max(kP, hsP), TP, c2, __popc(ntriv)) <= rem;
@@ -4017,6 +4062,8 @@ DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool no
     for (int i = 0; i < sp.ncuts && sp.ncuts <= 4; i++)
       if (q < NQ && sp.rad[i] > 1 && (sp.cutmask[i] == 1 << q || sp.cutmask[i] == (N - 1) - (1 << q))) sp.qcut[q] = (uint8_t)(2 * i);
   }
+  sp.cuts3 = NQ == 3 && sp.ncuts == 3 && sp.qcut[0] != QC_NONE && sp.qcut[1] != QC_NONE && sp.qcut[2] != QC_NONE &&
+             sp.rad[0] == 3 && sp.rad[1] == 3 && sp.rad[2] == 3;
   gi.assign((size_t)GMAX * 64, int4{0, 0, 0, 0});
   for (int g = 0; g < hs.G; g++)
     for (int i = 0; i < LMAX * LMAX; i++) {
