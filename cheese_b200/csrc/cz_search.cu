@@ -53,6 +53,8 @@ constexpr int INHERIT_KMAX = 60;
 enum GateKind : uint8_t { GK_GENERAL = 0, GK_ONEQ = 1, GK_PERM = 2 };   // the T bound is computed exactly (mod 2^32 / 2^64) only while 2(n + k) <= 128
 
 constexpr uint8_t QC_NONE = 0xff;
+// gcol: kind in the low 3 bits, qubit a in bits 3-4, qubit b in bits 5-6
+enum ColKind : uint8_t { COL_UNKNOWN = 0, COL_SAME = 1, COL_S = 2, COL_H = 3, COL_CX = 4 };
 
 // ---------------- device-side spec ----------------
 struct DevSpec {
@@ -67,6 +69,7 @@ struct DevSpec {
   uint8_t gkind[GMAX];                 // GK_*: how the child update multiplies by the gate
   uint8_t gph[GMAX][4];                // one-qubit unit gates: w-power of ginv[m][lc] at [2 m + lc] (8: zero)
   uint8_t gmono[GMAX][8];              // GF_UNITMON gates: column c of S g^-1 is column src of S times w^p: src | p << 4
+  uint8_t gcol[GMAX];                  // how a Clifford gate permutes the transfer matrix's columns: COL_* | qubit(s)
   int cuts3;                           // 3 qubits and exactly the three one-qubit cuts
   uint8_t qcut[3];                     // per qubit: bit offset in NodeMeta.needs of the cut around it, QC_NONE if none
   uint8_t gperm[GMAX][8];              // permutation gates: local column lc takes local row gperm[lc]
@@ -84,8 +87,10 @@ struct DevSpec {
 };
 
 // per frontier node: exponent, bounds carried to the children, last two gates (0xff: none), H structure (bit 0:
-// hs = 2) with the mask of qubits acted on non-trivially (bits 1..3), per-cut CX needs (2 bits per cut)
-struct NodeMeta { int16_t k; uint8_t T, c2, g1, g2, hsn, needs; };
+// hs = 2) with the mask of qubits acted on non-trivially (bits 1..3), per-cut CX needs (2 bits per cut), and the columns
+// of the Pauli transfer matrix with an entry of sde T (see cols_t_least; 0: not known)
+struct NodeMeta { int16_t k; uint8_t T, c2, g1, g2, hsn, needs; uint64_t cols; };
+static_assert(sizeof(NodeMeta) == 16, "node record");
 
 struct DevStats {
   unsigned long long w2, w3, dead, alive, found, first_found, n_surv, t_evals, children, work, full;
@@ -288,6 +293,54 @@ __device__ __forceinline__ int tbound_lanes(const Z4<ST> *S, int k, int lane) {
   const int top = 2 * (NQ + k);
   return top - v > 0 ? top - v : 0;
 }
+// ---- columns of the transfer matrix that reach the T bound (3 qubits) ----
+// (Of the T evaluations of the budget 12 proofs 86 % are decided from these 64 bits before they are queued.)
+// Column (zc, fc) belongs to the input Pauli with X part fc and Z part zc and is bit 8 zc + fc of a 64-bit mask. M holds the
+// columns with an entry of sde T. Right multiplication by a Clifford permutes columns, so M follows along. A T on qubit q
+// leaves the columns with fc_q = 0 and turns a pair (zc, zc ^ 1 << q) with fc_q = 1 into (u +- w) / sqrt2: where one of
+// the pair has an entry of sde T and the other none, u +- w has one of sde T and the child's bound is T + 1; and an entry
+// of sde T in an unchanged column keeps the child's bound at T or more.
+__device__ __forceinline__ uint64_t cols_x0(int q) {   // fc_q = 0
+  return q == 0 ? 0x5555555555555555ULL : (q == 1 ? 0x3333333333333333ULL : 0x0f0f0f0f0f0f0f0fULL);
+}
+__device__ __forceinline__ uint64_t cols_z0(int q) {   // zc_q = 0
+  return q == 0 ? 0x00ff00ff00ff00ffULL : (q == 1 ? 0x0000ffff0000ffffULL : 0x00000000ffffffffULL);
+}
+__device__ __forceinline__ uint64_t cols_flip_z(uint64_t M, int q) {   // zc -> zc ^ 1 << q
+  const uint64_t m = cols_z0(q);
+  return ((M & m) << (8 << q)) | ((M >> (8 << q)) & m);
+}
+// the least T bound of the child of an odd diagonal on qubit q
+__device__ __forceinline__ int cols_t_least(uint64_t M, int T, int q) {
+  if (!M) return T - 1;
+  const uint64_t x0 = cols_x0(q);
+  if ((M ^ cols_flip_z(M, q)) & ~x0) return T + 1;
+  return (M & x0) ? T : T - 1;
+}
+// the columns after right multiplication with a Clifford gate (gcol code)
+__device__ __forceinline__ uint64_t cols_after(uint64_t M, int code) {
+  const int a = (code >> 3) & 3, b = (code >> 5) & 3;
+  switch (code & 7) {
+    case COL_SAME: return M;
+    case COL_S: {                                        // X <-> Y on a
+      const uint64_t x0 = cols_x0(a);
+      return (M & x0) | (cols_flip_z(M, a) & ~x0);
+    }
+    case COL_H: {                                        // X <-> Z on a: bits a and 3 + a of the index exchanged
+      const int d = 7 << a;
+      const uint64_t x = ((M >> d) ^ M) & ~cols_x0(a) & cols_z0(a);
+      return M ^ x ^ (x << d);
+    }
+    case COL_CX: {                                       // control a, target b: fc_b ^= fc_a, zc_a ^= zc_b
+      const uint64_t fa = ~cols_x0(a), fb = cols_x0(b);
+      M = (M & ~fa) | ((M & fa & fb) << (1 << b)) | ((M & fa & ~fb) >> (1 << b));
+      const uint64_t zb = ~cols_z0(b), za = cols_z0(a);
+      return (M & ~zb) | ((M & zb & za) << (8 << a)) | ((M & zb & ~za) >> (8 << a));
+    }
+    default: return 0;
+  }
+}
+
 // ---- the same T bound for unitary residuals of small exponent, four components to a register ----
 // In a unitary residual (entries sqrt2^k U) sum |entry|^2 per row is 2^k in both embeddings of Z[sqrt2], so an entry's
 // coefficients satisfy a^2 + b^2 + c^2 + d^2 <= 2^k, and a transform output X_f(z) = 2^k N PTM(f, z) has |A| <= 2^(n +
@@ -309,13 +362,12 @@ template <typename ST> __device__ __forceinline__ int4 pack_entry(const Z4<ST> &
   return make_int4(pack4(a, b, c, d), pack4(-c, -d, a, b), pack4(b - d, a + c, b + d, c - a),
                    pack4(-b - d, a - c, b - d, a + c));
 }
-// OR of the output bytes of pair f (0 for f = 0); the point map as in tbound_round
+// The transform of pair f into v (0 for f = 0). Point map as in tbound_round, the inserted 0 at the lowest row bit of f if
+// it has one (then the column bits of e, and of the output index, are bits 0 to NQ - 1), else at its lowest column bit.
 template <int NQ, bool IDENT>
-__device__ __forceinline__ unsigned packed_round(const int4 *Y, const int *X, int f) {
-  constexpr int E = 1 << (2 * NQ), HP = E / 2;
-  if (f == 0) return 0;
-  const int lomask = IDENT ? E - 1 : ((f & HP) ? E - 1 : (f & -f) - 1);
-  int v[HP];
+__device__ __forceinline__ void packed_round(const int4 *Y, const int *X, int f, int (&v)[1 << (2 * NQ - 1)]) {
+  constexpr int E = 1 << (2 * NQ), HP = E / 2, ROWS = E - (1 << NQ);
+  const int fl = (f & ROWS) ? f & ROWS : f, lomask = IDENT ? E - 1 : ((f & HP) ? E - 1 : (fl & -fl) - 1);
 #pragma unroll
   for (int i = 0; i < HP; i++) {
     const int e = IDENT ? i : (i & lomask) | ((i & ~lomask) << 1);
@@ -336,10 +388,6 @@ __device__ __forceinline__ unsigned packed_round(const int4 *Y, const int *X, in
         v[i] = u + w;
         v[i | h] = u - w;
       }
-  int o = 0;
-#pragma unroll
-  for (int i = 0; i < HP; i++) o |= v[i];
-  return (unsigned)o;
 }
 // the bound from the OR words of the transform outputs: O1 = OR of 2A, X, alpha, beta, O2 = OR of 2A, alpha
 template <int NQ> __device__ __forceinline__ int bound_of(unsigned O1, unsigned O2, int k) {
@@ -355,44 +403,101 @@ __device__ __forceinline__ void unpack_or(unsigned o, unsigned &O1, unsigned &O2
 // T bound of the residual packed in Y and X (E words). At 3 qubits the 32 pairs f >= 32 come first: a bound above thr
 // already decides the entry (bounds only grow with further pairs); then the rest is left out and the result is a
 // lower bound above thr. On the deep proofs 92 % of the entries are dead and these 32 pairs show it for every one.
+// cols (3 qubits, when asked for): the columns with an entry of that sde. A lane's outputs of pair (fr, fc) belong to the
+// columns (zc, fc); their ORs by zc are joined over fr, and the bit that decides the bound is tested in each.
 template <int NQ>
-__device__ __forceinline__ int packed_tbound(const int4 *Y, const int *X, int k, int lane, int thr) {
-  constexpr int E = 1 << (2 * NQ), PL = E > 32 ? E / 32 : 1;
-  unsigned o = 0, O1, O2;
+__device__ __forceinline__ int packed_tbound(const int4 *Y, const int *X, int k, int lane, int thr, bool want_cols,
+                                             uint64_t &cols) {
+  constexpr int E = 1 << (2 * NQ), HP = E / 2, PL = E > 32 ? E / 32 : 1, ZC = 1 << NQ;
+  unsigned o = 0, O1, O2, oc[ZC];
+  int v[HP];
+  cols = 0;
+#pragma unroll
+  for (int z = 0; z < ZC; z++) oc[z] = 0;
   if constexpr (E == 64) {
-    o = __reduce_or_sync(FULL, packed_round<NQ, true>(Y, X, 32 + lane));
+    packed_round<NQ, true>(Y, X, 32 + lane, v);
+#pragma unroll
+    for (int i = 0; i < HP; i++) oc[i & 7] |= (unsigned)v[i];
+#pragma unroll
+    for (int z = 0; z < 8; z++) o |= oc[z];
+    o = __reduce_or_sync(FULL, o);
     unpack_or(o, O1, O2);
     const int T = bound_of<NQ>(O1, O2, k);
     if (T > thr) return T;
   }
-  o |= packed_round<NQ, false>(Y, X, lane < E ? lane : 0);
+  const int f = lane < E ? lane : 0;
+  packed_round<NQ, false>(Y, X, f, v);
+  unsigned o2 = 0;
+#pragma unroll
+  for (int i = 0; i < HP; i++) o2 |= (unsigned)v[i];
+  if (f) o |= o2;
+  if constexpr (E == 64) {
+    if (want_cols) {
+      if (lane >= 8) {                         // fr != 0: the output index keeps the column bits
+#pragma unroll
+        for (int i = 0; i < HP; i++) oc[i & 7] |= (unsigned)v[i];
+      } else if (lane) {
+        // fr = 0: the index lacks column bit j; of the two columns it stands for, the real components (bytes 0 and 2)
+        // belong to the one with even fc & zc, the imaginary ones to the other
+        const int j = __ffs(lane) - 1, lo = (1 << j) - 1;
+        unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < HP; i++) w[i & 3] |= (unsigned)v[i];
+#pragma unroll
+        for (int z = 0; z < 8; z++) {
+          const int t = ((z >> (j + 1)) << j) | (z & lo);
+          const unsigned wt = (t & 2) ? ((t & 1) ? w[3] : w[2]) : ((t & 1) ? w[1] : w[0]);
+          oc[z] |= wt & ((__popc(lane & z) & 1) ? 0xff00ff00u : 0x00ff00ffu);
+        }
+      }
+    }
+  }
   // f = 0: alpha + 2^16 beta over all E points across the warp (|alpha| <= 2^7, |beta| < 2^7)
-  int v[PL];
+  int q[PL];
 #pragma unroll
   for (int t = 0; t < PL; t++) {
     const int4 y = lane + 32 * t < E ? Y[lane + 32 * t] : make_int4(0, 0, 0, 0);
     // beta = ab + bc + cd - da: half of (a, b, c, d) . (b - d, a + c, b + d, c - a)
-    v[t] = __dp4a(y.x, y.x, 0) + ((__dp4a(y.x, y.z, 0) >> 1) << 16);
+    q[t] = __dp4a(y.x, y.x, 0) + ((__dp4a(y.x, y.z, 0) >> 1) << 16);
   }
 #pragma unroll
   for (int h = 1; h < PL; h <<= 1)
 #pragma unroll
     for (int t = 0; t < PL; t++)
-      if (!(t & h)) { const int u = v[t], w = v[t | h]; v[t] = u + w; v[t | h] = u - w; }
+      if (!(t & h)) { const int u = q[t], w = q[t | h]; q[t] = u + w; q[t | h] = u - w; }
   unsigned R = 0;
 #pragma unroll
   for (int t = 0; t < PL; t++) {
 #pragma unroll
     for (int h = 1; h < 32 && h < E; h <<= 1) {
-      const int u = __shfl_xor_sync(FULL, v[t], h);
-      v[t] = (lane & h) ? u - v[t] : u + v[t];
+      const int u = __shfl_xor_sync(FULL, q[t], h);
+      q[t] = (lane & h) ? u - q[t] : u + q[t];
     }
-    R |= (unsigned)(v[t] + 0x8000) ^ 0x8000u;
+    R |= (unsigned)(q[t] + 0x8000) ^ 0x8000u;
   }
   o = __reduce_or_sync(FULL, o);
-  R = __reduce_or_sync(FULL, R);
+  const unsigned Ra = __reduce_or_sync(FULL, R);
   unpack_or(o, O1, O2);
-  return bound_of<NQ>(O1 | (R & 0xffffu) | (R >> 16), O2 | (R & 0xffffu), k);
+  O1 |= (Ra & 0xffffu) | (Ra >> 16);
+  O2 |= Ra & 0xffffu;
+  if constexpr (E == 64) {
+    if (want_cols && O1) {
+      const int mv = __ffs((int)O1) - 1;
+      const bool even = (O2 >> mv) & 1;        // the least valuation is even: 2 A or alpha reaches it, else X or beta
+      const unsigned tm = even ? (mv ? 0x0101u << (mv - 1) : 0u) : 0x01010000u << mv;
+      R |= __shfl_xor_sync(FULL, R, 8);        // output z of f = 0 is in lane z mod 32: joined over the row bits
+      R |= __shfl_xor_sync(FULL, R, 16);
+      const unsigned z0 = __ballot_sync(FULL, ((even ? R : R >> 16) >> mv) & 1);
+      unsigned half[2] = {0, 0};
+#pragma unroll
+      for (int z = 0; z < 8; z++) {
+        const unsigned has = __ballot_sync(FULL, (oc[z] & tm) != 0);
+        half[z >> 2] |= (((has | has >> 8 | has >> 16 | has >> 24) & 0xffu) | ((z0 >> z) & 1u)) << (8 * (z & 3));
+      }
+      cols = half[0] | (uint64_t)half[1] << 32;
+    }
+  }
+  return bound_of<NQ>(O1, O2, k);
 }
 // 32-bit residues in one pass (3 qubits: 128 transform values per lane); 64-bit residues (k > 29, rare) one
 // component per pass
@@ -1213,7 +1318,7 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
         const bool oneq = fl & GF_ONEQ, ent = oneq && entangled(q0, pm.needs);
         int hlo = kP - ik;
         if ((fl & GF_MONAFF) && hsP > hlo) hlo = hsP;
-        const int tlo = (fl & GF_CLIFFORD) ? TP : ((fl & GF_TDIAG) ? TP - 1 : 0);
+        const int tlo = (fl & GF_CLIFFORD) ? TP : ((fl & GF_TDIAG) ? (NQ == 3 ? cols_t_least(pm.cols, TP, q0) : TP - 1) : 0);
         const int clo = oneq ? c2P : ((fl & GF_RANK2) ? c2P - 1 : 0);
         const int slo = ent ? suppP : suppP - sps->gnq[g];
         if (combine(max(hlo, 0), max(tlo, 0), max(clo, 0), max(slo, 0)) > rem) fate = DEADP;
@@ -1396,6 +1501,7 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
           nm.k = (int16_t)k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = (uint8_t)c2; nm.g1 = (uint8_t)g; nm.g2 = pm.g1;
           nm.hsn = (uint8_t)((hs == 2 ? 1 : 0) | (ntriv << 1));
           nm.needs = (uint8_t)needs;
+          nm.cols = NQ == 3 && (fl & GF_CLIFFORD) ? cols_after(pm.cols, sps->gcol[g]) : 0;   // (only Cliffords get here)
           o.smeta[slot] = nm;
         }
       } else if (lane == 0) {
@@ -1826,7 +1932,8 @@ template <typename ST> struct TBoundArgs {
 };
 // One block's warps walk the queue with a fixed stride. Bound by issue: a dead entry (most are) is the child's update,
 // its packing and one packed round. 3.96 M entries of two budget 12 proofs: 32.7 ms with 32-bit components, 11.7 ms
-// packed, 6.4 ms with the diagonal update in registers, the general form in a walk of its own and one alive test.
+// packed, 5.9 ms with the diagonal update in registers, the general form in a walk of its own and one alive test;
+// with the children that their parent's columns already decide (cols_t_least) left out, 0.57 M entries in 2.4 ms.
 template <int NQ, typename ST, bool BATCHED = false>
 __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
     k_tbound(const __grid_constant__ DevSpec sp0, const TBoundArgs<ST> a) {
@@ -1934,6 +2041,7 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
       }
       bool ovf;
       int T = 0;
+      uint64_t cols = 0;
       if (mine) neval++;
       if constexpr (GENERAL) {
         if (mine) {
@@ -1950,7 +2058,8 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
             sX[w][lane + 32 * j] = y.x;
           }
         __syncwarp();
-        T = packed_tbound<NQ>(sY[w], sX[w], q.k, lane, max(thr[0], thr[1]));   // T <= 2 (NQ + k) < 31: thr is exact
+        T = packed_tbound<NQ>(sY[w], sX[w], q.k, lane, max(thr[0], thr[1]), keep && NQ == 3, cols);   // T <= 2 (NQ + k) < 31:
+                                                                                            // thr is exact
       }
       for (int s2 = 0; s2 < mine; s2++) {
         const bool alive = T < 31 ? T <= thr[s2]
@@ -1982,6 +2091,11 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
             nm.k = q.k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = q.c2; nm.g1 = q.g[s2]; nm.g2 = pm.g1;
             nm.hsn = (uint8_t)((q.hs == 2 ? 1 : 0) | (q.ntriv[s2] << 1));
             nm.needs = q.needs;
+            nm.cols = cols;
+            if (s2 && cols) {                        // the sibling differs by a power of S: an odd one exchanges X and Y
+              const uint8_t *a0 = sp.gph[q.g[0]], *a1 = sp.gph[q.g[1]];
+              if ((a0[3] - a0[0] - a1[3] + a1[0]) & 3) nm.cols = cols_after(cols, COL_S | sp.gq[q.g[0]][0] << 3);
+            }
             a.smeta[slot] = nm;
           }
         } else if (lane == 0) {
@@ -2016,12 +2130,13 @@ template <int NQ, typename ST> __global__ void k_root(const DevSpec sp, const Z4
   for (int e = lane; e < E; e += 32) S[e] = R[e];
   __syncwarp();
   int T = 0, c2 = 0, needs = 0;
+  uint64_t cols = 0;
   Cheap ch{false, 0, 0};
   if (sp.standard || sp.lite) {
     if (sp.unit && NQ + tk <= PACK_MAX) {
       for (int e = lane; e < E; e += 32) { Y[e] = pack_entry(S[e]); X[e] = Y[e].x; }
       __syncwarp();
-      T = packed_tbound<NQ>(Y, X, tk, lane, INT_MAX);
+      T = packed_tbound<NQ>(Y, X, tk, lane, INT_MAX, NQ == 3, cols);
     } else {
       T = ptm_bound<NQ, ST>(S, tk, lane);
     }
@@ -2035,6 +2150,7 @@ template <int NQ, typename ST> __global__ void k_root(const DevSpec sp, const Z4
     m.k = (int16_t)tk; m.T = (uint8_t)(T > 255 ? 255 : T); m.c2 = (uint8_t)c2; m.g1 = m.g2 = 0xff;
     m.hsn = (uint8_t)((ch.hs == 2 ? 1 : 0) | (ch.ntriv << 1));
     m.needs = (uint8_t)needs;
+    m.cols = cols;
     *meta = m;
   }
 }
@@ -3058,11 +3174,11 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
     // every child); when more survive, the level is redone once with the exact count (the kernel counts every
     // survivor, stored or not)
     size_t lim_bytes = (size_t)8 << 30;         // above 8 GiB of records, up to 40 % of the free device memory
-    if (keep && 1.5 * surv_rate * (double)m * G * 40.0 > (double)lim_bytes) {
+    if (keep && 1.5 * surv_rate * (double)m * G * 48.0 > (double)lim_bytes) {
       size_t fr = 0, tot = 0;
       if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) lim_bytes = std::max(lim_bytes, (size_t)(0.4 * (double)fr));
     }
-    unsigned long long cap = keep ? survivor_room((unsigned long long)m * G, surv_rate, 40, lim_bytes) : 0;
+    unsigned long long cap = keep ? survivor_room((unsigned long long)m * G, surv_rate, 48, lim_bytes) : 0;
     DevStats *dst = stats.as<DevStats>();
     // deferred T evaluations: at most one entry per child of a gate whose T bound is not inherited
     int ncl = 0;
@@ -4057,6 +4173,23 @@ DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool no
     }
     if (ok) sp.gflags[g] |= GF_UNITMON;
   }
+  for (int g = 0; g < hs.G; g++) {      // the Cliffords whose action on the Paulis is one of the simple ones
+    sp.gcol[g] = COL_UNKNOWN;
+    if (!(hs.gflags[g] & GF_CLIFFORD) || hs.states) continue;
+    const int q = hs.gq[g][0];
+    if (sp.gkind[g] == GK_ONEQ) {
+      const int p00 = sp.gph[g][0], p01 = sp.gph[g][1], p10 = sp.gph[g][2], p11 = sp.gph[g][3];
+      if (p00 < 8 && p11 < 8 && p01 == 8 && p10 == 8) sp.gcol[g] = (uint8_t)((((p11 - p00) & 3) == 0 ? COL_SAME : COL_S) | q << 3);
+      else if (p00 == 8 && p11 == 8 && p01 < 8 && p10 < 8) sp.gcol[g] = (uint8_t)((((p10 - p01) & 3) == 0 ? COL_SAME : COL_S) | q << 3);
+      else if (p00 < 8 && p01 == p00 && p10 == p00 && p11 == ((p00 + 4) & 7)) sp.gcol[g] = (uint8_t)(COL_H | q << 3);
+    } else if (sp.gkind[g] == GK_PERM && hs.gnq[g] == 2) {
+      for (int c = 0; c < 2; c++) {      // local control c, target 1 - c
+        bool cx = true;
+        for (int l = 0; l < 4; l++) cx = cx && sp.gperm[g][l] == (l ^ (((l >> c) & 1) << (1 - c)));
+        if (cx) sp.gcol[g] = (uint8_t)(COL_CX | hs.gq[g][c] << 3 | hs.gq[g][1 - c] << 5);
+      }
+    }
+  }
   for (int q = 0; q < 3; q++) {
     sp.qcut[q] = QC_NONE;
     for (int i = 0; i < sp.ncuts && sp.ncuts <= 4; i++)
@@ -4466,6 +4599,7 @@ __global__ void k_root_batch(const DevSpec *specs, const uint32_t *rjob, const i
     m.k = (int16_t)tk; m.T = (uint8_t)(T > 255 ? 255 : T); m.c2 = (uint8_t)c2; m.g1 = m.g2 = 0xff;
     m.hsn = (uint8_t)((ch.hs == 2 ? 1 : 0) | (ch.ntriv << 1));
     m.needs = (uint8_t)needs;
+    m.cols = 0;
     meta[i] = m;
   }
 }
@@ -4657,7 +4791,7 @@ struct BatchImpl : BatchSession::Impl {
 
   // device bytes of a frontier node with its tree entry, and of a survivor record with its dedupe sort entries
   static constexpr size_t NODE_BYTES = E * sizeof(Z4<ST>) + sizeof(NodeMeta) + 4 + 5;
-  static constexpr size_t SURV_BYTES = 40 + 48;
+  static constexpr size_t SURV_BYTES = 48 + 48;
   static constexpr unsigned long long SOLO_CHILDREN = 1ull << 22;
   // expected nodes of the job's next frontier: its children at the previous level's survivor and distinct rates,
   // with a quarter more survivors and 1024 nodes to spare (every child at the first level)
