@@ -3046,6 +3046,7 @@ struct Engine::Impl {
   bool lean_level = false;                 // the last level of a levels() call keeps its tree and keys, not its
                                            // residuals (the last searched level of --table K)                  // keep the frontier's class keys (fK1, fK2)
   DBuf fK1, fK2, tptrs, keys2, old;
+  DBuf outb;                               // a table candidate's symmetry elements and residual
   DevStats *hstats = nullptr;              // pinned
   long long launches = 0, expand_launches = 0, h2d = 0, d2h = 0;
   long long front_m = 1;                   // nodes in the current frontier
@@ -3080,7 +3081,7 @@ struct Engine::Impl {
   size_t trim() {
     size_t n = 0;
     for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &k0, &k1, &v0, &v1, &hist, &part,
-                    &work, &tmp, &kidx, &kslot, &fK1, &fK2, &keys2, &old, &gshort}) {
+                    &work, &tmp, &kidx, &kslot, &fK1, &fK2, &keys2, &old, &gshort, &outb}) {
       n += b->cap;
       b->release();
     }
@@ -3097,7 +3098,7 @@ struct Engine::Impl {
       b->release();
     for (auto &sd : specs) sd.release();
     for (auto &kv : dtabs) { kv.second->release(); delete kv.second; }
-    for (DBuf *b : {&fK1, &fK2, &tptrs, &keys2, &old, &gshort}) b->release();
+    for (DBuf *b : {&fK1, &fK2, &tptrs, &keys2, &old, &gshort, &outb}) b->release();
     for (auto &b : par) b.release();
     for (auto &b : gat) b.release();
     side.release();
@@ -3793,7 +3794,6 @@ int Engine::Impl::run_table(const HostSpec &hs, const Options &opt, const std::f
     }
     std::sort(cand.begin(), cand.end());
     const void *const *tp = upload_tree(D->par, D->gat, D->nl);
-    DBuf outb;
     outb.ensure(64 * sizeof(int2) + 16 + E * sizeof(Z4<int32_t>) + 16);
     Z4<int32_t> *cres = (Z4<int32_t> *)((char *)outb.p + 64 * sizeof(int2) + 16);
     for (const auto &cd : cand) {
