@@ -96,7 +96,7 @@ struct DevStats {
   unsigned long long w2, w3, dead, alive, found, first_found, n_surv, t_evals, children, work, full;
   unsigned int ovf, surv_overflow;
   unsigned long long n_work, n_kept;
-  unsigned long long n_tq, tq_work;   // deferred T evaluations: queued, taken
+  unsigned long long n_tq;            // deferred T evaluations queued
   unsigned int sort_err, pad;         // a dedupe sort's look-back gave up (its result is not used)
   unsigned long long work2;           // parent counter of the level kernel's second part (multi-qubit gates)
 };

@@ -6,12 +6,12 @@
 // (:258-276, 368-390). The search peels rotations off U level by level and looks every node up in the table; the
 // first level with a hit gives the optimum, the node with the smallest table level wins (:497-529).
 //
-// B200 design: one 256-thread CTA per parent holds the parent's 64 x 64 matrix (x and y limbs, int32) in shared
-// memory and derives all 63 children from it (the reference replays the whole path for every child); the coset
-// key is a sum over columns of a hash of the sign-normalised column (invariant under signed column permutations,
-// i.e. right Cliffords) computed with per-column shared-memory atomics; equality of cosets is the exact multiset
-// comparison of sign-normalised columns. Dedupe reuses the radix sort of the gate-count search. Tables stay
-// resident in HBM for the engine's lifetime.
+// B200 design: a 256-thread CTA holds a parent's 64 x 64 matrix (x and y limbs, int32) in shared memory and each of its
+// warps derives children from it, one at a time (the reference replays the whole path for every child); the coset key
+// is a sum over columns of a hash of the sign-normalised column (invariant under signed column permutations, i.e. right
+// Cliffords); equality of cosets is the exact multiset comparison of sign-normalised columns, by warps over columns in
+// the order of their hashes. Dedupe reuses the radix sort of the gate-count search. Tables stay resident in HBM for the
+// engine's lifetime.
 #include <cuda_runtime.h>
 
 #include <algorithm>
