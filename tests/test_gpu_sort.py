@@ -54,3 +54,22 @@ def test_sort_refuses_partial_bytes(engine):
     v = torch.zeros(4, dtype=torch.int32, device="cuda")
     with pytest.raises(RuntimeError):
         engine.sort_pairs(k.data_ptr(), v.data_ptr(), 4, 0, 12)
+
+
+@pytest.mark.parametrize("lo,hi", [(32, 64), (0, 8), (0, 64), (24, 64)])
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 1023, 1025, 8191, 8192, 8193, 8193 + 2048])
+def test_counted_and_digit_sorts_meet(engine, n, lo, hi):
+    """sorts of up to 8192 pairs are placed by counting, larger ones by digit passes: block and tile edges on both
+    sides, 32-bit and 64-bit digits, half of the keys equal"""
+    import torch
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(7 * n + lo + hi)
+    keys = torch.randint(-(1 << 62), 1 << 62, (n,), dtype=torch.int64, device=dev, generator=g) * 2
+    keys[::2] = keys[0].clone()
+    vals = torch.arange(n, dtype=torch.int32, device=dev)
+    want_k, want_v = stable_reference(keys, vals, lo, hi)
+    torch.cuda.synchronize()
+    engine.sort_pairs(keys.data_ptr(), vals.data_ptr(), n, lo, hi)
+    torch.cuda.synchronize()
+    assert torch.equal(vals, want_v)
+    assert torch.equal(keys, want_k)
