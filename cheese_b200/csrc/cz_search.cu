@@ -3489,8 +3489,8 @@ constexpr uint32_t DT_KEY_VERSION = 2;   // 2: 32-bit weighted sums per orbit el
 // the goal (the identity, exponent 0)
 bool host_circuit_ok(const HostSpec &hs, const std::vector<int> &c) {
   const int n = hs.n, N = 1 << n;
-  std::vector<Zw> S(hs.target.begin(), hs.target.end()), T(N * N);
-  int k = hs.tk;
+  std::vector<Zw> S(hs.root.begin(), hs.root.end()), T(N * N);
+  int k = hs.rk;
   for (int g : c) {
     const int nq = hs.gnq[g], L = 1 << nq;
     int mask = 0;
@@ -3644,7 +3644,8 @@ Engine::Impl::DistTable *Engine::Impl::get_table(const HostSpec &hs, const SymGr
   HostSpec hI = hs;                                   // the identity as target, no bounds, never "found"
   hI.target.assign(E, Zw{0, 0, 0, 0});
   for (int i = 0; i < N; i++) hI.target[i * N + i] = Zw{1, 0, 0, 0};
-  hI.tk = 0; hI.standard = 0; hI.lite = 0; hI.uid = hs.uid ^ 0x7461626c65ULL;
+  hI.root = hI.target;
+  hI.tk = hI.rk = 0; hI.standard = 0; hI.lite = 0; hI.uid = hs.uid ^ 0x7461626c65ULL;
   const DevSpec sp = prepare<NQ>(hI, grp, K + 1, true);
   DistTable *D = new DistTable;
   if (table_load(path, *D, K, hs.G)) {
@@ -3746,10 +3747,10 @@ int Engine::Impl::run_table(const HostSpec &hs, const Options &opt, const std::f
   const DevSpec sp = prepare<NQ>(hs, grp, depth, false);
   {
     std::vector<Z4<int32_t>> t32(E);
-    for (int i = 0; i < E; i++) t32[i] = {(int32_t)hs.target[i].a, (int32_t)hs.target[i].b, (int32_t)hs.target[i].c, (int32_t)hs.target[i].d};
+    for (int i = 0; i < E; i++) t32[i] = {(int32_t)hs.root[i].a, (int32_t)hs.root[i].b, (int32_t)hs.root[i].c, (int32_t)hs.root[i].d};
     fR.ensure(E * sizeof(Z4<int32_t>)); fMeta.ensure(sizeof(NodeMeta));
     ck(cudaMemcpyAsync(fR.p, t32.data(), E * sizeof(Z4<int32_t>), cudaMemcpyHostToDevice, s), "h2d");
-    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.tk);
+    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.rk);
     launches++;
     table_levels_keys<NQ>(sp, 1);
     ck(cudaStreamSynchronize(s), "root");
@@ -3908,9 +3909,9 @@ int Engine::Impl::run_mitm(const HostSpec &hs, const Options &opt, const std::fu
   std::vector<Z4<int32_t>> hU(E), hUd(E);
   for (int r = 0; r < N; r++)
     for (int c = 0; c < N; c++) {
-      const Zw x = hs.target[r * N + c];
+      const Zw x = hs.root[r * N + c];
       hU[r * N + c] = {(int32_t)x.a, (int32_t)x.b, (int32_t)x.c, (int32_t)x.d};
-      const Zw t = hs.target[c * N + r];                // U^dag (conjugate transpose), same sqrt2 exponent
+      const Zw t = hs.root[c * N + r];                  // U^dag (conjugate transpose), same sqrt2 exponent
       const Zw y{t.a, -t.d, -t.c, -t.b};
       hUd[r * N + c] = {(int32_t)y.a, (int32_t)y.b, (int32_t)y.c, (int32_t)y.d};
     }
@@ -3923,7 +3924,7 @@ int Engine::Impl::run_mitm(const HostSpec &hs, const Options &opt, const std::fu
   auto root = [&](const Z4<int32_t> *M) {              // the current tree restarts at M
     fR.ensure(E * sizeof(Z4<int32_t>)); fMeta.ensure(sizeof(NodeMeta));
     ck(cudaMemcpyAsync(fR.p, M, E * sizeof(Z4<int32_t>), cudaMemcpyDeviceToDevice, s), "d2d");
-    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.tk);
+    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.rk);
     launches++;
     ck(cudaGetLastError(), "root kernel");
     front_m = 1;
@@ -3998,7 +3999,7 @@ int Engine::Impl::run_mitm(const HostSpec &hs, const Options &opt, const std::fu
   B1.ensure(nb * 8); B2.ensure(nb * 8); flags.ensure(16);
   ck(cudaMemsetAsync(flags.p, 0, 16, s), "memset");
   const unsigned gw = (unsigned)std::max<long long>(1, std::min<long long>((nb + RES_WARPS - 1) / RES_WARPS, (long long)nsm * 16));
-  k_mitm_bwd_keys<NQ><<<gw, RES_WARPS * 32, 0, s>>>(sp, U, Ud, hs.tk, lv, (const uint32_t *const *)tp,
+  k_mitm_bwd_keys<NQ><<<gw, RES_WARPS * 32, 0, s>>>(sp, U, Ud, hs.rk, lv, (const uint32_t *const *)tp,
                                                     (const uint8_t *const *)(tp + b + 1), nb, B1.as<uint64_t>(),
                                                     B2.as<uint64_t>(), flags.as<int>());
   launches++;
@@ -4036,7 +4037,7 @@ int Engine::Impl::run_mitm(const HostSpec &hs, const Options &opt, const std::fu
     DBuf mb;
     mb.ensure(nh * 8);
     const unsigned gc = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((nh + RES_WARPS - 1) / RES_WARPS, (unsigned long long)nsm * 16));
-    k_mitm_confirm<NQ><<<gc, RES_WARPS * 32, 0, s>>>(sp, U, Ud, hs.tk, lv, (const uint32_t *const *)tp,
+    k_mitm_confirm<NQ><<<gc, RES_WARPS * 32, 0, s>>>(sp, U, Ud, hs.rk, lv, (const uint32_t *const *)tp,
                                                      (const uint8_t *const *)(tp + b + 1), hits.as<long long>(),
                                                      (long long)nh, pos.as<long long>(), S1.as<uint64_t>(),
                                                      S2.as<uint64_t>(), Si.as<uint32_t>(), nf, fR.as<Z4<int32_t>>(),
@@ -4209,7 +4210,7 @@ DevSpec devspec_host(const HostSpec &hs, const SymGroup &grp, int depth, bool no
       gl[2 * (r * N + c)] = make_longlong2(r == c ? 1 : 0, 0);
       gl[2 * (r * N + c) + 1] = make_longlong2(0, 0);
     }
-  sp.unit = !hs.states && unitary(hs.target.data(), N, hs.tk);
+  sp.unit = !hs.states && unitary(hs.root.data(), N, hs.rk);
   for (int g = 0; g < hs.G; g++) sp.unit = sp.unit && unitary(hs.ginv[g].data(), 1 << hs.gnq[g], hs.gik[g]);
   sp.states = hs.states;
   sp.m = hs.states ? hs.m : N;
@@ -4285,16 +4286,16 @@ int Engine::Impl::run(const HostSpec &hs, const Options &opt, const std::functio
   fMeta.ensure(sizeof(NodeMeta));
   if (!wide) {
     std::vector<Z4<int32_t>> t32(E);
-    for (int i = 0; i < E; i++) t32[i] = {(int32_t)hs.target[i].a, (int32_t)hs.target[i].b, (int32_t)hs.target[i].c, (int32_t)hs.target[i].d};
+    for (int i = 0; i < E; i++) t32[i] = {(int32_t)hs.root[i].a, (int32_t)hs.root[i].b, (int32_t)hs.root[i].c, (int32_t)hs.root[i].d};
     fR.ensure(E * sizeof(Z4<int32_t>));
     ck(cudaMemcpyAsync(fR.p, t32.data(), E * sizeof(Z4<int32_t>), cudaMemcpyHostToDevice, s), "h2d");
     h2d += E * sizeof(Z4<int32_t>);
-    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.tk);
+    k_root<NQ, int32_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int32_t>>(), fMeta.as<NodeMeta>(), hs.rk);
   } else {
     fR.ensure(E * sizeof(Z4<int64_t>));
-    ck(cudaMemcpyAsync(fR.p, hs.target.data(), E * sizeof(Zw), cudaMemcpyHostToDevice, s), "h2d");
+    ck(cudaMemcpyAsync(fR.p, hs.root.data(), E * sizeof(Zw), cudaMemcpyHostToDevice, s), "h2d");
     h2d += E * sizeof(Zw);
-    k_root<NQ, int64_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int64_t>>(), fMeta.as<NodeMeta>(), hs.tk);
+    k_root<NQ, int64_t><<<1, 32, 0, s>>>(sp, fR.as<Z4<int64_t>>(), fMeta.as<NodeMeta>(), hs.rk);
   }
   launches++;
   ck(cudaGetLastError(), "root kernel");
@@ -4943,10 +4944,10 @@ struct BatchImpl : BatchSession::Impl {
     for (size_t i = 0; i < roots.size(); i++) {
       Job &j = J[roots[i]];
       for (int e = 0; e < E; e++)
-        rr[i * E + e] = {(int32_t)j.hs.target[e].a, (int32_t)j.hs.target[e].b, (int32_t)j.hs.target[e].c,
-                         (int32_t)j.hs.target[e].d};
+        rr[i * E + e] = {(int32_t)j.hs.root[e].a, (int32_t)j.hs.root[e].b, (int32_t)j.hs.root[e].c,
+                         (int32_t)j.hs.root[e].d};
       rjk[i] = (uint32_t)roots[i];
-      rjk[roots.size() + i] = (uint32_t)j.hs.tk;
+      rjk[roots.size() + i] = (uint32_t)j.hs.rk;
       sps[roots[i] - qlo] = j.sp;
       j.t = 1;
       j.seg = 1;

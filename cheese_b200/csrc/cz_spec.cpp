@@ -255,6 +255,19 @@ int parse_spec(const char *text, size_t len, HostSpec &s, std::string &err) {
   if (s.n < 1 || s.n > NQMAX) { err = "n = " + std::to_string(s.n) + " not built"; return RC_USAGE; }
   const int N = 1 << s.n;
   if ((int)s.target.size() != N * N) { s.target.assign(N * N, Zw{0, 0, 0, 0}); }
+  s.root = s.target;
+  s.rk = s.tk;
+  // (a zero matrix is left alone, and one whose coefficients are so large that the differences could overflow)
+  constexpr int64_t LIM = (int64_t)1 << 61;
+  const bool plain = std::any_of(s.root.begin(), s.root.end(), [](const Zw &z) { return !zzero(z); }) &&
+                     std::all_of(s.root.begin(), s.root.end(), [&](const Zw &z) {
+                       return std::max(std::max(z.a, z.b), std::max(z.c, z.d)) < LIM &&
+                              std::min(std::min(z.a, z.b), std::min(z.c, z.d)) > -LIM;
+                     });
+  while (plain && s.rk > 0 && std::all_of(s.root.begin(), s.root.end(), zdiv2ok)) {
+    for (Zw &z : s.root) z = zdown(z);
+    s.rk--;
+  }
   if (s.bad2.empty()) s.bad2.assign((size_t)s.G * s.G, 0);
   if (s.bad3.empty()) s.bad3.assign(((size_t)s.G * s.G * s.G + 31) / 32, 0);
   // the window tables are indexed by candidate on the device: their sizes must be those of the final gate list
