@@ -29,6 +29,7 @@
 #include <map>
 #include <stdexcept>
 
+#include "cz_buf.h"
 #include "cz_clifford.h"
 #include "cz_sort.cuh"
 #include "cz_tableau.h"
@@ -79,20 +80,16 @@ void clk(cudaError_t e, const char *what) {
 }
 double cl_now() { return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count(); }
 
-struct CBuf {
-  void *p = nullptr;
-  size_t cap = 0;
-  void ensure(size_t b) {
-    if (b <= cap) return;
-    if (p) clk(cudaFree(p), "free");
-    size_t c = std::max(b, cap + cap / 2);
-    c = (c + 255) & ~(size_t)255;
-    clk(cudaMalloc(&p, c), "cudaMalloc");
-    cap = c;
+struct ClMemory {
+  static void *get(size_t n) {
+    void *p = nullptr;
+    clk(cudaMalloc(&p, n), "cudaMalloc");
+    return p;
   }
-  template <typename T> T *as() const { return (T *)p; }
-  void release() { if (p) cudaFree(p); p = nullptr; cap = 0; }
+  static void put(void *p) { clk(cudaFree(p), "free"); }
+  static void drop(void *p) { cudaFree(p); }
 };
+using CBuf = GrowBuf<ClMemory>;
 
 // ---------------- kernels ----------------
 // The group is the symplectic parts S (1,451,520 at n = 3) times the 4^n sign vectors, and rank = 4^n rank(S) + signs.

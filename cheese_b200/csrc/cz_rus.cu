@@ -23,6 +23,7 @@
 #include <map>
 #include <stdexcept>
 
+#include "cz_buf.h"
 #include "cz_rus.h"
 #include "cz_rus_node.h"
 #include "cz_sort.cuh"
@@ -172,20 +173,16 @@ void rck(cudaError_t e, const char *what) {
     throw RusCudaError(std::string("CUDA error after ") + what + ": " + cudaGetErrorString(e));
   }
 }
-struct Buf {
-  void *p = nullptr;
-  size_t cap = 0;
-  void ensure(size_t b) {
-    if (b <= cap) return;
-    if (p) rck(cudaFree(p), "free");
-    size_t c = std::max(b, cap + cap / 2);
-    c = (c + 255) & ~(size_t)255;
-    rck(cudaMalloc(&p, c), "cudaMalloc");
-    cap = c;
+struct RusMemory {
+  static void *get(size_t n) {
+    void *p = nullptr;
+    rck(cudaMalloc(&p, n), "cudaMalloc");
+    return p;
   }
-  template <typename T> T *as() const { return (T *)p; }
-  void release() { if (p) cudaFree(p); p = nullptr; cap = 0; }
+  static void put(void *p) { rck(cudaFree(p), "free"); }
+  static void drop(void *p) { cudaFree(p); }
 };
+using Buf = GrowBuf<RusMemory>;
 
 // a tree of peel sequences over its roots: level l holds (parent, rotation) per node; the top level's matrices and
 // keys (the matrices only while the tree grows)
@@ -627,6 +624,7 @@ class RusContext {
     const int Dtop = tab->D.top();
     Tree &T = search;
     T.n.assign(1, 0);
+    ReleaseUnlessDone<Tree> guard{search};
     {
       std::vector<int> mats;
       for (int r = 0; r < spec.nroot; r++) {
@@ -684,6 +682,7 @@ class RusContext {
       }
       res.rc = rc;
     }
+    guard.done = true;
     res.launches = launches - l0;
     res.total_seconds = now_s() - t0;
     return res.rc;

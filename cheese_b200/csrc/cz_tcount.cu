@@ -23,6 +23,7 @@
 #include <map>
 #include <stdexcept>
 
+#include "cz_buf.h"
 #include "cz_sort.cuh"
 #include "cz_text.h"
 #include "cz_tcount.h"
@@ -694,20 +695,16 @@ void tck(cudaError_t e, const char *what) {
     throw TcCudaError(std::string("CUDA error after ") + what + ": " + cudaGetErrorString(e));
   }
 }
-struct Buf {
-  void *p = nullptr;
-  size_t cap = 0;
-  void ensure(size_t b) {
-    if (b <= cap) return;
-    if (p) tck(cudaFree(p), "free");
-    size_t c = std::max(b, cap + cap / 2);
-    c = (c + 255) & ~(size_t)255;
-    tck(cudaMalloc(&p, c), "cudaMalloc");
-    cap = c;
+struct TcMemory {
+  static void *get(size_t n) {
+    void *p = nullptr;
+    tck(cudaMalloc(&p, n), "cudaMalloc");
+    return p;
   }
-  template <typename T> T *as() const { return (T *)p; }
-  void release() { if (p) cudaFree(p); p = nullptr; cap = 0; }
+  static void put(void *p) { tck(cudaFree(p), "free"); }
+  static void drop(void *p) { cudaFree(p); }
 };
+using Buf = GrowBuf<TcMemory>;
 
 // a tree of peel sequences: level l holds (parent, rotation) per node; keys of the top level
 struct Tree {
@@ -1220,6 +1217,7 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
     res.table_levels = tab->D.top();
     Tree &T = ctx->search;                                        // search: peel rotations off U
     T.n.assign(1, 1);
+    ReleaseUnlessDone<Tree> guard{ctx->search};
     ctx->level_keys(su, T, 0);
     ctx->check_ovf();
     int rc = 1;
@@ -1268,6 +1266,7 @@ int tcount_run(TcountContext *ctx, const TSpec &sp, const TcOptions &opt,
       if (j + tab->D.top() >= opt.maxt) break;
     }
     res.rc = rc;
+    guard.done = true;
   } catch (const std::overflow_error &e) {
     res.error = e.what();
     res.rc = 4;
