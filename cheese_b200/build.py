@@ -28,7 +28,8 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-ccbin", HOSTCXX, "-Xcompiler", "-f
 LIB_SOURCES = ["cz_search.cu", "cz_tcount.cu", "cz_clifford.cu", "cz_rus.cu", "cz_spec.cpp", "cz_specgen.cpp",
                "cz_capi.cpp", "cz_serve.cpp"]
 HEADERS = ["cz_common.h", "cz_spec.h", "cz_engine.h", "cz_sort.cuh", "cz_tcount.h", "cz_clifford.h", "cz_tableau.h",
-           "cz_capi_internal.h", "cz_specgen.h", "cz_rus.h", "cz_rus_node.h", "cz_text.h", "cz_buf.h"]
+           "cz_capi_internal.h", "cz_specgen.h", "cz_rus.h", "cz_rus_node.h", "cz_text.h", "cz_buf.h",
+           "cz_place.h"]
 BINARIES = {"cheese": "cli_cheese.cpp", "tcount": "cli_tcount.cpp", "cliffopt": "cli_cliffopt.cpp",
             "cheese-spec": "cli_spec.cpp", "rus": "cli_rus.cpp"}
 

@@ -7,6 +7,8 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "cz_place.h"
+
 namespace cz {
 namespace {   // each translation unit that sorts gets its own copy of these kernels
 
@@ -327,17 +329,19 @@ __global__ void __launch_bounds__(OS_THREADS, 4) k_sort_onesweep(const uint64_t 
 // memory, and a key is compared with 32 at once from a broadcast. n^2 / 32 compares, but no passes, no scratch and one
 // launch where the digit passes need 1 + passes and a memset: up to SORT_COUNT_MAX keys it is faster (32-bit
 // digits on the B200, us: 1000 keys 36 -> 11, 4000 43 -> 16, 8192 46 -> 25; 8193 by digit passes 45).
+// Keys that change while they are sorted (a caller's, not ordered before the call) can give two pairs one place, or one the
+// place n, which is not written. Where the caller's flags are given, the places' marks are summed: see SortFlags.
 constexpr int SORT_COUNT_MAX = 8192;
 constexpr int SC_THREADS = 256, SC_TILE = 1024;
 template <typename K>     // uint32_t when hi - lo <= 32, else uint64_t: the digits compared
 __global__ void __launch_bounds__(SC_THREADS) k_sort_count(const uint64_t *kin, const uint32_t *vin, uint64_t *kout, uint32_t *vout,
-                                                           int n, int lo, uint64_t mask, unsigned *err) {
+                                                           int n, int lo, uint64_t mask, unsigned long long *places) {
   constexpr int NW = SC_THREADS / 32, PER = SC_TILE / NW;
   __shared__ K tile[SC_TILE];
   __shared__ int part[NW][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i0 = blockIdx.x * 32, i = i0 + lane;
-  if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;      // the scratch's flag, as a digit sort clears it
-  const K mine = i < n ? (K)((kin[i] >> lo) & mask) : 0;
+  const uint64_t key = i < n ? kin[i] : 0;
+  const K mine = (K)((key >> lo) & mask);
   int cnt = 0;
   for (int t0 = 0; t0 < n; t0 += SC_TILE) {
     const int tn = min(SC_TILE, n - t0);
@@ -357,20 +361,33 @@ __global__ void __launch_bounds__(SC_THREADS) k_sort_count(const uint64_t *kin, 
   }
   part[w][lane] = cnt;
   __syncthreads();
-  if (w == 0 && i < n) {
-    int pos = 0;
+  if (w == 0) {
+    unsigned pos = 0;
 #pragma unroll
-    for (int x = 0; x < NW; x++) pos += part[x][lane];
-    kout[pos] = kin[i];
-    vout[pos] = vin[i];
+    for (int x = 0; x < NW; x++) pos += (unsigned)part[x][lane];
+    if (i < n && pos < (unsigned)n) {
+      kout[pos] = key;
+      vout[pos] = vin[i];
+    }
+    if (places) {
+      uint64_t d = i < n ? place_mark(pos) - place_mark((uint32_t)i) : 0;
+#pragma unroll
+      for (int m = 16; m; m >>= 1) d += __shfl_xor_sync(0xffffffffu, d, m);
+      if (lane == 0 && d) atomicAdd(places, (unsigned long long)d);
+    }
   }
 }
 
+// what a sort tells of itself: both words are 0 before it and after a good one, so nothing clears them between sorts
+struct SortFlags {
+  uint32_t err, pad;              // digit passes: bit 0, a look-back wait gave up; bit 1, a position outside the array
+  unsigned long long places;      // counting sort: the sum of its places' marks, 0 for a permutation
+};
 struct SortScratch {
   uint32_t *hist = nullptr;       // sort scratch: sort_hist_words(n) words
   uint32_t *partials = nullptr;   // scan partials: scan_partials_words(sort_hist_words(n)) words (large sorts)
   size_t cap_hist = 0, cap_part = 0;
-  uint32_t *err = nullptr;        // where a failed look-back is flagged (nullptr: the scratch's own word)
+  SortFlags *flags = nullptr;     // for sort_failed (nullptr: not read)
 };
 
 // sorts (k0, v0) by bits [lo, hi) of the key (hi - lo a multiple of 8, at most 64), stable; uses (k1, v1) as the
@@ -379,12 +396,12 @@ inline bool radix_sort(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, s
                        const SortScratch &sc, cudaStream_t s, int *launches) {
   if (n <= 1 || hi <= lo) return false;
   if (n <= (size_t)SORT_COUNT_MAX) {
-    unsigned *own = sc.err ? nullptr : sc.hist + 256 * OS_MAXPASS + OS_MAXPASS;
+    unsigned long long *places = sc.flags ? &sc.flags->places : nullptr;
     const unsigned nb = (unsigned)((n + 31) / 32);
     if (hi - lo <= 32)
-      k_sort_count<uint32_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 32 ? 0xffffffffULL : (1ULL << (hi - lo)) - 1, own);
+      k_sort_count<uint32_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 32 ? 0xffffffffULL : (1ULL << (hi - lo)) - 1, places);
     else
-      k_sort_count<uint64_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 64 ? ~0ULL : (1ULL << (hi - lo)) - 1, own);
+      k_sort_count<uint64_t><<<nb, SC_THREADS, 0, s>>>(k0, v0, k1, v1, (int)n, lo, hi - lo == 64 ? ~0ULL : (1ULL << (hi - lo)) - 1, places);
     if (launches) (*launches)++;
     return true;
   }
@@ -394,7 +411,7 @@ inline bool radix_sort(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, s
   cudaMemsetAsync(sc.hist, 0, (OS_HEAD_WORDS + (scan ? 0 : 2 * 256 * ntiles)) * 4, s);
   unsigned long long *status = (unsigned long long *)(sc.hist + OS_HEAD_WORDS);
   uint32_t *offs = sc.hist + OS_HEAD_WORDS;                  // scan path: the digit-major tile histograms
-  unsigned *err = sc.err ? sc.err : sc.hist + 256 * OS_MAXPASS + OS_MAXPASS;
+  unsigned *err = sc.flags ? &sc.flags->err : sc.hist + 256 * OS_MAXPASS + OS_MAXPASS;
   if (!scan) {
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
@@ -422,14 +439,15 @@ inline bool radix_sort(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, s
   if (launches) *launches += scan ? 5 * npass : 1 + npass;
   return flip;
 }
-// the last sort's flags on this scratch (synchronises the stream): bit 0, a look-back wait gave up (the result is
+// the last sort's flags (synchronises the stream; the scratch has them): bit 0, a look-back wait gave up (the result is
 // exact all the same: the tile counted its predecessors' digits itself); bit 1, a scatter position fell outside the
-// array (the keys changed while the sort ran; those writes were skipped and the result is not to be used)
+// array, or a small sort's places are no permutation (the keys changed while the sort ran; the result is not to be used)
 inline uint32_t sort_failed(const SortScratch &sc, cudaStream_t s) {
-  uint32_t e = 0;
-  cudaMemcpyAsync(&e, sc.err ? sc.err : sc.hist + 256 * OS_MAXPASS + OS_MAXPASS, 4, cudaMemcpyDeviceToHost, s);
+  SortFlags f{0, 0, 0};
+  cudaMemcpyAsync(&f, sc.flags, sizeof f, cudaMemcpyDeviceToHost, s);
   cudaStreamSynchronize(s);
-  return e;
+  if (f.err || f.places) cudaMemsetAsync(sc.flags, 0, sizeof f, s);
+  return f.err | (f.places ? 2u : 0u);
 }
 
 }  // namespace
