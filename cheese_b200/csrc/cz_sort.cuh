@@ -327,11 +327,16 @@ __global__ void __launch_bounds__(OS_THREADS, 4) k_sort_onesweep(const uint64_t 
 // Small sorts in one launch: a pair's place is the number of smaller keys plus the number of equal keys before it,
 // counted directly. A block places 32 pairs (one per lane); its warps share the keys, read tile by tile into shared
 // memory, and a key is compared with 32 at once from a broadcast. n^2 / 32 compares, but no passes, no scratch and one
-// launch where the digit passes need 1 + passes and a memset: up to SORT_COUNT_MAX keys it is faster (32-bit
-// digits on the B200, us: 1000 keys 36 -> 11, 4000 43 -> 16, 8192 46 -> 25; 8193 by digit passes 45).
+// launch where the digit passes need 1 + passes and a memset. On the B200 (us; counting / digit passes):
+//   pairs   8 bits       16 bits      32 bits      64 bits
+//   1000    11 / 16      11 / 22      11 / 34      12 / 59
+//   4096    16 / 17.5    16 / 26      16 / 42      16 / 75
+//   6000    20 / 18      20 / 26      20 / 42      24 / 75
+//   8192    24.5 / 18    24.5 / 26    24.5 / 42    29 / 75
+// so one pass is counted up to 4096 pairs, and two or more, which meet counting at about 8400, up to 8192.
 // Keys that change while they are sorted (a caller's, not ordered before the call) can give two pairs one place, or one the
 // place n, which is not written. Where the caller's flags are given, the places' marks are summed: see SortFlags.
-constexpr int SORT_COUNT_MAX = 8192;
+constexpr size_t sort_count_max(int bits) { return bits <= 8 ? 4096 : 8192; }   // pairs sorted by counting
 constexpr int SC_THREADS = 256, SC_TILE = 1024;
 template <typename K>     // uint32_t when hi - lo <= 32, else uint64_t: the digits compared
 __global__ void __launch_bounds__(SC_THREADS) k_sort_count(const uint64_t *kin, const uint32_t *vin, uint64_t *kout, uint32_t *vout,
@@ -395,7 +400,7 @@ struct SortScratch {
 inline bool radix_sort(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, size_t n, int lo, int hi,
                        const SortScratch &sc, cudaStream_t s, int *launches) {
   if (n <= 1 || hi <= lo) return false;
-  if (n <= (size_t)SORT_COUNT_MAX) {
+  if (n <= sort_count_max(hi - lo)) {
     unsigned long long *places = sc.flags ? &sc.flags->places : nullptr;
     const unsigned nb = (unsigned)((n + 31) / 32);
     if (hi - lo <= 32)

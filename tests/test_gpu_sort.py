@@ -73,3 +73,21 @@ def test_counted_and_digit_sorts_meet(engine, n, lo, hi):
     torch.cuda.synchronize()
     assert torch.equal(vals, want_v)
     assert torch.equal(keys, want_k)
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 6144])
+def test_one_byte_sorts_meet(engine, n):
+    """one digit pass is counted only up to 4096 pairs: both sides of that line, equal keys in their order"""
+    import torch
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(n)
+    keys = torch.randint(-(1 << 62), 1 << 62, (n,), dtype=torch.int64, device=dev, generator=g) * 2
+    vals = torch.arange(n, dtype=torch.int32, device=dev)
+    for lo in (0, 32, 56):
+        want_k, want_v = stable_reference(keys, vals, lo, lo + 8)
+        k, v = keys.clone(), vals.clone()
+        torch.cuda.synchronize()
+        engine.sort_pairs(k.data_ptr(), v.data_ptr(), n, lo, lo + 8)
+        torch.cuda.synchronize()
+        assert torch.equal(v, want_v)
+        assert torch.equal(k, want_k)
