@@ -96,7 +96,7 @@ struct DevStats {
   unsigned long long w2, w3, dead, alive, found, first_found, n_surv, t_evals, children, work, full;
   unsigned int ovf, surv_overflow;
   unsigned long long n_work, n_kept;
-  unsigned long long n_tq;            // deferred T evaluations queued
+  unsigned long long n_tq, n_left;    // deferred T evaluations queued; those the packed form left to the general one
   unsigned int sort_err, pad;         // a dedupe sort's look-back gave up (its result is not used)
   unsigned long long work2;           // parent counter of the level kernel's second part (multi-qubit gates)
 };
@@ -506,10 +506,6 @@ template <int NQ, typename ST> __device__ __noinline__ int warp_tbound32(const Z
 }
 template <int NQ, typename ST> __device__ __noinline__ int warp_tbound64(const Z4<ST> *S, int k, int lane) {
   return tbound_lanes<NQ, uint64_t, 4>(S, k, lane);
-}
-// the same values one component per pass: a quarter of the registers, for kernels where this is the rare path
-template <int NQ, typename ST> __device__ __noinline__ int warp_tbound_slim(const Z4<ST> *S, int k, int lane) {
-  return 2 * (NQ + k) > 64 ? tbound_lanes<NQ, uint64_t, 4>(S, k, lane) : tbound_lanes<NQ, uint32_t, 4>(S, k, lane);
 }
 template <int NQ, typename ST> __device__ __forceinline__ int ptm_bound(const Z4<ST> *S, int k, int lane) {
   return 2 * (NQ + k) > 64 ? warp_tbound64<NQ, ST>(S, k, lane) : warp_tbound32<NQ, ST>(S, k, lane);
@@ -1920,6 +1916,7 @@ template <typename ST> struct TBoundArgs {
   const NodeMeta *meta;
   const TQEntry *tq;
   unsigned long long tqcap;
+  uint32_t *left;                   // the entries that the packed form leaves to the general one (nullptr: all of them)
   int GS, rem, keep;                // rem, keep: without jobs
   const uint32_t *fjob;
   const DevSpec *specs;
@@ -1932,13 +1929,16 @@ template <typename ST> struct TBoundArgs {
 };
 // One block's warps walk the queue with a fixed stride. Bound by issue: a dead entry (most are) is the child's update,
 // its packing and one packed round. 3.96 M entries of two budget 12 proofs: 32.7 ms with 32-bit components, 11.7 ms
-// packed, 5.9 ms with the diagonal update in registers, the general form in a walk of its own and one alive test;
-// with the children that their parent's columns already decide (cols_t_least) left out, 0.57 M entries in 2.4 ms.
-template <int NQ, typename ST, bool BATCHED = false>
-__global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
+// packed, 5.9 ms with the diagonal update in registers, the general form apart and one alive test; with the children
+// that their parent's columns already decide (cols_t_least) left out, 0.57 M entries in 2.4 ms.
+// GENERAL: the general form, in a launch of its own over the entries that the packed one listed (or the whole queue): its
+// 128 transform values per lane take the registers of one block per SM.
+template <int NQ, typename ST, bool BATCHED, bool GENERAL>
+__global__ void __launch_bounds__(TB_WARPS * 32, GENERAL ? 1 : TB_MINB)
     k_tbound(const __grid_constant__ DevSpec sp0, const TBoundArgs<ST> a) {
   constexpr int N = 1 << NQ, E = N * N, EPL = E >= 32 ? E / 32 : 1, CHUNKS = E * (int)sizeof(Z4<ST>) / 16;
-  constexpr bool PACKED = sizeof(ST) == 4;               // the packed T bound (int32 limbs)
+  constexpr bool PACKED = !GENERAL;
+  static_assert(GENERAL || sizeof(ST) == 4, "the packed form is of int32 limbs");
   constexpr int NB = sizeof(ST) == 4 ? 2 : 1;            // int64 limbs: one buffer (shared memory), no overlap
   __shared__ __align__(16) Z4<ST> sP[TB_WARPS][NB][E];  // the entry's parent, and the next entry's arriving
   __shared__ Z4<ST> sC[TB_WARPS][E];
@@ -1946,7 +1946,7 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
   __shared__ int sX[PACKED ? TB_WARPS : 1][PACKED ? E : 1];
   __shared__ uint64_t W[E];
   __shared__ DevSpec s_sp;
-  const unsigned long long n = a.st->n_tq < a.tqcap ? a.st->n_tq : a.tqcap;
+  const unsigned long long queued = GENERAL && a.left ? a.st->n_left : a.st->n_tq, n = queued < a.tqcap ? queued : a.tqcap;
   const unsigned long long stride = (unsigned long long)gridDim.x * TB_WARPS;
   if ((unsigned long long)blockIdx.x * TB_WARPS >= n) return;
   init_weights(W, E);
@@ -1976,146 +1976,138 @@ __global__ void __launch_bounds__(TB_WARPS * 32, sizeof(ST) == 4 ? TB_MINB : 1)
   // (cp.async) while the current entry's T bound runs
   auto take = [&](TQEntry &q, unsigned long long e, int b) {
     if (e >= n) return false;
-    q = a.tq[e];
+    q = a.tq[GENERAL && a.left ? a.left[e] : e];
     const char *src = (const char *)(a.R + q.p * (unsigned long long)E);
     char *dst = (char *)sP[w][b];
     for (int i = lane; i < CHUNKS; i += 32) cp_async16(dst + 16 * i, src + 16 * i);
     return true;
   };
-  // one walk over the warp's entries with the packed form; those it does not take, if any, in a second walk with the
-  // general one (a call in the loop would cost the packed form its registers)
-  bool left = !PACKED;
-  auto walk = [&](auto general) {
-    constexpr bool GENERAL = decltype(general)::value;
-    TQEntry q;
-    int b = 0;
-    unsigned long long e = (unsigned long long)blockIdx.x * TB_WARPS + w;
-    bool have = take(q, e, 0);
-    cp_async_commit();
-    while (have) {
-      TQEntry q2;
-      bool more = false;
-      e += stride;
-      if constexpr (NB == 2) {
-        more = take(q2, e, b ^ 1);
-        cp_async_commit();
-        cp_async_wait<1>();                            // this entry's parent has arrived (the next may be in flight)
-      } else {
-        cp_async_wait<0>();
+  TQEntry q;
+  int b = 0;
+  unsigned long long e = (unsigned long long)blockIdx.x * TB_WARPS + w;
+  bool have = take(q, e, 0);
+  cp_async_commit();
+  while (have) {
+    TQEntry q2;
+    bool more = false;
+    e += stride;
+    if constexpr (NB == 2) {
+      more = take(q2, e, b ^ 1);
+      cp_async_commit();
+      cp_async_wait<1>();                            // this entry's parent has arrived (the next may be in flight)
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncwarp();
+    const Z4<ST> *P = sP[w][b];
+    if constexpr (BATCHED) {
+      const int pj = (int)a.fjob[q.p];
+      if (pj != job) {                               // the spec of this entry's job
+        if (job >= 0) flush(a.jst + job);
+        job = pj;
+        spp = a.specs + job;
+        const int t = a.jt[job];
+        rem = spp->depth - t; keep = t < spp->depth;
+        conjmask = 0;
+        for (int i = 0; i < spp->nsym; i++) conjmask |= (unsigned)(spp->symconj[i] != 0) << i;
       }
-      __syncwarp();
-      const Z4<ST> *P = sP[w][b];
-      if constexpr (BATCHED) {
-        const int pj = (int)a.fjob[q.p];
-        if (pj != job) {                               // the spec of this entry's job
-          if (job >= 0) flush(a.jst + job);
-          job = pj;
-          spp = a.specs + job;
-          const int t = a.jt[job];
-          rem = spp->depth - t; keep = t < spp->depth;
-          conjmask = 0;
-          for (int i = 0; i < spp->nsym; i++) conjmask |= (unsigned)(spp->symconj[i] != 0) << i;
-        }
-      }
-      const DevSpec &sp = *spp;
-      const NodeMeta pm = a.meta[q.p];
-      // the largest T bound a child lives with: lane T tries T (combine is monotone in it), so one evaluation per child
-      int thr[2];
-      const int h = q.k > q.hs ? q.k : q.hs;
+    }
+    const DevSpec &sp = *spp;
+    const NodeMeta pm = a.meta[q.p];
+    // the largest T bound a child lives with: lane T tries T (combine is monotone in it), so one evaluation per child
+    int thr[2];
+    const int h = q.k > q.hs ? q.k : q.hs;
 #pragma unroll
-      for (int s2 = 0; s2 < 2; s2++) {
-        const bool ok = s2 < q.n && (sp.lite ? q.k + (lane + sp.tdiv - 1) / sp.tdiv <= rem
-                                             : combine(h, lane, q.c2, __popc(q.ntriv[s2])) <= rem);
-        thr[s2] = 31 - __clz((int)__ballot_sync(FULL, ok));
+    for (int s2 = 0; s2 < 2; s2++) {
+      const bool ok = s2 < q.n && (sp.lite ? q.k + (lane + sp.tdiv - 1) / sp.tdiv <= rem
+                                           : combine(h, lane, q.c2, __popc(q.ntriv[s2])) <= rem);
+      thr[s2] = 31 - __clz((int)__ballot_sync(FULL, ok));
+    }
+    // the packed form takes the children of one-qubit unit monomials (t, tdg): the parent's entries times units, so the
+    // exponent stays the parent's (tbound_forms knows when every entry is such)
+    const int col = lane & (N - 1);
+    int mine = q.n;                                  // the entry's children, none when it is left to the general form
+    if (PACKED && !(sp.unit && NQ + q.k <= PACK_MAX && q.k == pm.k && (sp.gflags[q.g[0]] & GF_UNITMON) &&
+                    (q.n < 2 || (sp.gflags[q.g[1]] & GF_UNITMON)))) {
+      mine = 0;
+      if (lane == 0) {
+        const unsigned long long l = atomicAdd(&a.st->n_left, 1ULL);
+        if (a.left) a.left[l] = (uint32_t)(e - stride);
       }
-      // the packed walk takes the children of one-qubit unit monomials (t, tdg): the parent's entries times units, so the
-      // exponent stays the parent's
-      const int col = lane & (N - 1);
-      bool packed = PACKED && sp.unit && NQ + q.k <= PACK_MAX && q.k == pm.k && (sp.gflags[q.g[0]] & GF_UNITMON);
-      const int mono0 = packed ? sp.gmono[q.g[0]][col] : 0;
-      if (q.n > 1) packed = packed && (sp.gflags[q.g[1]] & GF_UNITMON);
-      int mine = q.n;                                // the entry's children, none when the other walk takes it
-      if (packed == GENERAL) {
-        mine = 0;
-        left = true;
-      }
-      bool ovf;
-      int T = 0;
-      uint64_t cols = 0;
-      if (mine) neval++;
-      if constexpr (GENERAL) {
-        if (mine) {
-          (void)warp_child<NQ, ST>(P, C, q.g[0], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
-          __syncwarp();
-          T = PACKED ? warp_tbound_slim<NQ, ST>(C, q.k, lane) : ptm_bound<NQ, ST>(C, q.k, lane);
+    }
+    bool ovf;
+    int T = 0;
+    uint64_t cols = 0;
+    if (mine) neval++;
+    if constexpr (GENERAL) {
+      (void)warp_child<NQ, ST>(P, C, q.g[0], pm.k, sp, &sp, lane, ovf);   // the level kernel's child residual
+      __syncwarp();
+      T = ptm_bound<NQ, ST>(C, q.k, lane);
+    } else if (mine) {
+      const int mono0 = sp.gmono[q.g[0]][col];
+#pragma unroll
+      for (int j = 0; j < EPL; j++)
+        if (lane + 32 * j < E) {
+          const int4 y = pack_entry(mono_entry<NQ>(P, mono0, lane, j));
+          sY[w][lane + 32 * j] = y;
+          sX[w][lane + 32 * j] = y.x;
         }
-      } else if (mine) {
+      __syncwarp();
+      T = packed_tbound<NQ>(sY[w], sX[w], q.k, lane, max(thr[0], thr[1]), keep && NQ == 3, cols);   // T <= 2 (NQ + k) < 31:
+                                                                                          // thr is exact
+    }
+    for (int s2 = 0; s2 < mine; s2++) {
+      const bool alive = T < 31 ? T <= thr[s2]
+                                : (sp.lite ? q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem
+                                           : combine(h, T, q.c2, __popc(q.ntriv[s2])) <= rem);
+      if (!alive) { ndead++; continue; }
+      nalive++;
+      if (!keep) continue;
+      if constexpr (GENERAL) {
+        if (s2) {                                    // the sibling's residual
+          __syncwarp();
+          (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);
+        }
+      } else {
 #pragma unroll
         for (int j = 0; j < EPL; j++)
-          if (lane + 32 * j < E) {
-            const int4 y = pack_entry(mono_entry<NQ>(P, mono0, lane, j));
-            sY[w][lane + 32 * j] = y;
-            sX[w][lane + 32 * j] = y.x;
-          }
-        __syncwarp();
-        T = packed_tbound<NQ>(sY[w], sX[w], q.k, lane, max(thr[0], thr[1]), keep && NQ == 3, cols);   // T <= 2 (NQ + k) < 31:
-                                                                                            // thr is exact
+          if (lane + 32 * j < E) C[lane + 32 * j] = mono_entry<NQ>(P, sp.gmono[q.g[s2]][col], lane, j);
       }
-      for (int s2 = 0; s2 < mine; s2++) {
-        const bool alive = T < 31 ? T <= thr[s2]
-                                  : (sp.lite ? q.k + (T + sp.tdiv - 1) / sp.tdiv <= rem
-                                             : combine(h, T, q.c2, __popc(q.ntriv[s2])) <= rem);
-        if (!alive) { ndead++; continue; }
-        nalive++;
-        if (!keep) continue;
-        if constexpr (GENERAL) {
-          if (s2) {                                    // the sibling's residual
-            __syncwarp();
-            (void)warp_child<NQ, ST>(P, C, q.g[s2], pm.k, sp, &sp, lane, ovf);
+      __syncwarp();
+      uint64_t k1, k2;
+      warp_class_key<NQ, ST>(C, q.k, sp.nsym, conjmask, sp.symperm, W, lane, k1, k2);
+      unsigned long long slot = 0;
+      if (lane == 0) slot = atomicAdd(&a.st->n_surv, 1ULL);
+      slot = __shfl_sync(FULL, slot, 0);
+      if (slot < a.cap) {
+        if (lane == 0) {
+          a.sh1[slot] = k1; a.sh2[slot] = k2; a.sidx[slot] = q.p * (unsigned long long)a.GS + q.g[s2];
+          NodeMeta nm;
+          nm.k = q.k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = q.c2; nm.g1 = q.g[s2]; nm.g2 = pm.g1;
+          nm.hsn = (uint8_t)((q.hs == 2 ? 1 : 0) | (q.ntriv[s2] << 1));
+          nm.needs = q.needs;
+          nm.cols = cols;
+          if (s2 && cols) {                        // the sibling differs by a power of S: an odd one exchanges X and Y
+            const uint8_t *a0 = sp.gph[q.g[0]], *a1 = sp.gph[q.g[1]];
+            if ((a0[3] - a0[0] - a1[3] + a1[0]) & 3) nm.cols = cols_after(cols, COL_S | sp.gq[q.g[0]][0] << 3);
           }
-        } else {
-#pragma unroll
-          for (int j = 0; j < EPL; j++)
-            if (lane + 32 * j < E) C[lane + 32 * j] = mono_entry<NQ>(P, sp.gmono[q.g[s2]][col], lane, j);
+          a.smeta[slot] = nm;
         }
-        __syncwarp();
-        uint64_t k1, k2;
-        warp_class_key<NQ, ST>(C, q.k, sp.nsym, conjmask, sp.symperm, W, lane, k1, k2);
-        unsigned long long slot = 0;
-        if (lane == 0) slot = atomicAdd(&a.st->n_surv, 1ULL);
-        slot = __shfl_sync(FULL, slot, 0);
-        if (slot < a.cap) {
-          if (lane == 0) {
-            a.sh1[slot] = k1; a.sh2[slot] = k2; a.sidx[slot] = q.p * (unsigned long long)a.GS + q.g[s2];
-            NodeMeta nm;
-            nm.k = q.k; nm.T = (uint8_t)(T > 255 ? 255 : T); nm.c2 = q.c2; nm.g1 = q.g[s2]; nm.g2 = pm.g1;
-            nm.hsn = (uint8_t)((q.hs == 2 ? 1 : 0) | (q.ntriv[s2] << 1));
-            nm.needs = q.needs;
-            nm.cols = cols;
-            if (s2 && cols) {                        // the sibling differs by a power of S: an odd one exchanges X and Y
-              const uint8_t *a0 = sp.gph[q.g[0]], *a1 = sp.gph[q.g[1]];
-              if ((a0[3] - a0[0] - a1[3] + a1[0]) & 3) nm.cols = cols_after(cols, COL_S | sp.gq[q.g[0]][0] << 3);
-            }
-            a.smeta[slot] = nm;
-          }
-        } else if (lane == 0) {
-          a.st->surv_overflow = 1;
-        }
-        __syncwarp();
+      } else if (lane == 0) {
+        a.st->surv_overflow = 1;
       }
-      __syncwarp();                                    // every lane is done with this buffer before it is refilled
-      if constexpr (NB == 1) {
-        more = take(q2, e, 0);
-        cp_async_commit();
-      }
-      have = more;
-      q = q2;
-      b ^= NB - 1;
+      __syncwarp();
     }
-    cp_async_wait<0>();
-  };
-  if constexpr (PACKED) walk(std::false_type{});
-  if (left) walk(std::true_type{});
+    __syncwarp();                                    // every lane is done with this buffer before it is refilled
+    if constexpr (NB == 1) {
+      more = take(q2, e, 0);
+      cp_async_commit();
+    }
+    have = more;
+    q = q2;
+    b ^= NB - 1;
+  }
+  cp_async_wait<0>();
   if constexpr (BATCHED) { if (job >= 0) flush(a.jst + job); }
   else flush(a.st);
 }
@@ -3011,7 +3003,7 @@ struct Engine::Impl {
   cudaEvent_t ev[4];
   DBuf fR, fMeta, fR2, fMeta2;             // frontier, next frontier
   DBuf sH1, sH2, sIdx, sMeta;              // survivors of the current level (32-byte records)
-  DBuf tq;                                 // deferred T evaluations of the current level
+  DBuf tq, tqleft;                         // deferred T evaluations of the current level; TBoundArgs::left
   DBuf k0, k1, v0, v1, hist, part;         // sort
   DBuf work, tmp, kidx, kslot;             // dedupe
   DBuf gshort;                             // the goal pass: its counters and candidate list
@@ -3083,7 +3075,7 @@ struct Engine::Impl {
   }
   size_t trim() {
     size_t n = 0;
-    for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &k0, &k1, &v0, &v1, &hist, &part,
+    for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &tqleft, &k0, &k1, &v0, &v1, &hist, &part,
                     &work, &tmp, &kidx, &kslot, &fK1, &fK2, &keys2, &old, &gshort, &outb}) {
       n += b->cap;
       b->release();
@@ -3096,7 +3088,7 @@ struct Engine::Impl {
   }
   ~Impl() {
     cudaSetDevice(dev);
-    for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &k0, &k1, &v0, &v1, &hist, &part,
+    for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &tqleft, &k0, &k1, &v0, &v1, &hist, &part,
                     &work, &tmp, &kidx, &kslot, &stats})
       b->release();
     for (auto &sd : specs) sd.release();
@@ -3142,6 +3134,34 @@ __global__ void k_walk_back(const __grid_constant__ TreeLevels tree, unsigned lo
     out[l - 1] = tree.gat[l][i];
     i = tree.par[l][i];
   }
+}
+
+// The forms of the T bound that the queue of level t can need. A spec that is not unitary, and int64 limbs, take the general
+// one alone. The packed one takes every child of a unit monomial while its exponent k allows: k is at most the root's plus
+// the most a gate adds on each of t - 1 levels, and an entry is queued only with k <= depth - t. The general launch is
+// left out where that shows it empty (a launch that finds nothing costs 3 us; small searches make 50 in a millisecond).
+struct TboundForms { bool packed, general; };
+template <int NQ, typename ST> TboundForms tbound_forms(const HostSpec &hs, const DevSpec &sp, int t, int depth) {
+  if (sizeof(ST) != 4 || !sp.unit) return {false, true};
+  if (!hs.standard && !hs.lite) return {true, false};          // no bounds, nothing queued
+  int up = 0;
+  for (int g = 0; g < hs.G; g++) {
+    if (!(hs.gflags[g] & GF_CLIFFORD) && !(sp.gflags[g] & GF_UNITMON)) return {true, true};
+    up = std::max(up, hs.gik[g]);
+  }
+  return {true, NQ + std::min(hs.rk + (t - 1) * up, depth - t) > PACK_MAX};
+}
+template <int NQ, typename ST, bool BATCHED>
+int launch_tbound(const DevSpec &sp, TBoundArgs<ST> a, uint32_t *left, TboundForms f, unsigned grid, cudaStream_t s) {
+  a.left = left;
+  if constexpr (sizeof(ST) == 4) {
+    if (f.packed) k_tbound<NQ, ST, BATCHED, false><<<grid, TB_WARPS * 32, 0, s>>>(sp, a);
+  }
+  if (f.general) {
+    if (!f.packed) a.left = nullptr;
+    k_tbound<NQ, ST, BATCHED, true><<<grid, TB_WARPS * 32, 0, s>>>(sp, a);
+  }
+  return (int)f.packed + (int)f.general;
 }
 
 template <int NQ, typename ST>
@@ -3216,6 +3236,8 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
         sMeta.ensure(cap * sizeof(NodeMeta));
       }
       tq.ensure(tqcap * sizeof(TQEntry));
+      const TboundForms forms = tbound_forms<NQ, ST>(hs, sp, t, depth);
+      if (forms.packed && forms.general) tqleft.ensure(tqcap * 4);
       if (attempt) { k_level_init<<<1, 32, 0, s>>>(nullptr, dst); launches++; }
       ExpandArgs<ST> a;
       a.m = m; a.t = t; a.rem = depth - t; a.keep = keep;
@@ -3240,8 +3262,8 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       tb.GS = G; tb.rem = depth - t; tb.keep = keep; tb.fjob = nullptr; tb.specs = nullptr; tb.jt = nullptr;
       tb.jst = nullptr; tb.st = dst; tb.cap = cap; tb.sh1 = sH1.as<uint64_t>(); tb.sh2 = sH2.as<uint64_t>();
       tb.sidx = sIdx.as<uint64_t>(); tb.smeta = sMeta.as<NodeMeta>();
-      k_tbound<NQ, ST><<<(unsigned)nsm * 4, TB_WARPS * 32, 0, s>>>(sp, tb);
-      launches += 2;
+      launches += 1 + launch_tbound<NQ, ST, false>(sp, tb, forms.general ? tqleft.as<uint32_t>() : nullptr, forms,
+                                                   (unsigned)nsm * 4, s);
       expand_launches++;
       ck(cudaGetLastError(), "expand kernel");
       if (opt.profile) ck(cudaEventRecord(ev[1], s), "event");
@@ -3266,6 +3288,10 @@ int Engine::Impl::levels(const HostSpec &hs, const DevSpec &sp, const Options &o
       return RC_CIRCUIT;
     }
     if (hstats->n_tq > tqcap) { res.error = "T queue overflow"; return RC_CUDA; }
+    if (hstats->n_left && !tbound_forms<NQ, ST>(hs, sp, t, depth).general) {
+      res.error = "T bounds left over";
+      return RC_CUDA;
+    }
     if (hstats->surv_overflow) { res.error = "survivor buffer overflow"; return RC_CUDA; }
     const DevStats h = *hstats;
     if (m * G > 0) surv_rate = (double)h.alive / ((double)m * G);
@@ -4734,7 +4760,7 @@ struct BatchImpl : BatchSession::Impl {
   VBuf sH1, sH2, sIdx, sMeta;              // survivors: 40-byte records
   DBuf stats;
   DBuf bgoal, jgoal;                       // the goal pass: counters + candidate list, per-job results
-  VBuf tq;                                 // deferred T evaluations
+  VBuf tq, tqleft;                         // deferred T evaluations; TBoundArgs::left
   VBuf k0, k1, v0, v1, work, tmp, kidx, kslot;
   DBuf hist, part, cnt;
   DBuf rJob, rTk, tptr, wbuf;
@@ -4763,7 +4789,7 @@ struct BatchImpl : BatchSession::Impl {
     for (DBuf *b : {&dspecs, &jt, &jst, &jact, &jdist, &stats, &hist, &part, &cnt, &rJob, &rTk, &tptr, &wbuf, &bgoal,
                     &jgoal})
       b->release();
-    for (VBuf *b : {&fR, &fMeta, &fJob, &fR2, &fMeta2, &fJob2, &sH1, &sH2, &sIdx, &sMeta, &tq, &k0, &k1, &v0, &v1,
+    for (VBuf *b : {&fR, &fMeta, &fJob, &fR2, &fMeta2, &fJob2, &sH1, &sH2, &sIdx, &sMeta, &tq, &tqleft, &k0, &k1, &v0, &v1,
                     &work, &tmp, &kidx, &kslot})
       b->release();
     for (auto &b : tpar) b.release();
@@ -4783,7 +4809,7 @@ struct BatchImpl : BatchSession::Impl {
     size_t b = 0;
     for (const DBuf *x : {&dspecs, &jt, &jst, &jact, &jdist, &hist, &part})
       b += x->cap;
-    for (const VBuf *x : {&fR, &fMeta, &fJob, &fR2, &fMeta2, &fJob2, &sH1, &sH2, &sIdx, &sMeta, &tq, &k0, &k1, &v0, &v1,
+    for (const VBuf *x : {&fR, &fMeta, &fJob, &fR2, &fMeta2, &fJob2, &sH1, &sH2, &sIdx, &sMeta, &tq, &tqleft, &k0, &k1, &v0, &v1,
                           &work, &tmp, &kidx, &kslot})
       b += x->cap;
     for (auto &x : tpar) b += x.cap;
@@ -5117,6 +5143,12 @@ struct BatchImpl : BatchSession::Impl {
         for (int g = 0; g < J[i].hs.G; g++) ncl += !(J[i].hs.gflags[g] & GF_CLIFFORD);
         tqcap += (unsigned long long)J[i].seg * (unsigned long long)std::max(1, ncl);
       }
+      TboundForms forms{false, false};                  // those that any of the chunk's jobs needs
+      for (int i : ch.jobs) {
+        const TboundForms f = tbound_forms<NQ, ST>(J[i].hs, J[i].sp, J[i].t, J[i].sp.depth);
+        forms.packed |= f.packed;
+        forms.general |= f.general;
+      }
       DevStats h{};
       // goal pass over the chunk: jobs whose goal it finds skip their found level in the level kernels
       bgoal.ensure(sizeof(GoalShort) + (size_t)GOAL_LIST * 4 + 64);
@@ -5139,6 +5171,7 @@ struct BatchImpl : BatchSession::Impl {
       std::vector<ulonglong2> hjg(jn);
       for (int attempt = 0; attempt < 2; attempt++) {
         tq.ensure(tqcap * sizeof(TQEntry));
+        if (forms.packed && forms.general) tqleft.ensure(tqcap * 4);
         if (cap) {
           sH1.ensure(cap * 8); sH2.ensure(cap * 8); sIdx.ensure(cap * 8);
           sMeta.ensure(cap * sizeof(NodeMeta));
@@ -5170,15 +5203,17 @@ struct BatchImpl : BatchSession::Impl {
         tb.GS = BATCH_GS; tb.rem = 0; tb.keep = 0; tb.fjob = fJob.as<uint32_t>(); tb.specs = dspecs.as<DevSpec>();
         tb.jt = jt.as<int>(); tb.jst = jst.as<DevStats>(); tb.st = dst; tb.cap = cap; tb.sh1 = sH1.as<uint64_t>();
         tb.sh2 = sH2.as<uint64_t>(); tb.sidx = sIdx.as<uint64_t>(); tb.smeta = sMeta.as<NodeMeta>();
+        const unsigned tgrid = (unsigned)(nsm * tune.tbound_blocks_per_sm);
+        int ntb;
         if (ch.jobs.size() == 1) {               // one job: the plain kernel, its spec a parameter (its tallies go
           const Job &jj = J[jlo];                 // to the chunk's block and are added to the job's below)
           tb.fjob = nullptr; tb.specs = nullptr; tb.jt = nullptr; tb.jst = nullptr;
           tb.rem = jj.sp.depth - jj.t; tb.keep = jj.t < jj.sp.depth;
-          k_tbound<NQ, ST, false><<<(unsigned)(nsm * tune.tbound_blocks_per_sm), TB_WARPS * 32, 0, s>>>(jj.sp, tb);
+          ntb = launch_tbound<NQ, ST, false>(jj.sp, tb, forms.general ? tqleft.as<uint32_t>() : nullptr, forms, tgrid, s);
         } else {
-          k_tbound<NQ, ST, true><<<(unsigned)(nsm * tune.tbound_blocks_per_sm), TB_WARPS * 32, 0, s>>>(DevSpec{}, tb);
+          ntb = launch_tbound<NQ, ST, true>(DevSpec{}, tb, forms.general ? tqleft.as<uint32_t>() : nullptr, forms, tgrid, s);
         }
-        nlaunch += 2;
+        nlaunch += 1 + ntb;
         ck(cudaGetLastError(), "batched expand");
         // the chunk's counters, the jobs' statistics and the goal pass's results, read back with one wait
         ck(cudaMemcpyAsync(&h, dst, sizeof(DevStats), cudaMemcpyDeviceToHost, s), "d2h");
@@ -5192,6 +5227,7 @@ struct BatchImpl : BatchSession::Impl {
         tqcap = std::max<unsigned long long>(tqcap, h.n_tq);
       }
       if (h.surv_overflow || h.n_tq > tqcap) throw std::runtime_error("survivor or T queue overflow");
+      if (h.n_left && !forms.general) throw std::logic_error("T bounds left over");
       if (ch.jobs.size() == 1) {                 // the one-job T kernel's tallies, kept in the chunk's block
         DevStats &d = hj[jlo];
         d.dead += h.dead; d.alive += h.alive; d.t_evals += h.t_evals;

@@ -76,3 +76,47 @@ def test_children_decided_from_their_parent(engine, oracle_bin, tmp_path, seed, 
     rc, lines = run_oracle(oracle_bin, p, ["--depth", "5"] + ([] if sym else ["--no-sym"]))
     out = engine.search(text, depth=5, sym=sym)
     assert (out.rc, out.lines()) == (rc, lines), circ
+
+
+def times3(text):
+    """the spec with its target's entries times 3: not unitary, the general form takes its whole queue"""
+    head, rest = text.split("\ntarget ", 1)
+    rows = rest.split("\n")
+    for r in range(1, 9):
+        rows[r] = " ".join(str(3 * int(v)) for v in rows[r].split())
+    return head + "\ntarget " + "\n".join(rows)
+
+
+def test_both_forms_in_one_batch(engine):
+    """jobs for the packed form alone, for both (residuals past the limit, non-monomial candidates) and for the general
+    one alone, advanced together: the same as each on its own"""
+    low = [workloads.make_spec(3, [("h", (0,)), ("t", (0,)), ("cx", (0, 1)), ("t", (1,)), ("h", (2,)), ("cx", (1, 2))], 6)]
+    high = [workloads.make_spec(3, target(s)[1], 10) for s in (85, 509, 581, 2740)]
+    texts = low + [spec_text("toffoli"), spec_text("ccx-lite")] + high + [times3(spec_text("toffoli")), times3(high[0])]
+    specs = [cz.Spec(t) for t in texts]
+    assert {s.n for s in specs} == {3}
+    for group in (specs, specs[:1], specs[2:3], specs[-1:], specs[1:4]):
+        b = cz.Batch(engine, 3)
+        ids = [b.submit(s, depth=8) for s in group]
+        b.run()
+        for s, i in zip(group, ids):
+            plain, got = engine.search(s, depth=8), b.result(i)
+            assert (got.rc, got.lines(), got.circuit) == (plain.rc, plain.lines(), plain.circuit)
+        b.close()
+
+
+@pytest.mark.parametrize("n,length,budget", [(1, 12, 12), (2, 14, 9), (3, 18, 9)])
+@pytest.mark.parametrize("seed", range(6))
+def test_root_exponents(engine, oracle_bin, tmp_path, n, length, budget, seed):
+    """roots of every small exponent at budgets where it bounds the residuals' exponents, and where the level does"""
+    rng = random.Random(100 * n + seed)
+    circ = []
+    for _ in range(length):
+        g = rng.choice(["h", "h", "t", "cx"] if n > 1 else ["h", "t", "t"])
+        circ.append((g, tuple(rng.sample(range(n), 2)) if g == "cx" else (rng.randrange(n),)))
+    text = workloads.make_spec(n, circ, budget)
+    p = tmp_path / "t.spec"
+    p.write_text(text)
+    rc, lines = run_oracle(oracle_bin, p, [])
+    out = engine.search(text)
+    assert (out.rc, out.lines()) == (rc, lines)
