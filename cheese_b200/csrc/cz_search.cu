@@ -1365,7 +1365,7 @@ __device__ __forceinline__ void expand_parent(const DevSpec &sp, const DevSpec *
     }
     for (; todo; todo &= todo - 1) {
       const int g = g0 + __ffs(todo) - 1;
-      int kind = __shfl_sync(FULL, fate, g - g0);
+      int kind = STATES ? (int)FULLC : __shfl_sync(FULL, fate, g - g0);
       const uint8_t fl = sp.gflags[g];
       const int gm = sp.gmask[g], gq0 = sp.gq[g][0];
       // the child's bounds (the parent's until shown otherwise) and the lane's entries of its residual
@@ -1571,7 +1571,10 @@ __global__ void __launch_bounds__(EXP_WARPS * 32) k_goal_level(const DevSpec sp,
 // A warp's parents: taken from a counter two ahead, the residual one ahead (copied into shared memory by cp.async while
 // the current parent is expanded), so neither the counter nor the loads are waited for. body(p, P, meta, sub). A level
 // with fewer parents than warps on the chip splits each parent's candidates over `split` warps (sub = 0 .. split - 1).
-template <int NQ, typename ST, typename Body>
+// AHEAD false: a warp takes a parent only when it is done with the one before. So for state targets: their children cost so
+// much (0.1 ms of a warp each) that a parent held by a busy warp delays the level's end, and the loads hidden are nothing beside
+// it (a 3-qubit search of 5.9 M prefixes: 71.1 ms of level kernels taking ahead, 66.5 ms so).
+template <int NQ, typename ST, bool AHEAD = true, typename Body>
 __device__ __forceinline__ void walk_parents(ExpandSmem<NQ, ST> &sm, unsigned long long *counter, unsigned long long p0,
                                              unsigned long long end, const Z4<ST> *R, const NodeMeta *meta, int w, int lane,
                                              int split, Body body) {
@@ -1588,8 +1591,19 @@ __device__ __forceinline__ void walk_parents(ExpandSmem<NQ, ST> &sm, unsigned lo
     }
     cp_async_commit();
   };
-  unsigned long long p = __shfl_sync(FULL, grab(), 0), raw = grab();
   NodeMeta m{}, mn{};
+  if constexpr (!AHEAD) {
+    for (;;) {
+      const unsigned long long p = __shfl_sync(FULL, grab(), 0);
+      if (p >= end) return;
+      fetch(p, 0, m);
+      cp_async_wait<0>();
+      __syncwarp();
+      body(parent(p), sm.P[w][0], m, split == 1 ? 0 : (int)((unsigned)p % (unsigned)split));
+      __syncwarp();
+    }
+  }
+  unsigned long long p = __shfl_sync(FULL, grab(), 0), raw = grab();
   int b = 0;
   fetch(p, 0, m);
   while (p < end) {
@@ -1625,7 +1639,7 @@ __global__ void __launch_bounds__(EXP_WARPS * 32, EXP_MINB) k_expand(const DevSp
   const ExpandOut<ST> o{a.st, a.cap, a.sh1, a.sh2, a.sidx, a.smeta, a.tq, a.tqcap};
   const auto weight = [&](int s, int e) { return sm.Wt[s][e & (E - 1)]; };
   WarpTally c;
-  walk_parents<NQ, ST>(sm, PART == 2 ? &a.st->work2 : &a.st->work, 0, (unsigned long long)a.m * a.split, a.R, a.meta, w,
+  walk_parents<NQ, ST, !STATES>(sm, PART == 2 ? &a.st->work2 : &a.st->work, 0, (unsigned long long)a.m * a.split, a.R, a.meta, w,
                        lane, a.split, [&](unsigned long long p, const Z4<ST> *P, const NodeMeta &pm, int sub) {
     expand_parent<NQ, ST, STATES, PART>(sp, &s_sp, weight, conjmask, P, sm.C[w], sm.F[w], p, pm, a.rem, a.keep != 0, sp.G,
                                         o, c, lane, a.split, sub);
