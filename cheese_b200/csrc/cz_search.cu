@@ -3052,7 +3052,6 @@ struct Engine::Impl {
   bool lean_level = false;                 // the last level of a levels() call keeps its tree and keys, not its
                                            // residuals (the last searched level of --table K)                  // keep the frontier's class keys (fK1, fK2)
   DBuf fK1, fK2, tptrs, keys2, old;
-  DBuf sflags;                             // cz_sort_pairs: its SortFlags
   DBuf outb;                               // a table candidate's symmetry elements and residual
   DevStats *hstats = nullptr;              // pinned
   long long launches = 0, expand_launches = 0, h2d = 0, d2h = 0;
@@ -3083,10 +3082,10 @@ struct Engine::Impl {
     for (auto &e : ev) ck(cudaEventCreate(&e), "event");
     ck(cudaMallocHost(&hstats, sizeof(DevStats) + sizeof(GoalShort)), "pinned");
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    stats.ensure(sizeof(DevStats) + sizeof(GoalShort));
-    sflags.ensure(sizeof(SortFlags));
-    ck(cudaMemsetAsync(sflags.p, 0, sizeof(SortFlags), s), "memset");
+    stats.ensure(sizeof(DevStats) + sizeof(GoalShort) + sizeof(SortFlags));
+    ck(cudaMemsetAsync(sort_flags(), 0, sizeof(SortFlags), s), "memset");
   }
+  SortFlags *sort_flags() { return (SortFlags *)(stats.as<char>() + sizeof(DevStats) + sizeof(GoalShort)); }
   size_t trim() {
     size_t n = 0;
     for (DBuf *b : {&fR, &fMeta, &fR2, &fMeta2, &sH1, &sH2, &sIdx, &sMeta, &tq, &tqleft, &k0, &k1, &v0, &v1, &hist, &part,
@@ -3107,7 +3106,7 @@ struct Engine::Impl {
       b->release();
     for (auto &sd : specs) sd.release();
     for (auto &kv : dtabs) { kv.second->release(); delete kv.second; }
-    for (DBuf *b : {&fK1, &fK2, &tptrs, &keys2, &old, &gshort, &outb, &sflags}) b->release();
+    for (DBuf *b : {&fK1, &fK2, &tptrs, &keys2, &old, &gshort, &outb}) b->release();
     for (auto &b : par) b.release();
     for (auto &b : gat) b.release();
     side.release();
@@ -4537,7 +4536,7 @@ int Engine::sort_pairs(uint64_t *keys, uint32_t *vals, size_t n, int lo, int hi,
     I.hist.ensure(sort_hist_words(n) * 4);
     I.part.ensure(scan_partials_words(sort_hist_words(n)) * 4);
     SortScratch sc{I.hist.as<uint32_t>(), I.part.as<uint32_t>(), I.hist.cap / 4, I.part.cap / 4};
-    sc.flags = I.sflags.as<SortFlags>();
+    sc.flags = I.sort_flags();
     ck(cudaEventRecord(I.ev[0], I.s), "event");
     int nl = 0;
     const bool f = radix_sort(keys, vals, I.k1.as<uint64_t>(), I.v1.as<uint32_t>(), n, lo, hi, sc, I.s, &nl);
