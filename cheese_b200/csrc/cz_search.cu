@@ -47,10 +47,10 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr int RC_STOP = -3;        // levels(): stopped after the requested level
 constexpr int EXP_WARPS = 8;       // warps per expand block
 constexpr int EXP_MINB = 4;        // expand blocks per SM: 32 warps (64 registers; latency-bound code, measured
-                                   // 6 % faster than 2 blocks of 128 registers despite small spills)
+                                   // 6 % faster than 2 blocks of 128 registers despite a spill of two registers)
 constexpr int EXPB_MINB = 3;       // batched: 3 blocks of 80 registers as fast as 4 of 64 with more spills, or 2
-constexpr int INHERIT_KMAX = 60;
-enum GateKind : uint8_t { GK_GENERAL = 0, GK_ONEQ = 1, GK_PERM = 2 };   // the T bound is computed exactly (mod 2^32 / 2^64) only while 2(n + k) <= 128
+constexpr int INHERIT_KMAX = 60;   // the T bound is computed exactly (mod 2^32 / 2^64) only while 2(n + k) <= 128
+enum GateKind : uint8_t { GK_GENERAL = 0, GK_ONEQ = 1, GK_PERM = 2 };
 
 constexpr uint8_t QC_NONE = 0xff;
 // gcol: kind in the low 3 bits, qubit a in bits 3-4, qubit b in bits 5-6
@@ -200,20 +200,19 @@ template <typename U> __device__ __forceinline__ U pair_component(int comp, cons
     default: return (y.a - y.c) * x.b + (y.b - y.d) * x.c + (y.a + y.c) * x.d - (y.b + y.d) * x.a;
   }
 }
-// the pairs of one round: f (f = 0 skipped) with point map e(i) = insert a 0 at bit j of i, or (IDENT: every f of
-// the round has the top bit) e(i) = i, known at compile time
-template <int NQ, typename U, int PASSES, bool IDENT, typename ST>
+// the pairs of one round: f (f = 0 skipped) with point map e(i) = insert a 0 at bit j of i
+template <int NQ, typename U, int PASSES, typename ST>
 __device__ __forceinline__ void tbound_round(const Z4<ST> *S, int f, U &P, U &Q) {
   constexpr int E = 1 << (2 * NQ), HP = E / 2, CPP = 4 / PASSES;
   static_assert(4 % PASSES == 0, "passes split the four components evenly");
   if (f == 0) return;
-  const int lomask = IDENT ? E - 1 : ((f & HP) ? E - 1 : (f & -f) - 1);   // bits below the inserted 0
+  const int lomask = (f & HP) ? E - 1 : (f & -f) - 1;   // bits below the inserted 0
 #pragma unroll 1
   for (int pass = 0; pass < PASSES; pass++) {
     U v[CPP][HP];
 #pragma unroll
     for (int i = 0; i < HP; i++) {
-      const int e = IDENT ? i : (i & lomask) | ((i & ~lomask) << 1);
+      const int e = (i & lomask) | ((i & ~lomask) << 1);
       const Z4<U> y = toU<U>(S[e]), x = toU<U>(S[e ^ f]);
 #pragma unroll
       for (int c = 0; c < CPP; c++) v[c][i] = pair_component<U>(pass * CPP + c, x, y);
@@ -240,17 +239,12 @@ __device__ __forceinline__ void tbound_round(const Z4<ST> *S, int f, U &P, U &Q)
     }
   }
 }
-template <int NQ, typename U, int PASSES, typename ST, bool SPLIT = false>
+template <int NQ, typename U, int PASSES, typename ST>
 __device__ __forceinline__ int tbound_lanes(const Z4<ST> *S, int k, int lane) {
   constexpr int E = 1 << (2 * NQ);
   U P = 0, Q = 0;
-  if constexpr (E == 64 && SPLIT) {        // round 0: f = lane (insert map), round 1: f = 32 + lane (top bit)
-    tbound_round<NQ, U, PASSES, false>(S, lane, P, Q);
-    tbound_round<NQ, U, PASSES, true>(S, 32 + lane, P, Q);
-  } else {
 #pragma unroll 1
-    for (int f = lane; f < E; f += 32) tbound_round<NQ, U, PASSES, false>(S, f, P, Q);
-  }
+  for (int f = lane; f < E; f += 32) tbound_round<NQ, U, PASSES>(S, f, P, Q);
   // f = 0: alpha = |y|^2 real part, beta its sqrt2 part, transformed over all E points across the warp
   constexpr int PL = E > 32 ? E / 32 : 1;   // points per lane
   U al[PL], be[PL];
@@ -3016,7 +3010,7 @@ struct Engine::Impl {
   cudaStream_t s = nullptr;
   cudaEvent_t ev[4];
   DBuf fR, fMeta, fR2, fMeta2;             // frontier, next frontier
-  DBuf sH1, sH2, sIdx, sMeta;              // survivors of the current level (32-byte records)
+  DBuf sH1, sH2, sIdx, sMeta;              // survivors of the current level (40-byte records)
   DBuf tq, tqleft;                         // deferred T evaluations of the current level; TBoundArgs::left
   DBuf k0, k1, v0, v1, hist, part;         // sort
   DBuf work, tmp, kidx, kslot;             // dedupe
@@ -3152,7 +3146,7 @@ __global__ void k_walk_back(const __grid_constant__ TreeLevels tree, unsigned lo
 // The forms of the T bound that the queue of level t can need. A spec that is not unitary, and int64 limbs, take the general
 // one alone. The packed one takes every child of a unit monomial while its exponent k allows: k is at most the root's plus
 // the most a gate adds on each of t - 1 levels, and an entry is queued only with k <= depth - t. The general launch is
-// left out where that shows it empty (a launch that finds nothing costs 3 us; small searches make 50 in a millisecond).
+// left out where that shows it empty (a launch that finds nothing costs about 4 us; small searches make 50 in a millisecond).
 struct TboundForms { bool packed, general; };
 template <int NQ, typename ST> TboundForms tbound_forms(const HostSpec &hs, const DevSpec &sp, int t, int depth) {
   if (sizeof(ST) != 4 || !sp.unit) return {false, true};

@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(TC_T) k_tc_keys(const TDev sp, const THist H, 
 // then each of its warps takes one rotation at a time; `split` CTAs share a parent when a level has few. With pmx, each
 // parent's matrix and exponent are kept (P^2 int2 at pmx + P^2 i, pe[i]) and per child its exponent (ce) and its columns in
 // the order of their hashes (co), so the exact dedupe compares two children column by column without searching.
-// Bound by issue (about 4000 instructions a child). One CTA per child, step by step, took 32 ns a child on
+// Bound by issue (7,400 instructions a child, 70 % of the issue slots). One CTA per child, step by step, took 32 ns a child on
 // the B200; a warp per child 10 ns (380,000 children of two queries of T count 7: 12.2 -> 3.8 ms).
 template <int LP>
 __global__ void __launch_bounds__(TC_T) k_tc_children(const TDev sp, const THist H, int tp, long long m, int split,
@@ -482,8 +482,9 @@ __global__ void k_tc_split(const uint64_t *keys, const uint32_t *vals, size_t n,
 // one warp per listed member: is it exactly the coset of its run's first member (equal h2 and exponent, and equal columns
 // up to sign in the order of their hashes)? Children's entries are recomputed from their kept parents. A member that is not,
 // be it for columns whose hashes agree by chance, counts as unresolved: the level is then deduped by the sequential
-// resolver instead, which handles any mix of cosets in a run. Bound by L2 (64 KB of parents a member); one CTA per member
-// with both children rebuilt, hashed and matched took 125 ns a member on the B200, this 11 ns (114,000 members: 14.3 -> 1.25 ms).
+// resolver instead, which handles any mix of cosets in a run. Bound by the latency of its loads (64 KB of parents a member,
+// L2 at 45 %); one CTA per member with both children rebuilt, hashed and matched took 125 ns a member on the B200, this
+// 11 ns (114,000 members: 14.3 -> 1.25 ms).
 template <int LP>
 __global__ void __launch_bounds__(TC_T) k_tc_dupcheck(const TDev sp, const uint64_t *keys, const uint32_t *vals,
                                                       size_t n, const uint32_t *check, const uint64_t *h2,
